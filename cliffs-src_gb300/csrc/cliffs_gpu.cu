@@ -17,6 +17,7 @@
 #include "batch.cuh"
 #include "staged.cuh"
 #include "ytile.cuh"
+#include "step.cuh"
 #include "depth_ssl.cuh"
 #include "boundary.cuh"
 
@@ -174,6 +175,10 @@ struct cliffs_ctx {
   // (the y-sweep of the tiled kernels when ytile_ok)
   CUtensorMap m_srf16[2], m_xu16[2], m_yv16[2];
   bool ytile_ok = false;
+  // the window maps of step_kernel (whole steps of the tiled kernels when
+  // step_ok)
+  CUtensorMap w_dep, w_srf[2], w_xu[2], w_yv[2];
+  bool step_ok = false;
   int grid_sx = 0, grid_sy = 0;  // resident blocks of staged_x / staged_y
   unsigned long long stage_ns = 2000000000ull;  // limit of one stage wait
   // fast-kernel sweeps launched as programmatic dependents of the previous
@@ -794,6 +799,83 @@ int launch_sweep(cliffs_ctx* c, int iu, int maxm, const double* fA, const double
   return CLIFFS_OK;
 }
 
+// Whether whole steps run as one kernel (step_kernel): two-dimensional grids
+// with the tiled kernels in their own block shapes, outside the per-sweep
+// profile.  A step in one kernel leaves the state in the other copy, so they
+// come in pairs (launch_step twice, or graphs of an even number of steps),
+// and a whole step call leaves the state where it found it.
+bool step_applies(const cliffs_ctx* c) {
+  return c->step_ok && c->sweep_kind == CLIFFS_SWEEP_TILED && c->blk_x == 128 && c->warps_y == 4 && !c->prof &&
+         !c->max_fresh;
+}
+
+// The two sweeps' arguments of one whole step from state copy s to 1 - s.
+void step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey, SweepArgs* X, SweepArgs* Y) {
+  *X = sweep_args(c, 1, false, s);
+  X->hmax_in = c->hmax;
+  X->velmax_in = c->velmax;
+  X->edges = ex;
+  *Y = sweep_args(c, 2, false, s);
+  Y->edges = ey;
+}
+
+PairConst pair_const(const SweepArgs& A) {
+  auto two = [](float a) {
+    uint32_t b;
+    std::memcpy(&b, &a, 4);
+    return (f2)b << 32 | (f2)b;
+  };
+  PairConst K;
+  K.g = two(A.ph.g);
+  K.gcrough = two(A.ph.gcrough);
+  K.mdt = two(-A.ph.dt);
+  K.half = two(0.5f);
+  K.quarter = two(0.25f);
+  K.nz = two(-0.f);
+  K.inv = two(A.geo0.x);
+  K.ndtx = two(-A.geo0.z);
+  K.ndfpm = two(-A.geo0.w);
+  return K;
+}
+
+dim3 step_grid(const cliffs_ctx* c) {
+  return dim3((c->nx + kStepW - 1) / kStepW, (c->ny + kStepR - 1) / kStepR);
+}
+
+// The variant for the grid's spacing: a table when an axis is not uniform,
+// else uniform spacing with or without the metric term.
+template <typename... Args>
+cudaError_t step_launch(const cliffs_ctx* c, const cudaLaunchConfig_t* cfg, Args... args) {
+  if (!c->geo_uni_x || !c->geo_uni_y) return cudaLaunchKernelEx(cfg, step_kernel<GEO_TABLE, GEO_TABLE>, args...);
+  if (c->scl_y || c->lscale) return cudaLaunchKernelEx(cfg, step_kernel<GEO_METRIC, GEO_METRIC>, args...);
+  return cudaLaunchKernelEx(cfg, step_kernel<GEO_FLAT, GEO_FLAT>, args...);
+}
+
+// One whole step on the context's stream, folding the previous step's end
+// state into the max-wave fields; ex, ey: the edge tables of a forced step.
+int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
+  SweepArgs X, Y;
+  const int s = c->cur;
+  step_args(c, s, ex, ey, &X, &Y);
+  const StepCtl C{S.wait_ns, S.extra, s};
+  const PairPair K{pair_const(X), pair_const(Y)};
+  const StepMaps M{c->w_dep, c->w_srf[s], c->w_xu[s], c->w_yv[s]};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = step_grid(c);
+  cfg.blockDim = dim3(kStepThreads);
+  cfg.stream = c->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = c->pdl ? 1 : 0;
+  ++c->launches;
+  CK(step_launch(c, &cfg, X, Y, M, C, K));
+  c->cur = 1 - s;
+  c->sweeps += 2u;
+  return CLIFFS_OK;
+}
+
 __global__ void k_maxwave_update(int nx, int ny, int pitch, const float* __restrict__ dep,
                                  const float* __restrict__ srf, const float* __restrict__ xu,
                                  const float* __restrict__ yv, float* hmax, float* velmax) {
@@ -1074,6 +1156,12 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
            !make_map(&c->m_xu16[k], c->xu[k], nx, ny, pp, 32, kYRows) &&
            !make_map(&c->m_yv16[k], c->yv[k], nx, ny, pp, 32, kYRows);
     c->ytile_ok = yt;
+    bool st = ok && c->xrun && c->yrun && !make_map(&c->w_dep, c->dep, nx, ny, pp, kStepWin, kStepRows);
+    for (int k = 0; k < 2 && st; ++k)
+      st = !make_map(&c->w_srf[k], c->srf[k], nx, ny, pp, kStepWin, kStepRows) &&
+           !make_map(&c->w_xu[k], c->xu[k], nx, ny, pp, kStepWin, kStepRows) &&
+           !make_map(&c->w_yv[k], c->yv[k], nx, ny, pp, kStepWin, kStepRows);
+    c->step_ok = st && cells < (1ull << 30);  // its stores take 32-bit byte offsets
     c->grid_sx = nsm * bx;
     c->grid_sy = nsm * by;
   }
@@ -1595,6 +1683,7 @@ int cliffs_gpu_feed_start(cliffs_ctx* c, double cuke) {
 // which the forcing ends is left to one_step.
 static int forced_graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* steps_done, int* done_out) {
   const int k = c->graph_k;
+  const bool whole = step_applies(c) && k % 2 == 0;
   *done_out = 0;
   if (!c->feed_on || k < 2 || nsteps < k || c->prof || c->rise_on || c->max_fresh || !c->xrun || !c->yrun)
     return CLIFFS_OK;
@@ -1635,10 +1724,15 @@ static int forced_graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* ste
         k, c->nx, c->ny, c->fw, c->fe, c->fs, c->fn, c->ring_irec, c->ring_cc, c->ring_x, c->ring_y);
     int r = cudaGetLastError() == cudaSuccess ? CLIFFS_OK : CLIFFS_ERR_CUDA;
     for (int s = 0; s < k && !r; ++s) {  // every step alike: the state is not fresh here
-      int mx, my;
-      step_modes(c, &mx, &my);
-      r = launch_sweep(c, 1, mx, c->fw, c->fe, c->ny, 2, 0.0, c->ring_x + (size_t)s * 6 * c->ny);
-      if (!r) r = launch_sweep(c, 2, my, c->fs, c->fn, c->nx, 2, 0.0, c->ring_y + (size_t)s * 6 * c->nx);
+      const float *ex = c->ring_x + (size_t)s * 6 * c->ny, *ey = c->ring_y + (size_t)s * 6 * c->nx;
+      if (whole) {
+        r = launch_step(c, ex, ey, StageCtl{c->stage_ns, 0u});
+      } else {
+        int mx, my;
+        step_modes(c, &mx, &my);
+        r = launch_sweep(c, 1, mx, c->fw, c->fe, c->ny, 2, 0.0, ex);
+        if (!r) r = launch_sweep(c, 2, my, c->fs, c->fn, c->nx, 2, 0.0, ey);
+      }
       step_done(c);
     }
     const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -1689,7 +1783,7 @@ static int forced_graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* ste
     CK(cudaEventRecord(c->ring_ev[slot], c->stream));
     c->ring_slot = (slot + 1) % cliffs_ctx::kRingSlots;
     CK(cudaGraphLaunch(c->fgraph, c->stream));
-    c->launches += 1 + 2 * (int64_t)k;
+    c->launches += 1 + (whole ? 1 : 2) * (int64_t)k;
     c->sweeps += 2u * (unsigned)k;
     *t = tt;
     c->irec = ir;
@@ -1740,14 +1834,19 @@ static int plain_graph(cliffs_ctx* c, int len, cliffs_ctx::PlainGraph** out) {
   const bool fresh = c->max_fresh, pending = c->max_pending;
   const int cur = c->cur;
   c->max_fresh = false;  // every captured step folds in the previous one
+  const bool whole = step_applies(c) && len % 2 == 0;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int r = CLIFFS_OK;
   for (int s = 0; s < len && !r; ++s) {
-    int mx, my;
-    step_modes(c, &mx, &my);
-    if (c->xrun) r = launch_sweep(c, 1, mx, nullptr, nullptr, c->ny, 2, 0.0);
-    if (!r && c->yrun) r = launch_sweep(c, 2, my, nullptr, nullptr, c->nx, 2, 0.0);
+    if (whole) {
+      r = launch_step(c, nullptr, nullptr, StageCtl{c->stage_ns, 0u});
+    } else {
+      int mx, my;
+      step_modes(c, &mx, &my);
+      if (c->xrun) r = launch_sweep(c, 1, mx, nullptr, nullptr, c->ny, 2, 0.0);
+      if (!r && c->yrun) r = launch_sweep(c, 2, my, nullptr, nullptr, c->nx, 2, 0.0);
+    }
     step_done(c);
   }
   const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
@@ -1780,13 +1879,16 @@ static bool plain_graphs_apply(const cliffs_ctx* c) {
   return c->graph_k >= 2 && !c->feed_on && !c->prof && !c->rise_on;
 }
 
-// Steps of the next graph for `remaining` steps: graph_k, or the rest; a
-// one-dimensional grid (one sweep per step) takes an even count, so that a
-// graph ends on the state copy it started from.  0: none (run directly).
+// Launches of a graph's step: its sweeps, or one for a whole step.
+static int step_launches(const cliffs_ctx* c) { return step_applies(c) ? 1 : (c->xrun ? 1 : 0) + (c->yrun ? 1 : 0); }
+
+// Steps of the next graph for `remaining` steps: graph_k, or the rest; with
+// one launch per step (a one-dimensional grid, whole steps in one kernel) an
+// even count, so that a graph ends on the state copy it started from.  0: none
+// (run directly).
 static int plain_graph_len(const cliffs_ctx* c, int remaining) {
-  const int per = (c->xrun ? 1 : 0) + (c->yrun ? 1 : 0);
   int len = std::min(c->graph_k, remaining);
-  if ((per * len) & 1) len -= 1;
+  if ((step_launches(c) * len) & 1) len -= 1;
   return len >= 2 ? len : 0;
 }
 
@@ -1806,7 +1908,7 @@ static int one_step(cliffs_ctx* c, double* t);
 static int graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* steps_done, int* done_out) {
   *done_out = 0;
   if (!plain_graphs_apply(c) || nsteps < 2) return CLIFFS_OK;
-  const int per = (c->xrun ? 1 : 0) + (c->yrun ? 1 : 0);
+  const int sweeps = (c->xrun ? 1 : 0) + (c->yrun ? 1 : 0), per = step_launches(c);
   int done = 0;
   for (int len; (len = plain_graph_len(c, nsteps - done)) > 0;) {
     cliffs_ctx::PlainGraph* pg = plain_graph_find(c, len);
@@ -1815,8 +1917,15 @@ static int graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* steps_done
       // the graph is captured and instantiated while the device works on
       // them, for the calls that follow (cliffs_gpu_prepare_steps builds it
       // ahead instead)
+      const bool whole = step_applies(c);
       for (int s = 0; s < len; ++s) {
-        RET(one_step(c, t));
+        if (whole) {
+          *t = *t + c->dt;
+          RET(launch_step(c, nullptr, nullptr, StageCtl{c->stage_ns, 0u}));
+          step_done(c);
+        } else {
+          RET(one_step(c, t));
+        }
         if (steps_done) *steps_done += 1;
       }
       RET(plain_graph(c, len, &pg));
@@ -1825,7 +1934,7 @@ static int graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* steps_done
     }
     CK(cudaGraphLaunch(pg->exec, c->stream));
     c->launches += (int64_t)per * len;
-    c->sweeps += (unsigned)(per * len);
+    c->sweeps += (unsigned)(sweeps * len);
     for (int s = 0; s < len; ++s) step_done(c);
     for (int s = 0; s < len; ++s) *t = *t + c->dt;
     if (steps_done) *steps_done += len;
@@ -1841,15 +1950,18 @@ int cliffs_gpu_prepare_steps(cliffs_ctx* c, int32_t nsteps) {
   if (!plain_graphs_apply(c)) return CLIFFS_OK;
   // the graphs cliffs_gpu_step(nsteps) would replay; a fresh state's first
   // step runs alone
-  int n = nsteps - (c->max_fresh && nsteps > 0 ? 1 : 0);
-  int last = -1;
-  for (int len; (len = plain_graph_len(c, n)) > 0; n -= len) {
+  const bool fresh = c->max_fresh;
+  int n = nsteps - (fresh && nsteps > 0 ? 1 : 0);
+  c->max_fresh = false;  // as the graphs' steps will find it
+  int r = CLIFFS_OK, last = -1;
+  for (int len; !r && (len = plain_graph_len(c, n)) > 0; n -= len) {
     if (len == last) continue;
     cliffs_ctx::PlainGraph* pg = nullptr;
-    RET(plain_graph(c, len, &pg));
+    r = plain_graph(c, len, &pg);
     last = len;
   }
-  return CLIFFS_OK;
+  c->max_fresh = fresh;
+  return r;
 }
 
 int cliffs_gpu_set_graph_steps(cliffs_ctx* c, int32_t k) {
@@ -1922,6 +2034,15 @@ int cliffs_gpu_step(cliffs_ctx* c, int32_t nsteps, double* t, int32_t* steps_don
   const int gr = graph_steps(c, nsteps - done, t, steps_done, &gdone);
   if (gr) return gr;
   done += gdone;
+  while (nsteps - done >= 2 && !c->feed_on && !c->rise_on && step_applies(c)) {  // no graphs: whole steps in pairs
+    for (int s = 0; s < 2; ++s) {
+      *t = *t + c->dt;
+      RET(launch_step(c, nullptr, nullptr, StageCtl{c->stage_ns, 0u}));
+      step_done(c);
+      ++done;
+      if (steps_done) *steps_done = done;
+    }
+  }
   for (; done < nsteps; ++done) {
     const int r = one_step(c, t);
     if (r) return r;
@@ -2427,6 +2548,22 @@ int cliffs_gpu_check_stage_timeout(cliffs_ctx* c, int32_t wait_ms) {
     else
       tile_y_kernel<false><<<grid, kStagedThreads, 0, c->stream>>>(Ay, M, S);
     CK(cudaGetLastError());
+    f = 0;
+    CK(cudaMemcpyAsync(&f, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (!(f & ST_STALL)) return CLIFFS_OK;
+  }
+  if (c->step_ok) {
+    // and for one whole step (step_kernel), whose blocks leave before the
+    // max-wave fold and before their first store
+    const int s = c->cur;
+    const int64_t launches = c->launches;
+    const unsigned sweeps = c->sweeps;
+    RET(launch_step(c, nullptr, nullptr, S));
+    c->cur = s;  // nothing was stored
+    c->launches = launches + 1;
+    c->sweeps = sweeps;
     f = 0;
     CK(cudaMemcpyAsync(&f, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->stream));

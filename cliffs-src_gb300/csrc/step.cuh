@@ -1,0 +1,991 @@
+// step.cuh -- one whole time step of a two-dimensional grid (the x-sweep and
+// the y-sweep of cliffs_main.f:317-345) in one kernel.
+//
+// A sweep per launch moves the state through memory twice a step: 72 bytes a
+// cell, and each cell's window is loaded, classified and converted once per
+// sweep.  Here a block takes a tile of kStepW columns x kStepR rows with one
+// halo row on each side (the y-sweep's), brings it into shared memory with
+// tensor-map copies, sweeps its rows in place, then its columns out of the
+// swept tile straight to the other copy of the state: 44 bytes a cell, the
+// max-wave fold included.
+//
+// Both sweeps march: a thread owns two lines of a sweep (two rows kStepPair
+// apart in the x phase, two adjacent columns in the y phase) over 8 cells and
+// carries the last cell and the last face's flux along, so that every celerity
+// is computed 10/8 and every face flux 9/8 times a cell (6/4 and 5/4 in
+// fast_kernel).  The two lines are the two halves of packed FP32 operations
+// (add/sub/mul/fma.rn.f32x2): the same roundings as march.cuh's scalar ones,
+// at half the issue slots.
+//
+// Classification.  As in sweep.cuh, a cell takes the plain update when it is
+// interior and it and its neighbours are wet and subcritical; every other cell
+// is left out of the thread's stores and, unless it is dry land at rest, put
+// on the block's list, which the whole block finishes through the full rules
+// after the phase (shore_cell for the most part: no cell is flooded; else
+// general_cell).  The x phase's listed cells are evaluated on the step's input
+// in global memory; the y phase's on the x-swept tile.
+//
+// Measured (us per step, replayed from graphs, against a launch per sweep;
+// the same state bits): 2048 x 2048 shelf 46.5 from 68.6; 4320 x 2160 sphere
+// 89.8 from 144.2; 600 x 600 15.4 from 18.4; 256 x 256 14.5 from 15.7.  On the
+// shelf 204 thread instructions a cell (400 in the two sweeps), 39 bytes a cell
+// to and from DRAM, 16 warps an SM at 128 registers and 0.54 instructions an
+// SM sub-core and cycle while it is busy: what bounds it is the latency of the
+// march and of the window's copies, then the end of the grid, whose last
+// blocks leave SMs idle for an eighth of the step.  The same march on one line
+// a thread in scalar operations (64 registers, 32 warps) issued 271
+// instructions a cell at 0.70 and took 50.6 us; 96 registers and 5 blocks an
+// SM 50.8 us (spills); tiles of 32 columns 48.9 us; the max-wave update on the
+// outputs, in the y phase, 49.5 us.
+#pragma once
+#include "staged.cuh"
+
+namespace cliffs {
+
+constexpr int kStepW = 64;                 // columns of a tile (32 or 64)
+constexpr int kStepThreads = 2 * kStepW;
+constexpr int kStepBlocks = 512 / kStepThreads;  // per SM: 128 registers a thread
+constexpr int kStepRows = 32;          // rows of its window
+constexpr int kStepR = kStepRows - 2;  // rows of a tile
+constexpr int kStepPair = 16;          // rows between the two lines of an x thread
+// columns of the window: one 16-byte chunk on the left, two on the right (the
+// second unused): rows of an odd number of 16-byte chunks, so that the x
+// phase's 16-byte accesses (2 rows x 4 segments a quarter warp) meet no bank
+// conflicts
+constexpr int kStepWin = kStepW + 12;
+constexpr int kStepField = kStepRows * kStepWin;  // floats of one field of the window
+constexpr uint32_t kStepBytes = 4u * kStepField * 4u;
+
+struct StepMaps {
+  CUtensorMap dep, srf, xu, yv;  // the input copy's fields, a kStepWin x kStepRows box
+};
+
+// ---- two FP32 lanes in a 64-bit register ---------------------------------------
+
+using f2 = unsigned long long;
+
+__device__ __forceinline__ f2 pk(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float lo2(f2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(f2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// A product that a sum takes in, as a fused operation with a zero of the sign
+// that leaves every product as it is: a packed product and the packed sum after
+// it come out of the compiler as one operation, and the sum's operand is to be
+// rounded.  nz is a pair of -0 that the compiler does not see.
+__device__ __forceinline__ f2 mulr2(f2 a, f2 b, f2 nz) { return fma2(a, b, nz); }
+__device__ __forceinline__ f2 both(float a) { return pk(a, a); }
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// The constants of packed operations on one axis, each in both halves.  A
+// phase reads them once from shared memory into registers, in a way that the
+// compiler cannot repeat: made of scalars or read from the kernel's
+// parameters they cost two moves at every use.  Signs are chosen so that one
+// of dt and -dt, and of dtx and -dtx, is enough.
+struct PairConst {
+  f2 g, gcrough, mdt;   // gravity, its product with the friction coefficient, -dt
+  f2 half, quarter, nz;  // 1/2, 1/4, -0 (mulr2)
+  f2 inv, ndtx, ndfpm;  // a uniform axis: 1/dx, -dt/(2 dx), 0
+};
+
+__device__ __forceinline__ f2 ld_const(const f2* p) {
+  f2 r;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"(smem_u32(p)));
+  return r;
+}
+__device__ __forceinline__ PairConst load_const(const PairConst* p) {
+  PairConst k;
+  k.g = ld_const(&p->g);
+  k.gcrough = ld_const(&p->gcrough);
+  k.mdt = ld_const(&p->mdt);
+  k.half = ld_const(&p->half);
+  k.quarter = ld_const(&p->quarter);
+  k.nz = ld_const(&p->nz);
+  k.inv = ld_const(&p->inv);
+  k.ndtx = ld_const(&p->ndtx);
+  k.ndfpm = ld_const(&p->ndfpm);
+  return k;
+}
+
+struct PairPair {
+  PairConst x, y;
+};
+
+struct StepCtl {
+  unsigned long long wait_ns;  // limit of the window's wait
+  unsigned extra;              // bytes it waits for beyond its copies: 0, except in the timeout self-test
+  int flip;                    // bands last to first
+};
+
+// rsqrtf for arguments that are not subnormal (celerities: g * max(H, ground);
+// speeds: max(., 1e-30); depths of wet cells): the same value without its
+// scaling of subnormal arguments.
+__device__ __forceinline__ float rsq(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// A cell of both lines as the march sees it.
+struct Cell2 {
+  f2 u, v, c, e;     // normal and tangential velocity, celerity, eta
+  f2 cc;             // friction (cliffs.f:204); not set on halo cells
+  float s[2], H[2];  // surface state, total depth
+};
+
+// Geometry kinds of an axis: uniform spacing alone; uniform spacing with a row
+// factor (x) or a metric term (y), as on a sphere; spacing from the table, with
+// either.
+enum { GEO_SCL = 1, GEO_DFPM = 2, GEO_FLAT = 0, GEO_METRIC = GEO_SCL, GEO_TABLE = GEO_SCL | GEO_DFPM };
+
+// Geometry of one position on both lines.
+struct Geo2 {
+  f2 inv;    // 1/dx of the face on the cell's right
+  f2 ndtx;   // -dt/(fm+fp) of the cell
+  f2 ndfpm;  // fm - fp of the cell
+  f2 scl8;   // 8 times the metric term of the cell
+};
+
+// What the march carries from cell to cell: the last cell, the tangential
+// velocity of the one before, and the last face's scaled fluxes.
+struct March {
+  Cell2 j;
+  f2 va;      // tangential velocity of the cell before j
+  f2 qP, qQ;  // FP/dx, FQ/dx of the face on j's left
+  f2 nqv;     // (v_a - v_j)/dx there
+};
+
+// HALO: a cell that is only a neighbour.
+template <bool HALO = false>
+__device__ __forceinline__ Cell2 make_cell2(const Phys<float>& p, const PairConst& K, float d0, float d1, float s0,
+                                            float s1, float u0, float u1, float v0, float v1) {
+  Cell2 n;
+  n.s[0] = s0;
+  n.s[1] = s1;
+  n.H[0] = add_rn(s0, fmaxf(d0, 0.f));
+  n.H[1] = add_rn(s1, fmaxf(d1, 0.f));
+  n.e = pk(sub_rn(s0, fminf(d0, 0.f)), sub_rn(s1, fminf(d1, 0.f)));
+  const f2 x = mul2(pk(fmaxf(n.H[0], p.ground), fmaxf(n.H[1], p.ground)), K.g);
+  n.c = mulr2(x, pk(rsq(lo2(x)), rsq(hi2(x))), K.nz);
+  n.u = pk(u0, u1);
+  n.v = pk(v0, v1);
+  n.cc = 0ull;
+  if (!HALO) {
+    const f2 w = fma2(n.u, n.u, mul2(n.v, n.v));
+    const f2 r = pk(rsq(n.H[0]), rsq(n.H[1]));
+    const f2 sp = mul2(w, pk(rsq(fmaxf(lo2(w), 1e-30f)), rsq(fmaxf(hi2(w), 1e-30f))));
+    n.cc = mulr2(mul2(mul2(n.u, K.gcrough), sp), mul2(mul2(r, r), r), K.nz);
+  }
+  return n;
+}
+
+// The scaled fluxes of the face between j and the next cell b (face_flux).
+__device__ __forceinline__ void face2(const Cell2& j, const Cell2& b, const PairConst& K, f2 inv, f2& qP, f2& qQ) {
+  const f2 U = add2(j.u, b.u), C = add2(j.c, b.c), du = sub2(b.u, j.u), dc = sub2(b.c, j.c);
+  const f2 gde = mulr2(sub2(b.e, j.e), K.g, K.nz);
+  const f2 Udc = mulr2(U, dc, K.nz);
+  const f2 FP = fma2(mul2(add2(U, C), K.half), du, add2(gde, Udc));
+  const f2 FQ = fma2(mul2(sub2(U, C), K.half), du, sub2(gde, Udc));
+  qP = mulr2(FP, inv, K.nz);
+  qQ = mulr2(FQ, inv, K.nz);
+}
+
+// The plain update (interior_update<float, false, SPH>) of the march's cell j,
+// with the fluxes qP, qQ of its right face and the next cell's tangential
+// velocity vb: new surface state, velocities and celerity of both lines.
+template <int G>
+__device__ __forceinline__ void update2(const March& m, f2 vb, f2 qP, f2 qQ, const Geo2& g, float ginv,
+                                        const PairConst& K, float (&os)[2], f2& ou, f2& ov, f2& cn) {
+  const f2 u = m.j.u, v = m.j.v, c = m.j.c;
+  const f2 ejP = add2(u, c), ejQ = sub2(u, c);
+  f2 QsP = mul2(add2(qP, m.qP), K.half);
+  f2 QsQ = mul2(add2(qQ, m.qQ), K.half);
+  QsP = fma2(mul2(ejP, g.ndtx), sub2(qP, m.qP), QsP);
+  QsQ = fma2(mul2(ejQ, g.ndtx), sub2(qQ, m.qQ), QsQ);
+  f2 qcP = add2(QsP, m.j.cc), qcQ = add2(QsQ, m.j.cc);
+  if (G & GEO_SCL) {
+    // 8 c u scl: the factor 8 is exact wherever it stands
+    const f2 sphr = mulr2(mul2(c, u), g.scl8, K.nz);
+    qcP = sub2(qcP, sphr);
+    qcQ = add2(qcQ, sphr);
+  }
+  const f2 dP = mulr2(qcP, K.mdt, K.nz), dQ = mulr2(qcQ, K.mdt, K.nz);
+  const f2 Qv = fma2(sub2(vb, v), g.inv, m.nqv);
+  const f2 nx = (G & GEO_DFPM) ? fma2(u, K.mdt, g.ndfpm) : mul2(u, K.mdt);  // -(u dt + fp - fm)
+  const f2 vx = fma2(Qv, nx, sub2(vb, m.va));
+  ov = fma2(mul2(u, g.ndtx), vx, v);
+  const f2 dc = mul2(sub2(dP, dQ), K.quarter);
+  cn = add2(c, dc);
+  ou = fma2(add2(dP, dQ), K.half, u);
+  // state_step of a wet cell that stays wet (cn > 0: the caller checks)
+  const f2 t = mul2(dc, add2(add2(c, c), dc));
+  os[0] = fma_rn(lo2(t), ginv, m.j.s[0]);
+  os[1] = fma_rn(hi2(t), ginv, m.j.s[1]);
+}
+
+// The sign bit set where a cell is wet, and where it is supercritical.
+__device__ __forceinline__ unsigned wet_sign(float H, const Phys<float>& p) {
+  return __float_as_uint(sub_rn(p.ground, H));
+}
+__device__ __forceinline__ unsigned sup_sign(float u, float c) { return __float_as_uint(sub_rn(c, fabsf(u))); }
+// A bit mask that takes in a sign bit: the newest cell at bit 0.
+__device__ __forceinline__ unsigned take_sign(unsigned mask, unsigned x) { return __funnelshift_l(x, mask, 1); }
+
+// ---- the cells that need the full rules ------------------------------------------
+
+// The value of line cell o where no flooding is in play: the cell and its two
+// neighbours are each either wet or stay land, so the cell becomes new land
+// (whatever its neighbours do), or takes its edge rule or the interior update
+// with mirror images in place of land neighbours (general_cell without its
+// flooding and limiter, which act on flooded cells only).  w: the raw cells
+// o-2 .. o+2; the outer two matter only to a wet cell, beside a land
+// neighbour.  Returns false when general_cell has to decide: the cell or a
+// neighbour of it is flooded, or a remainder of water or velocity lies on land
+// with no wet cell in reach.
+__device__ __forceinline__ bool shore_cell(const RawCell<float> (&w)[5], int o, int n, const LineCtx<float>& C,
+                                           const Geo<float>& g, const Phys<float>& p, OutCell<float>& out) {
+  float H[5], E[5];
+  bool wet[5];
+  bool anywet = false;
+#pragma unroll
+  for (int t = 0; t < 5; ++t) {
+    H[t] = depth_of(w[t].s, w[t].d);
+    E[t] = eta_of(w[t].s, w[t].d);
+    wet[t] = w[t].present && H[t] > p.ground;
+    anywet |= wet[t];
+  }
+  bool flooded = false;
+#pragma unroll
+  for (int t = 1; t <= 3; ++t) {
+    const bool fr = wet[t - 1] && w[t - 1].u >= 0.f && E[t - 1] + w[t].d > p.ground;
+    const bool fl = wet[t + 1] && w[t + 1].u <= 0.f && E[t + 1] + w[t].d > p.ground;
+    flooded |= w[t].present && !wet[t] && (t == 2 || wet[2]) && (fr || fl);
+  }
+  if (flooded) return false;
+  if (!wet[2]) {
+    if (!anywet && !(H[2] == 0.f && w[2].u == 0.f && w[2].v == 0.f)) return false;
+    out = OutCell<float>{state_from_depth(0.f, w[2].d), 0.f, 0.f};
+    return true;
+  }
+  CellState<float> f[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const RawCell<float>& r = w[t + 1];
+    const float h = H[t + 1];
+    f[t] = CellState<float>{r.u, fsqrt_pos(p.g * (h > p.ground ? h : p.ground)), E[t + 1], r.d, r.v, h};
+  }
+  const CellState<float>& j = f[1];
+  if (o == 1 || o == n) {
+    out = OutCell<float>{w[2].s, w[2].u, w[2].v};
+    const EdgeVals<float>& e = o == 1 ? C.eL : C.eR;
+    if (!(o == 1 ? wet[3] : wet[1]) || !(e.eta + j.d > p.ground)) return true;
+    float cn;
+    if (o == 1)
+      edge_left(j, f[2], e, C.inv_dx1, C.scl1, p, cn, out.u, out.v, out.s);
+    else
+      edge_right(f[0], j, e, C.inv_dxn1, C.scln, p, cn, out.u, out.v, out.s);
+    return true;
+  }
+  const CellState<float> mir{-j.u, j.c, j.e, j.d, j.v, j.H};
+  const CellState<float> a = wet[1] ? f[0] : mir, b = wet[3] ? f[2] : mir;
+  float FPl, FQl, FPr, FQr, cn;
+  face_flux(a.u, a.c, a.e, j.u, j.c, j.e, p, FPl, FQl);
+  face_flux(j.u, j.c, j.e, b.u, b.c, b.e, p, FPr, FQr);
+  out = interior_update(a, j, b, FPl, FQl, FPr, FQr, g, p, &cn);
+  return true;
+}
+
+// general_value<0> out of line: the rare remainder of step_x_value.
+__device__ __noinline__ OutCell<float> step_x_general(const SweepArgs& X, int L, int i) {
+  return general_value<0, false>(X, L, i);
+}
+
+// The x-swept value of grid cell (row L, column i), 1-based, from the step's
+// input in global memory.
+__device__ __noinline__ OutCell<float> step_x_value(const SweepArgs& X, int L, int i) {
+  const bool swept = L >= X.lo && L <= X.hi;
+  const int n = X.n;
+  RawCell<float> w[5];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) {
+    const int k = i - 2 + t;
+    w[t] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
+    if (k >= 1 && k <= n) {
+      const size_t q = cidx<0>(L, k, X.pitch);
+      w[t] = RawCell<float>{__ldg(X.dep + q), __ldg(X.srf + q), __ldg(X.xu + q), __ldg(X.yv + q), true};
+    }
+  }
+  if (!swept) return OutCell<float>{w[2].s, w[2].u, w[2].v};  // a row that is not swept
+  float alpha = 1.f, ialpha = 1.f;
+  if (X.lscale) {
+    const float2 a = __ldg(X.lscale + (L - 1));
+    alpha = a.x;
+    ialpha = a.y;
+  }
+  LineCtx<float> C;
+  C.eL = i == 1 ? edge_vals(X, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.eR = i == n ? edge_vals(X, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.inv_dx1 = X.inv_dx1 * ialpha;
+  C.inv_dxn1 = X.inv_dxn1 * ialpha;
+  C.scl1 = C.scln = 0.f;
+  OutCell<float> out;
+  if (shore_cell(w, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, out)) return out;
+  return step_x_general(X, L, i);
+}
+
+// Whether the x-swept cell (row L, column i) is wet.  A dry cell between dry
+// neighbours stays dry without an evaluation.
+__device__ __forceinline__ bool step_x_wet(const SweepArgs& X, int L, int i) {
+  bool any = false;
+  float dq = 0.f;
+  for (int k = max(i - 1, 1); k <= min(i + 1, X.n); ++k) {
+    const size_t q = cidx<0>(L, k, X.pitch);
+    const float d = __ldg(X.dep + q);
+    any = any || depth_of(__ldg(X.srf + q), d) > X.ph.ground;
+    if (k == i) dq = d;
+  }
+  return any && depth_of(step_x_value(X, L, i).s, dq) > X.ph.ground;
+}
+
+// The constants of column L that the rules at and beside cell o need.
+__device__ __forceinline__ LineCtx<float> y_line(const SweepArgs& Y, int L, int o) {
+  LineCtx<float> C;
+  C.n = Y.n;
+  C.wet = true;
+  C.eL = o == 1 ? edge_vals(Y, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.eR = o == Y.n ? edge_vals(Y, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.inv_dx1 = Y.inv_dx1;
+  C.inv_dxn1 = Y.inv_dxn1;
+  C.scl1 = Y.scl ? Y.scl[0] : 0.f;
+  C.scln = Y.scl ? Y.scl[Y.n - 1] : 0.f;
+  return C;
+}
+
+// step_y_value's full rules: the raw cells o-3 .. o+3, those outside the
+// window swept again from the step's input.
+__device__ __noinline__ OutCell<float> step_y_general(const SweepArgs& X, const SweepArgs& Y, const float* sm, int r0,
+                                                      int c0, int t, int c, bool& scan) {
+  const int o = r0 + t, L = c0 + c + 1, n = Y.n;
+  RawCell<float> w[7];
+  bool anywet = false;
+#pragma unroll 1
+  for (int q = 0; q < 7; ++q) {
+    const int k = o - 3 + q, tt = t - 3 + q;
+    RawCell<float> r{0.f, 0.f, 0.f, 0.f, false};
+    if (k >= 1 && k <= n) {
+      if (tt >= 0 && tt < kStepRows) {
+        const float* f = sm + tt * kStepWin + 4 + c;
+        r = RawCell<float>{f[0], f[kStepField], f[3 * kStepField], f[2 * kStepField], true};
+      } else {
+        const OutCell<float> x = step_x_value(X, k, L);
+        r = RawCell<float>{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
+      }
+      anywet |= depth_of(r.s, r.d) > Y.ph.ground;
+    }
+    w[q] = r;
+  }
+  scan = !anywet && !(depth_of(w[3].s, w[3].d) == 0.f && w[3].u == 0.f && w[3].v == 0.f);
+  if (scan) return OutCell<float>{w[3].s, w[3].u, w[3].v};
+  LineCtx<float> C = y_line(Y, L, o);
+  C.wet = anywet;
+  Geo<float> g[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) g[q] = geo_at(Y, o - 1 + q, 1.f, 1.f);
+  return general_cell(w, o, C, g, Y.ph);
+}
+
+// The y-swept value of tile cell (t, c) (row r0 + t, column c0 + c + 1,
+// 1-based) from the x-swept window sm.  scan: the cell keeps a remainder of
+// water or velocity with no wet cell in reach, and whether its column holds
+// one elsewhere decides (cliffs.f:113); nothing is returned then.
+__device__ __noinline__ OutCell<float> step_y_value(const SweepArgs& X, const SweepArgs& Y, const float* sm, int r0,
+                                                    int c0, int t, int c, bool& scan) {
+  const int o = r0 + t, L = c0 + c + 1, n = Y.n;
+  scan = false;
+  RawCell<float> w[5];
+  bool have[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int k = o - 2 + q, tt = t - 2 + q;
+    w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
+    have[q] = k < 1 || k > n || (tt >= 0 && tt < kStepRows);
+    if (k >= 1 && k <= n && have[q]) {
+      const float* f = sm + tt * kStepWin + 4 + c;
+      w[q] = RawCell<float>{f[0], f[kStepField], f[3 * kStepField], f[2 * kStepField], true};
+    }
+  }
+  // an outer cell outside the window matters to a wet cell beside a land
+  // neighbour, and to a remainder on land
+  if (!have[0] || !have[4]) {
+    const bool rest = w[2].u == 0.f && w[2].v == 0.f && depth_of(w[2].s, w[2].d) == 0.f;
+    const int q = have[0] ? 4 : 0, k = o - 2 + q;
+    const RawCell<float>& a = have[0] ? w[3] : w[1];
+    if (!rest && !(depth_of(a.s, a.d) > Y.ph.ground)) {
+      const OutCell<float> x = step_x_value(X, k, L);
+      const RawCell<float> r{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
+      if (have[0]) w[4] = r;
+      else w[0] = r;
+    }
+  }
+  OutCell<float> out;
+  if (shore_cell(w, o, n, y_line(Y, L, o), geo_at(Y, o, 1.f, 1.f), Y.ph, out)) return out;
+  return step_y_general(X, Y, sm, r0, c0, t, c, scan);
+}
+
+__device__ __forceinline__ void courant_status(const SweepArgs& A, float cour) {
+  if (__any_sync(0xffffffffu, cour > 0.5f)) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(2.f * cour));
+    if ((threadIdx.x & 31) == 0) {
+      atomicOr(A.status, ST_CFL);
+      atomicMax(A.status + 1, m);
+    }
+  }
+}
+
+// ---- the x phase ------------------------------------------------------------------
+
+// Appends the entries first + (bits of mask) to the block's list.
+__device__ __forceinline__ void list_push(unsigned mask, unsigned first, uint16_t* s_list, unsigned* s_n) {
+  if (!mask) return;
+  unsigned at = atomicAdd(s_n, (unsigned)__popc(mask));
+  for (; mask; mask &= mask - 1u) s_list[at++] = (uint16_t)(first + (unsigned)(__ffs(mask) - 1));
+}
+
+// Land at rest between dry cells: a cell that stays as it is.  near: the wet
+// bits of the cell and its neighbours.
+__device__ __forceinline__ bool at_rest(unsigned near, float H, float u, float v) {
+  return (near & 7u) == 0u && H == 0.f && u == 0.f && v == 0.f;
+}
+
+template <int GX>
+__device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst* sK, float* sm, int r0, int c0,
+                                             uint16_t* s_list, unsigned* s_n, bool& bad) {
+  const Phys<float>& p = X.ph;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a quarter warp takes 4 segments of 2 neighbouring rows; the warp, all
+  // segments of its rows
+  constexpr int kPairs = 256 / kStepW;  // row pairs of a warp
+  const int q4 = lane >> 3;
+  const int seg = (lane & 3) | (kStepW == 64 ? (q4 & 1) * 4 : 0);
+  const int tA = warp * kPairs + (kStepW == 64 ? q4 >> 1 : q4) * 2 + ((lane >> 2) & 1), tB = tA + kStepPair;
+  const int n = X.n, k0 = c0 + 8 * seg + 1;
+  float* rowA = sm + tA * kStepWin + 4 + 8 * seg;
+  float* rowB = rowA + kStepPair * kStepWin;
+  // the halo cells, before a neighbouring segment's results replace them
+  float hl[8], hr[8];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    hl[2 * f] = rowA[f * kStepField - 1];
+    hl[2 * f + 1] = rowB[f * kStepField - 1];
+    hr[2 * f] = rowA[f * kStepField + 8];
+    hr[2 * f + 1] = rowB[f * kStepField + 8];
+  }
+  __syncwarp();
+  const int LA = r0 + tA, LB = r0 + tB;  // 1-based rows
+  const bool swA = LA >= X.lo && LA <= X.hi && k0 <= n, swB = LB >= X.lo && LB <= X.hi && k0 <= n;
+  float cour = 0.f;
+  if (swA || swB) {
+    const PairConst K = load_const(sK);
+    f2 al = 0ull, ial = 0ull;  // row factors
+    Geo2 g{K.inv, K.ndtx, 0ull, 0ull};
+    if (GX != GEO_FLAT) {
+      float2 a = make_float2(1.f, 1.f), b = a;
+      if (X.lscale) {
+        a = __ldg(X.lscale + min(max(LA, X.lo), X.hi) - 1);
+        b = __ldg(X.lscale + min(max(LB, X.lo), X.hi) - 1);
+      }
+      al = pk(a.x, b.x);
+      ial = pk(a.y, b.y);
+      g.inv = mul2(K.inv, ial);
+      g.ndtx = mul2(K.ndtx, ial);
+    }
+    // sign bits of the cells taken in, the newest at bit 0
+    unsigned wetA = 0u, wetB = 0u, okA = 0u, okB = 0u;
+    unsigned restA = 0u, restB = 0u;  // listed cells: cell i at bit i
+    float cmA = 0.f, cmB = 0.f;       // the largest |u| + c of each line (times dt/(fm+fp) with GEO_TABLE)
+    f2 chk = 0ull;                    // 0 * results: NaN when one is not finite
+    // every cell of the segment interior, on swept rows
+    const bool inner = swA && swB && k0 >= 2 && k0 + 7 <= n - 1;
+    March m;
+    auto flags = [&](const Cell2& c) {
+      const unsigned a = wet_sign(c.H[0], p), b = wet_sign(c.H[1], p);
+      wetA = take_sign(wetA, a);
+      wetB = take_sign(wetB, b);
+      okA = take_sign(okA, a & ~sup_sign(lo2(c.u), lo2(c.c)));
+      okB = take_sign(okB, b & ~sup_sign(hi2(c.u), hi2(c.c)));
+    };
+    // the scaled fluxes of the face between m.j and the cell b at position k
+    auto face = [&](const Cell2& b, int k, f2& inv, f2& qP, f2& qQ) {
+      inv = g.inv;
+      if (GX == GEO_TABLE) {
+        // 1/dx(k-1): the table's left spacing of k or right spacing of k-1
+        // (the ends of the line have no entry)
+        const float x = k >= 2 && k <= n - 1 ? __ldg(X.geo + (k - 1)).x : (k == n ? __ldg(X.geo + (n - 2)).y : 0.f);
+        inv = mul2(both(x), ial);
+      }
+      face2(m.j, b, K, inv, qP, qQ);
+    };
+    auto take = [&](const Cell2& b, f2 inv, f2 qP, f2 qQ) {
+      m.nqv = mul2(sub2(m.j.v, b.v), inv);
+      m.qP = qP;
+      m.qQ = qQ;
+      m.va = m.j.v;
+      m.j = b;
+    };
+    // finishes cell i = m.j, with cell i + 1, and goes on to that one
+    auto advance = [&](const Cell2& b, int i) {
+      f2 inv, qP, qQ;
+      face(b, k0 + i + 1, inv, qP, qQ);
+      Geo2 gk = g;
+      if (GX == GEO_TABLE) {
+        const float4 q = __ldg(X.geo + (min(k0 + i, n) - 1));
+        gk.inv = inv;
+        gk.ndtx = mul2(both(-q.z), ial);
+        gk.ndfpm = mul2(both(-q.w), al);
+      }
+      float os[2];
+      f2 ou, ov, cn;
+      update2<GX & GEO_DFPM>(m, b.v, qP, qQ, gk, p.ginv, K, os, ou, ov, cn);
+      flags(b);
+      float *const fA = rowA + i, *const fB = rowB + i;
+      if ((okA & okB & 7u) == 7u && inner && fminf(lo2(cn), hi2(cn)) > 0.f) {
+        fA[kStepField] = os[0];
+        fA[2 * kStepField] = lo2(ou);
+        fA[3 * kStepField] = lo2(ov);
+        fB[kStepField] = os[1];
+        fB[2 * kStepField] = hi2(ou);
+        fB[3 * kStepField] = hi2(ov);
+        chk = fma2(pk(os[0], os[1]), 0ull, fma2(ou, 0ull, fma2(ov, 0ull, chk)));
+      } else {
+        const int k = k0 + i;
+        const bool in = k >= 2 && k <= n - 1;
+        const bool pA = in && swA && (okA & 7u) == 7u && lo2(cn) > 0.f;
+        const bool pB = in && swB && (okB & 7u) == 7u && hi2(cn) > 0.f;
+        if (pA) {
+          fA[kStepField] = os[0];
+          fA[2 * kStepField] = lo2(ou);
+          fA[3 * kStepField] = lo2(ov);
+        }
+        if (pB) {
+          fB[kStepField] = os[1];
+          fB[2 * kStepField] = hi2(ou);
+          fB[3 * kStepField] = hi2(ov);
+        }
+        // a finite sum of the stored values (0 where none is)
+        const float z = (pA ? os[0] + lo2(ou) + lo2(ov) : 0.f) * 0.f + (pB ? os[1] + hi2(ou) + hi2(ov) : 0.f) * 0.f;
+        bad = bad || z != z;
+        const bool lA = !pA && swA && !at_rest(wetA, m.j.H[0], lo2(m.j.u), lo2(m.j.v));
+        const bool lB = !pB && swB && !at_rest(wetB, m.j.H[1], hi2(m.j.u), hi2(m.j.v));
+        if (k <= n) {
+          restA |= (lA ? 1u : 0u) << i;
+          restB |= (lB ? 1u : 0u) << i;
+        }
+      }
+      float a = add_rn(fabsf(lo2(m.j.u)), lo2(m.j.c)), c = add_rn(fabsf(hi2(m.j.u)), hi2(m.j.c));
+      if (GX == GEO_TABLE) {
+        a *= -lo2(gk.ndtx);
+        c *= -hi2(gk.ndtx);
+      }
+      cmA = fmaxf(cmA, a);
+      cmB = fmaxf(cmB, c);
+      take(b, inv, qP, qQ);
+    };
+    // Cells i and i + 1 of both rows at once.  The next cell is made ready
+    // while one is finished: its square roots do not depend on the march, and
+    // hide the latency of the chain from face to update.
+    struct Two {
+      float2 d[2], s[2], u[2], v[2];
+    };
+    auto load = [&](int i) {
+      Two t;
+      t.d[0] = *reinterpret_cast<const float2*>(rowA + i);
+      t.d[1] = *reinterpret_cast<const float2*>(rowB + i);
+      t.s[0] = *reinterpret_cast<const float2*>(rowA + kStepField + i);
+      t.s[1] = *reinterpret_cast<const float2*>(rowB + kStepField + i);
+      t.u[0] = *reinterpret_cast<const float2*>(rowA + 2 * kStepField + i);
+      t.u[1] = *reinterpret_cast<const float2*>(rowB + 2 * kStepField + i);
+      t.v[0] = *reinterpret_cast<const float2*>(rowA + 3 * kStepField + i);
+      t.v[1] = *reinterpret_cast<const float2*>(rowB + 3 * kStepField + i);
+      return t;
+    };
+    auto first = [&](const Two& t) {
+      return make_cell2(p, K, t.d[0].x, t.d[1].x, t.s[0].x, t.s[1].x, t.u[0].x, t.u[1].x, t.v[0].x, t.v[1].x);
+    };
+    auto second = [&](const Two& t) {
+      return make_cell2(p, K, t.d[0].y, t.d[1].y, t.s[0].y, t.s[1].y, t.u[0].y, t.u[1].y, t.v[0].y, t.v[1].y);
+    };
+    Cell2 b;  // the cell after m.j
+    {
+      m.j = make_cell2<true>(p, K, hl[0], hl[1], hl[2], hl[3], hl[4], hl[5], hl[6], hl[7]);
+      flags(m.j);
+      const Two t = load(0);
+      const Cell2 j = first(t);
+      b = second(t);
+      f2 inv, qP, qQ;
+      face(j, k0, inv, qP, qQ);
+      flags(j);
+      take(j, inv, qP, qQ);
+    }
+#pragma unroll 1
+    for (int i = 0; i < 6; i += 2) {
+      const Two t = load(i + 2);
+      const Cell2 c = first(t);
+      advance(b, i);
+      b = second(t);
+      advance(c, i + 1);
+    }
+    const Cell2 h = make_cell2<true>(p, K, hr[0], hr[1], hr[2], hr[3], hr[4], hr[5], hr[6], hr[7]);
+    advance(b, 6);
+    advance(h, 7);
+    bad = bad || (swA && lo2(chk) != lo2(chk)) || (swB && hi2(chk) != hi2(chk));
+    list_push(restA, tA * kStepW + 8 * seg, s_list, s_n);
+    list_push(restB, tB * kStepW + 8 * seg, s_list, s_n);
+    if (GX != GEO_TABLE) {
+      cmA *= -lo2(g.ndtx);
+      cmB *= -hi2(g.ndtx);
+    }
+    cour = fmaxf(swA ? cmA : 0.f, swB ? cmB : 0.f);
+  }
+  courant_status(X, cour);
+}
+
+// ---- the y phase ------------------------------------------------------------------
+
+template <int GY>
+__device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst* sK, const float* sm, int r0, int c0,
+                                             uint16_t* s_list, unsigned* s_n, bool& bad) {
+  const Phys<float>& p = Y.ph;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int part = kStepW == 64 ? warp : 2 * warp + (lane >> 4);  // of four, 8 rows each
+  const int c = 2 * (kStepW == 64 ? lane : lane & 15), L = c0 + c + 1, n = Y.n;
+  const int t0 = 1 + 8 * part;
+  const int rows = min(min(8, kStepR - 8 * part), n - (r0 + t0) + 1);  // output rows of this thread
+  float cour = 0.f;
+  if (rows > 0 && L <= Y.nlines) {
+    const PairConst K = load_const(sK);
+    const bool sw0 = L >= Y.lo && L <= Y.hi, sw1 = L + 1 >= Y.lo && L + 1 <= Y.hi;
+    // every cell interior, on swept columns
+    const bool inner = sw0 && sw1 && r0 + t0 >= 2 && r0 + t0 + rows - 1 <= n - 1;
+    unsigned rest = 0u;  // listed cells: bit 2i + k, row t0 + i and column c + k
+    const float* at = sm + (t0 - 1) * kStepWin + 4 + c;
+    auto load = [&](const float* f) {
+      const float2 d = *reinterpret_cast<const float2*>(f), s = *reinterpret_cast<const float2*>(f + kStepField);
+      const float2 x = *reinterpret_cast<const float2*>(f + 2 * kStepField);
+      const float2 y = *reinterpret_cast<const float2*>(f + 3 * kStepField);
+      return make_cell2(p, K, d.x, d.y, s.x, s.y, y.x, y.y, x.x, x.y);
+    };
+    Cell2 b;  // the cell after m.j, made ready while m.j is finished
+    const Geo2 g{K.inv, K.ndtx, 0ull, 0ull};
+    March m;
+    // wet cells, and wet subcritical ones, of either column, the newest at bit 0
+    unsigned wet0 = 0u, wet1 = 0u, ok0 = 0u, ok1 = 0u;
+    auto flags = [&](const Cell2& b) {
+      const unsigned a0 = wet_sign(b.H[0], p), a1 = wet_sign(b.H[1], p);
+      wet0 = take_sign(wet0, a0);
+      wet1 = take_sign(wet1, a1);
+      ok0 = take_sign(ok0, a0 & ~sup_sign(lo2(b.u), lo2(b.c)));
+      ok1 = take_sign(ok1, a1 & ~sup_sign(hi2(b.u), hi2(b.c)));
+    };
+    float cm0 = 0.f, cm1 = 0.f;
+    f2 chk = 0ull;
+    auto face = [&](const Cell2& b, int k, f2& inv, f2& qP, f2& qQ) {  // between rows k - 1 and k
+      inv = g.inv;
+      if (GY == GEO_TABLE) {
+        const float x = k >= 2 && k <= n - 1 ? __ldg(Y.geo + (k - 1)).x : (k == n ? __ldg(Y.geo + (n - 2)).y : 0.f);
+        inv = both(x);
+      }
+      face2(m.j, b, K, inv, qP, qQ);
+    };
+    auto take = [&](const Cell2& b, f2 inv, f2 qP, f2 qQ) {
+      m.nqv = mul2(sub2(m.j.v, b.v), inv);
+      m.qP = qP;
+      m.qQ = qQ;
+      m.va = m.j.v;
+      m.j = b;
+    };
+    m.j = load(at);
+    m.va = 0ull;
+    flags(m.j);
+    {
+      const Cell2 j = load(at + kStepWin);
+      b = load(at + 2 * kStepWin);
+      f2 inv, qP, qQ;
+      face(j, r0 + t0, inv, qP, qQ);
+      take(j, inv, qP, qQ);
+      flags(j);
+    }
+    at += 2 * kStepWin;
+    // byte offset of the output pair (a field is below 4 GB)
+    uint32_t q = ((uint32_t)(r0 + t0 - 1) * (uint32_t)Y.pitch + (uint32_t)(L - 1)) * 4u;
+    char *const ps = reinterpret_cast<char*>(Y.srf_o), *const px = reinterpret_cast<char*>(Y.xu_o),
+               *const py = reinterpret_cast<char*>(Y.yv_o);
+#pragma unroll 2
+    for (int i = 0; i < rows; ++i, q += 4u * (uint32_t)Y.pitch) {
+      const int o = r0 + t0 + i;  // the row finished here
+      at += kStepWin;
+      // past the window's last row in a tile's last round: not used, within
+      // the block's shared memory
+      const Cell2 next = load(at);
+      f2 inv, qP, qQ;
+      face(b, o + 1, inv, qP, qQ);
+      Geo2 gk = g;
+      if (GY == GEO_TABLE) {
+        const float4 t = __ldg(Y.geo + (o - 1));
+        gk.inv = inv;
+        gk.ndtx = both(-t.z);
+        gk.ndfpm = both(-t.w);
+      }
+      if (GY & GEO_SCL) gk.scl8 = both(Y.scl ? 8.f * __ldg(Y.scl + (o - 1)) : 0.f);
+      float os[2];
+      f2 ou, ov, cn;
+      update2<GY>(m, b.v, qP, qQ, gk, p.ginv, K, os, ou, ov, cn);
+      flags(b);
+      if ((ok0 & ok1 & 7u) == 7u && inner && fminf(lo2(cn), hi2(cn)) > 0.f) {
+        *reinterpret_cast<float2*>(ps + q) = make_float2(os[0], os[1]);
+        *reinterpret_cast<f2*>(px + q) = ov;
+        *reinterpret_cast<f2*>(py + q) = ou;
+        chk = fma2(pk(os[0], os[1]), 0ull, fma2(ou, 0ull, fma2(ov, 0ull, chk)));
+      } else {
+        // plain cells take their results; columns that are not swept and land
+        // at rest keep their x-swept values; the others are listed
+        const bool in = o >= 2 && o <= n - 1;
+        const bool p0 = in && sw0 && (ok0 & 7u) == 7u && lo2(cn) > 0.f;
+        const bool p1 = in && sw1 && (ok1 & 7u) == 7u && hi2(cn) > 0.f;
+        const bool k0 = !sw0 || at_rest(wet0, m.j.H[0], lo2(m.j.u), lo2(m.j.v));
+        const bool k1 = !sw1 || at_rest(wet1, m.j.H[1], hi2(m.j.u), hi2(m.j.v));
+        const float s0 = p0 ? os[0] : m.j.s[0], x0 = p0 ? lo2(ov) : lo2(m.j.v), y0 = p0 ? lo2(ou) : lo2(m.j.u);
+        const float s1 = p1 ? os[1] : m.j.s[1], x1 = p1 ? hi2(ov) : hi2(m.j.v), y1 = p1 ? hi2(ou) : hi2(m.j.u);
+        const bool w0 = p0 || k0, w1 = (p1 || k1) && L + 1 <= Y.nlines;
+        if (w0) {
+          *reinterpret_cast<float*>(ps + q) = s0;
+          *reinterpret_cast<float*>(px + q) = x0;
+          *reinterpret_cast<float*>(py + q) = y0;
+        }
+        if (w1) {
+          *reinterpret_cast<float*>(ps + q + 4) = s1;
+          *reinterpret_cast<float*>(px + q + 4) = x1;
+          *reinterpret_cast<float*>(py + q + 4) = y1;
+        }
+        const float z = (w0 ? s0 + x0 + y0 : 0.f) * 0.f + (w1 ? s1 + x1 + y1 : 0.f) * 0.f;
+        bad = bad || z != z;
+        rest |= ((p0 || k0 ? 0u : 1u) | (p1 || k1 ? 0u : 2u)) << (2 * i);
+      }
+      float a0 = add_rn(fabsf(lo2(m.j.u)), lo2(m.j.c)), a1 = add_rn(fabsf(hi2(m.j.u)), hi2(m.j.c));
+      if (GY == GEO_TABLE) {
+        a0 *= -lo2(gk.ndtx);
+        a1 *= -lo2(gk.ndtx);
+      }
+      cm0 = fmaxf(cm0, a0);
+      cm1 = fmaxf(cm1, a1);
+      take(b, inv, qP, qQ);
+      b = next;
+    }
+    if (rest) {
+      unsigned w = atomicAdd(s_n, (unsigned)__popc(rest));
+      for (; rest; rest &= rest - 1u) {
+        const int b = __ffs(rest) - 1;
+        s_list[w++] = (uint16_t)((t0 + (b >> 1)) * kStepW + c + (b & 1));
+      }
+    }
+    cour = fmaxf(sw0 ? cm0 : 0.f, sw1 ? cm1 : 0.f);
+    if (GY != GEO_TABLE) cour *= -lo2(g.ndtx);
+    bad = bad || lo2(chk) != lo2(chk) || hi2(chk) != hi2(chk);
+  }
+  courant_status(Y, cour);
+}
+
+// ---- the step ---------------------------------------------------------------------
+
+struct StepShared {
+  __align__(128) float win[4 * kStepField];  // dep, srf, xu, yv: [row + 1 - r0][col + 4 - c0]
+  uint16_t list[kStepRows * kStepW];         // listed cells: window row * kStepW + tile column
+  unsigned n[2];                             // their number, x phase and y phase
+  unsigned scans;
+  PairConst k[2];                            // x and y axis
+  __align__(8) uint64_t bar;
+};
+
+// The max-wave fold of the step's input (cliffs_main.f:347-355) over the rows
+// of the window that the calling warp sweeps: loads issued before the wait for
+// the window's copies.
+struct Fold {
+  float4 h[4], v[4];
+};
+
+// Fold item k of a lane: window row and tile column (a float4).
+__device__ __forceinline__ void fold_item(int k, int& t, int& c) {
+  constexpr int kPairs = 256 / kStepW, kVecs = kStepW / 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = (32 * k + lane) / kVecs;  // of the warp's 2 * kPairs rows
+  t = warp * kPairs + r % kPairs + (r / kPairs) * kStepPair;
+  c = (lane % kVecs) * 4;
+}
+
+__device__ __forceinline__ bool fold_cell(const SweepArgs& X, int r0, int c0, int t, int c, size_t& q) {
+  const int row = r0 + t - 1;  // 0-based
+  q = (size_t)row * (size_t)X.pitch + (size_t)(c0 + c);
+  return t >= 1 && t <= kStepR && row < X.nlines && c0 + c < X.n;
+}
+
+template <int GX, int GY>
+__device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y, const StepMaps& M, int r0, int c0,
+                                          const StepCtl& C, StepShared& S) {
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    mbar_expect_tx(&S.bar, kStepBytes + C.extra);
+    tma_load_2d(S.win, &M.dep, &S.bar, c0 - 4, r0 - 1);
+    tma_load_2d(S.win + kStepField, &M.srf, &S.bar, c0 - 4, r0 - 1);
+    tma_load_2d(S.win + 2 * kStepField, &M.xu, &S.bar, c0 - 4, r0 - 1);
+    tma_load_2d(S.win + 3 * kStepField, &M.yv, &S.bar, c0 - 4, r0 - 1);
+  }
+  Fold F;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    int t, c;
+    size_t q;
+    fold_item(k, t, c);
+    F.h[k] = F.v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (fold_cell(X, r0, c0, t, c, q)) {
+      F.h[k] = __ldg(reinterpret_cast<const float4*>(X.hmax_in + q));
+      F.v[k] = __ldg(reinterpret_cast<const float4*>(X.velmax_in + q));
+    }
+  }
+  const bool ok = mbar_wait_ns(&S.bar, 0u, C.wait_ns);
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) {
+      atomicOr(X.status, ST_STALL);
+      mbar_wait_ns(&S.bar, 0u, C.wait_ns);  // the copies in flight, before the block's memory goes
+    }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    int t, c;
+    size_t q;
+    fold_item(k, t, c);
+    if (!fold_cell(X, r0, c0, t, c, q)) continue;
+    const float* f = S.win + t * kStepWin + 4 + c;
+    const float4 d = *reinterpret_cast<const float4*>(f), s = *reinterpret_cast<const float4*>(f + kStepField);
+    const float4 x = *reinterpret_cast<const float4*>(f + 2 * kStepField);
+    const float4 y = *reinterpret_cast<const float4*>(f + 3 * kStepField);
+    F.h[k].x = fmaxf(F.h[k].x, eta_of(s.x, d.x));
+    F.h[k].y = fmaxf(F.h[k].y, eta_of(s.y, d.y));
+    F.h[k].z = fmaxf(F.h[k].z, eta_of(s.z, d.z));
+    F.h[k].w = fmaxf(F.h[k].w, eta_of(s.w, d.w));
+    F.v[k].x = fmaxf(F.v[k].x, fma_rn(x.x, x.x, mul_rn(y.x, y.x)));
+    F.v[k].y = fmaxf(F.v[k].y, fma_rn(x.y, x.y, mul_rn(y.y, y.y)));
+    F.v[k].z = fmaxf(F.v[k].z, fma_rn(x.z, x.z, mul_rn(y.z, y.z)));
+    F.v[k].w = fmaxf(F.v[k].w, fma_rn(x.w, x.w, mul_rn(y.w, y.w)));
+    *reinterpret_cast<float4*>(X.hmax_in + q) = F.h[k];
+    *reinterpret_cast<float4*>(X.velmax_in + q) = F.v[k];
+  }
+  __syncwarp();  // the warp's rows are read before they are swept in place
+  bool bad = false;
+  step_x_phase<GX>(X, &S.k[0], S.win, r0, c0, S.list, &S.n[0], bad);
+  __syncthreads();
+  const unsigned cx = S.n[0];
+  if (cx) {
+    for (unsigned i = tid; i < cx; i += kStepThreads) {
+      const int t = S.list[i] / kStepW, c = S.list[i] % kStepW;
+      const OutCell<float> r = step_x_value(X, r0 + t, c0 + c + 1);
+      float* f = S.win + t * kStepWin + 4 + c;
+      f[kStepField] = r.s;
+      f[2 * kStepField] = r.u;
+      f[3 * kStepField] = r.v;
+      bad = bad || !isfinite(r.s + r.u + r.v);
+    }
+    __syncthreads();
+  }
+  step_y_phase<GY>(Y, &S.k[1], S.win, r0, c0, S.list, &S.n[1], bad);
+  __syncthreads();
+  const unsigned cy = S.n[1];
+  if (cy) {
+    for (unsigned i = tid; i < cy; i += kStepThreads) {
+      const int t = S.list[i] / kStepW, c = S.list[i] % kStepW;
+      bool scan;
+      const OutCell<float> r = step_y_value(X, Y, S.win, r0, c0, t, c, scan);
+      if (scan) {
+        S.list[i] |= 0x8000u;
+        S.scans = 1u;
+        continue;
+      }
+      const size_t q = (size_t)(r0 + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
+      Y.srf_o[q] = r.s;
+      Y.xu_o[q] = r.v;
+      Y.yv_o[q] = r.u;
+      bad = bad || !isfinite(r.s + r.u + r.v);
+    }
+    __syncthreads();
+    if (S.scans) {
+      // remainders on land: zeroed when the x-swept column holds a wet cell
+      // anywhere, else left as they are; the block looks through the column
+      // together, once for each run of entries of one column
+      int col = -1;
+      bool wet = false;
+      for (unsigned i = 0; i < cy; ++i) {
+        const unsigned ent = S.list[i];
+        if (!(ent & 0x8000u)) continue;
+        const int t = (int)(ent & 0x7fffu) / kStepW, c = (int)(ent & 0x7fffu) % kStepW;
+        if (c != col) {
+          col = c;
+          wet = false;
+          for (int j = 0; j < Y.n && !wet; j += kStepThreads)
+            wet = __syncthreads_or(j + tid < Y.n && step_x_wet(X, j + tid + 1, c0 + c + 1));
+        }
+        if (tid == 0) {
+          const float* f = S.win + t * kStepWin + 4 + c;
+          const size_t q = (size_t)(r0 + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
+          Y.srf_o[q] = wet ? state_from_depth(0.f, f[0]) : f[kStepField];
+          Y.xu_o[q] = wet ? 0.f : f[2 * kStepField];
+          Y.yv_o[q] = wet ? 0.f : f[3 * kStepField];
+        }
+      }
+    }
+  }
+  if (bad) atomicOr(X.status, ST_NAN);
+}
+
+// Tiles in bands of kStepR rows, the last band first when `flip` is set: a
+// step starts on the rows that the one before it wrote last, which are still
+// in L2.
+template <int GX, int GY>
+__global__ void __launch_bounds__(kStepThreads, kStepBlocks)
+    step_kernel(const __grid_constant__ SweepArgs X, const __grid_constant__ SweepArgs Y,
+                const __grid_constant__ StepMaps M, const StepCtl C, const __grid_constant__ PairPair K) {
+  __shared__ StepShared S;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (threadIdx.x == 0) {
+    mbar_init(&S.bar, 1);
+    S.n[0] = S.n[1] = S.scans = 0u;
+    S.k[0] = K.x;
+    S.k[1] = K.y;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int by = C.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+  step_tile<GX, GY>(X, Y, M, by * kStepR, (int)blockIdx.x * kStepW, C, S);
+}
+
+}  // namespace cliffs
