@@ -13,6 +13,9 @@
 //                     y tiles, meet again, and so on;
 //   batch_phase<DIR>  one launch per sweep direction and step covering every
 //                     scenario, for capture in a CUDA graph.
+// In graphs of one-tile list entries whole steps run as one launch instead
+// (batch_step_kernel, step.cuh), in pairs; the phases take a call's last odd
+// step, first steps from a fresh state and other tile shapes.
 // A scenario's tiles do the same arithmetic as its own sweep launches, so a
 // batched run is bit-identical to stepping the grids one by one.  Two
 // argument sets: "fused" (the y-sweep updates the max-wave fields with its

@@ -809,16 +809,6 @@ bool step_applies(const cliffs_ctx* c) {
          !c->max_fresh;
 }
 
-// The two sweeps' arguments of one whole step from state copy s to 1 - s.
-void step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey, SweepArgs* X, SweepArgs* Y) {
-  *X = sweep_args(c, 1, false, s);
-  X->hmax_in = c->hmax;
-  X->velmax_in = c->velmax;
-  X->edges = ex;
-  *Y = sweep_args(c, 2, false, s);
-  Y->edges = ey;
-}
-
 PairConst pair_const(const SweepArgs& A) {
   auto two = [](float a) {
     uint32_t b;
@@ -838,6 +828,20 @@ PairConst pair_const(const SweepArgs& A) {
   return K;
 }
 
+// The arguments of one whole step from state copy s to 1 - s.
+StepArgs step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey) {
+  StepArgs A;
+  A.X = sweep_args(c, 1, false, s);
+  A.X.hmax_in = c->hmax;
+  A.X.velmax_in = c->velmax;
+  A.X.edges = ex;
+  A.Y = sweep_args(c, 2, false, s);
+  A.Y.edges = ey;
+  A.K = PairPair{pair_const(A.X), pair_const(A.Y)};
+  A.M = StepMaps{c->w_dep, c->w_srf[s], c->w_xu[s], c->w_yv[s]};
+  return A;
+}
+
 dim3 step_grid(const cliffs_ctx* c) {
   return dim3((c->nx + kStepW - 1) / kStepW, (c->ny + kStepR - 1) / kStepR);
 }
@@ -854,12 +858,9 @@ cudaError_t step_launch(const cliffs_ctx* c, const cudaLaunchConfig_t* cfg, Args
 // One whole step on the context's stream, folding the previous step's end
 // state into the max-wave fields; ex, ey: the edge tables of a forced step.
 int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
-  SweepArgs X, Y;
   const int s = c->cur;
-  step_args(c, s, ex, ey, &X, &Y);
+  const StepArgs A = step_args(c, s, ex, ey);
   const StepCtl C{S.wait_ns, S.extra, s};
-  const PairPair K{pair_const(X), pair_const(Y)};
-  const StepMaps M{c->w_dep, c->w_srf[s], c->w_xu[s], c->w_yv[s]};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -870,7 +871,7 @@ int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl&
   cfg.attrs = at;
   cfg.numAttrs = c->pdl ? 1 : 0;
   ++c->launches;
-  CK(step_launch(c, &cfg, X, Y, M, C, K));
+  CK(step_launch(c, &cfg, A.X, A.Y, A.M, C, A.K));
   c->cur = 1 - s;
   c->sweeps += 2u;
   return CLIFFS_OK;
@@ -2774,6 +2775,13 @@ struct cliffs_batch {
   // runs batch_tile_y when flat along y
   YTileMaps* d_ymaps = nullptr;
   bool ytile = false;
+  // whole steps in one kernel (batch_step_kernel) for the one-tile graph
+  // plans: every scenario's arguments for the steps from its state copy cur
+  // ([0]) and back to it ([1]), the tile list, and the variant
+  StepArgs* d_step[2] = {nullptr, nullptr};
+  int* d_step_off = nullptr;  // n + 1 offsets, then n tiles across
+  int step_tiles = 0;
+  int step_geo = GEO_FLAT;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
   // groups, column groups); the list of a plan's tile shape is built from them
   std::vector<int> tx, ty, lx, ly;
@@ -2838,6 +2846,9 @@ static void batch_free(cliffs_batch* b) {
   if (b->d_gauge) cudaFree(b->d_gauge);
   if (b->d_grec) cudaFree(b->d_grec);
   if (b->d_ymaps) cudaFree(b->d_ymaps);
+  for (StepArgs* a : b->d_step)
+    if (a) cudaFree(a);
+  if (b->d_step_off) cudaFree(b->d_step_off);
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -2917,6 +2928,31 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
         return fail(CLIFFS_ERR_CUDA);
       b->ytile = true;
     }
+  }
+  bool whole = true;
+  for (int k = 0; k < n; ++k) whole = whole && ctxs[k]->step_ok;
+  if (whole) {
+    std::vector<StepArgs> sa[2];
+    std::vector<int> so((size_t)n + 1, 0), sg;
+    bool uniform = true, plain = true;
+    for (int k = 0; k < n; ++k) {
+      const cliffs_ctx* c = ctxs[k];
+      for (int q = 0; q < 2; ++q) sa[q].push_back(step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr));
+      const dim3 g = step_grid(c);
+      so[k + 1] = so[k] + (int)(g.x * g.y);
+      sg.push_back((int)g.x);
+      uniform = uniform && c->geo_uni_x && c->geo_uni_y;
+      plain = plain && !c->scl_y && !c->lscale;
+    }
+    b->step_geo = !uniform ? GEO_TABLE : plain ? GEO_FLAT : GEO_METRIC;
+    b->step_tiles = so[n];
+    so.insert(so.end(), sg.begin(), sg.end());
+    if (dalloc(&b->d_step[0], (size_t)n) || dalloc(&b->d_step[1], (size_t)n) || dalloc(&b->d_step_off, so.size()))
+      return fail(CLIFFS_ERR_NOMEM);
+    if (cudaMemcpy(b->d_step[0], sa[0].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(b->d_step[1], sa[1].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(b->d_step_off, so.data(), so.size() * sizeof(int), cudaMemcpyHostToDevice))
+      return fail(CLIFFS_ERR_CUDA);
   }
   b->plan.mode = b->max_ctas > 0 ? CLIFFS_BATCH_PERSISTENT : CLIFFS_BATCH_GRAPH;
   b->plan.ctas_per_sm = std::max(1, b->max_ctas);
@@ -3005,6 +3041,41 @@ static int batch_launch_phases(cliffs_batch* b, int steps, bool fold) {
   return cudaGetLastError() == cudaSuccess ? CLIFFS_OK : CLIFFS_ERR_CUDA;
 }
 
+// Whether the graph plan runs whole steps in one kernel: plans of one tile
+// per list entry (the shape of the sweeps' lists means nothing to it).
+static bool batch_whole(const cliffs_batch* b) {
+  return b->d_step[0] && b->plan.x_rows <= 1 && b->plan.y_groups <= 1;
+}
+
+static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
+  const BatchStep B{b->d_step[odd], b->d_step_off, b->d_step_off + b->ctx.size() + 1, (int)b->ctx.size()};
+  const StepCtl C{S.wait_ns, S.extra, odd};
+  const unsigned g = (unsigned)b->step_tiles;
+  if (b->step_geo == GEO_FLAT)
+    batch_step_kernel<GEO_FLAT, GEO_FLAT><<<g, kStepThreads, 0, b->stream>>>(B, C);
+  else if (b->step_geo == GEO_METRIC)
+    batch_step_kernel<GEO_METRIC, GEO_METRIC><<<g, kStepThreads, 0, b->stream>>>(B, C);
+  else
+    batch_step_kernel<GEO_TABLE, GEO_TABLE><<<g, kStepThreads, 0, b->stream>>>(B, C);
+  ++b->launches;
+  return cudaGetLastError() == cudaSuccess ? CLIFFS_OK : CLIFFS_ERR_CUDA;
+}
+
+// Steps that fold the previous step's end state in: whole steps in pairs, so
+// that the state ends in the copy it started from, and a launch per sweep for
+// what is left.
+static int batch_launch_steps(cliffs_batch* b, int steps) {
+  if (batch_whole(b))
+    for (; steps >= 2; steps -= 2)
+      for (int odd = 0; odd < 2; ++odd) RET(batch_launch_whole(b, odd, StageCtl{kBarrierNs, 0u}));
+  return steps > 0 ? batch_launch_phases(b, steps, true) : CLIFFS_OK;
+}
+
+// The launches of batch_launch_steps.
+static int64_t batch_step_launches(const cliffs_batch* b, int steps) {
+  return batch_whole(b) ? steps / 2 * 2 + steps % 2 * 2 : 2 * (int64_t)steps;
+}
+
 static int batch_build_graph(cliffs_batch* b, int slot, int steps) {
   if (b->graph[slot]) {
     cudaGraphExecDestroy(b->graph[slot]);
@@ -3014,7 +3085,7 @@ static int batch_build_graph(cliffs_batch* b, int slot, int steps) {
   const int64_t before = b->launches;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  const int r = batch_launch_phases(b, steps, true);
+  const int r = batch_launch_steps(b, steps);
   const cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   b->launches = before;  // captured, not launched
   if (r || e != cudaSuccess) {
@@ -3121,10 +3192,10 @@ int cliffs_batch_step(cliffs_batch* b, int32_t nsteps) {
       const int slot = len == k ? 0 : 1;
       if (b->graph_built[slot] != len) r = batch_build_graph(b, slot, len);
       if (!r && cudaGraphLaunch(b->graph[slot], b->stream) != cudaSuccess) r = CLIFFS_ERR_CUDA;
-      b->launches += 2 * (int64_t)len;
+      b->launches += batch_step_launches(b, len);
       done += len;
     }
-    if (!r && done < nsteps) r = batch_launch_phases(b, nsteps - done, true);
+    if (!r && done < nsteps) r = batch_launch_steps(b, nsteps - done);
     if (cudaStreamSynchronize(b->stream) != cudaSuccess && !r) r = CLIFFS_ERR_CUDA;
   }
   if (!r)
@@ -3231,6 +3302,20 @@ int cliffs_batch_check_barrier_timeout(cliffs_batch* b, int32_t wait_ms) {
     for (cliffs_ctx* c : b->ctx)
       if (cudaMemsetAsync(c->status, 0, sizeof(unsigned), b->stream) != cudaSuccess) return CLIFFS_ERR_CUDA;
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return CLIFFS_ERR_CUDA;
+    if (!flags[1]) return CLIFFS_OK;
+  }
+  if (b->d_step[0]) {
+    // and the window waits of a batched whole step, which leaves before its
+    // first store
+    RET(batch_launch_whole(b, 0, StageCtl{B.wait_ns, 16u}));
+    flags[1] = 0;
+    for (cliffs_ctx* c : b->ctx) {
+      unsigned st = 0;
+      CK(cudaMemcpyAsync(&st, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost, b->stream));
+      CK(cudaMemsetAsync(c->status, 0, sizeof(unsigned), b->stream));
+      CK(cudaStreamSynchronize(b->stream));
+      flags[1] |= st & ST_STALL;
+    }
   }
   return flags[1] ? CLIFFS_ERR_TIMEOUT : CLIFFS_OK;
 }

@@ -38,6 +38,7 @@
 // SM 50.8 us (spills); tiles of 32 columns 48.9 us; the max-wave update on the
 // outputs, in the y phase, 49.5 us.
 #pragma once
+#include "batch.cuh"
 #include "staged.cuh"
 
 namespace cliffs {
@@ -481,7 +482,7 @@ __device__ __forceinline__ bool at_rest(unsigned near, float H, float u, float v
 template <int GX>
 __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst* sK, float* sm, int r0, int c0,
                                              uint16_t* s_list, unsigned* s_n, bool& bad) {
-  const Phys<float>& p = X.ph;
+  const Phys<float> p = X.ph;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // a quarter warp takes 4 segments of 2 neighbouring rows; the warp, all
   // segments of its rows
@@ -675,7 +676,7 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
 template <int GY>
 __device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst* sK, const float* sm, int r0, int c0,
                                              uint16_t* s_list, unsigned* s_n, bool& bad) {
-  const Phys<float>& p = Y.ph;
+  const Phys<float> p = Y.ph;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int part = kStepW == 64 ? warp : 2 * warp + (lane >> 4);  // of four, 8 rows each
   const int c = 2 * (kStepW == 64 ? lane : lane & 15), L = c0 + c + 1, n = Y.n;
@@ -986,6 +987,51 @@ __global__ void __launch_bounds__(kStepThreads, kStepBlocks)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int by = C.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
   step_tile<GX, GY>(X, Y, M, by * kStepR, (int)blockIdx.x * kStepW, C, S);
+}
+
+// One whole step of many grids (batch.cuh): a block per tile of the list of
+// all scenarios' tiles, the scenario found by bisection, its arguments staged
+// in shared memory and its tensor maps read from device memory.  24 scenarios
+// of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with its uploads
+// and maxima: 7.0 ms, from 12.2 with a launch per sweep phase.
+struct StepArgs {
+  SweepArgs X, Y;
+  PairPair K;
+  StepMaps M;
+};
+
+struct BatchStep {
+  const StepArgs* args;  // per scenario, for the state copy that the step reads
+  const int* off;        // first tile of a scenario; [n] the total
+  const int* gx;         // tiles across a scenario
+  int n;
+};
+
+template <int GX, int GY>
+__global__ void __launch_bounds__(kStepThreads, kStepBlocks) batch_step_kernel(const BatchStep B, const StepCtl C) {
+  __shared__ StepShared S;
+  __shared__ SweepArgs sA[2];
+  const int tid = threadIdx.x;
+  // every other step takes the tiles last to first, as step_kernel its bands
+  const int tile = C.flip ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
+  const int k = batch_scenario(B.off, B.n, tile);
+  const StepArgs* A = B.args + k;
+  const int local = tile - __ldg(B.off + k), g = __ldg(B.gx + k);
+  static_assert(sizeof(SweepArgs) % 8 == 0 && sizeof(PairPair) % 8 == 0, "copied in 8-byte words");
+  const auto copy = [&](void* to, const void* from, int bytes) {
+    for (int w = tid; w < bytes / 8; w += kStepThreads)
+      reinterpret_cast<unsigned long long*>(to)[w] = __ldg(reinterpret_cast<const unsigned long long*>(from) + w);
+  };
+  copy(&sA[0], &A->X, sizeof(SweepArgs));
+  copy(&sA[1], &A->Y, sizeof(SweepArgs));
+  copy(S.k, &A->K, sizeof(PairPair));
+  if (tid == 0) {
+    mbar_init(&S.bar, 1);
+    S.n[0] = S.n[1] = S.scans = 0u;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  step_tile<GX, GY>(sA[0], sA[1], A->M, local / g * kStepR, local % g * kStepW, C, S);
 }
 
 }  // namespace cliffs

@@ -77,11 +77,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
-// The box of a 2-D tensor map at (x, y) into L2.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
-}
-
 // The box of a 2-D tensor map at (x, y) from shared src (128-byte aligned),
 // into a bulk-async group; elements outside the tensor are not written.  x
 // times the element size must be a multiple of 16 bytes and x, y >= 0.

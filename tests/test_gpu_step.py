@@ -85,3 +85,22 @@ def test_contexts_in_turn():
             g.step(18)
     for x, y in zip(a, b):
         _same(x, y)
+
+
+@pytest.mark.parametrize("metrics", [("plane", "plane", "plane"), ("sphere", "plane", "sphere"),
+                                     ("plane", "stretched", "sphere")])
+def test_batched_whole_steps_match_sweeps(metrics):
+    """Uneven grids in one batch, by steps of odd and even length."""
+    sizes = [(3, 40), (65, 31), (190, 97)]
+    cs = [_case(nx, ny, m, nx) for (nx, ny), m in zip(sizes, metrics)]
+    a, b = [_grid(c, cg.TILED) for c in cs], [_grid(c, cg.DIRECT) for c in cs]
+    batch = pkg.Batch(a)
+    for graph_steps in (8, 5):
+        batch.set_plan(cg.GRAPH, graph_steps=graph_steps)
+        for steps in (21, 2, 7):
+            batch.step(steps)
+            for g in b:
+                g.step(steps)
+    for x, y in zip(a, b):
+        _same(x, y)
+    batch.close()
