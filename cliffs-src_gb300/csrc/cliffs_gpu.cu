@@ -18,6 +18,7 @@
 #include "staged.cuh"
 #include "ytile.cuh"
 #include "step.cuh"
+#include "line.cuh"
 #include "depth_ssl.cuh"
 #include "boundary.cuh"
 
@@ -874,6 +875,50 @@ int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl&
   CK(step_launch(c, &cfg, A.X, A.Y, A.M, C, A.K));
   c->cur = 1 - s;
   c->sweeps += 2u;
+  return CLIFFS_OK;
+}
+
+// Whether the steps of a one-dimensional grid run many to a launch
+// (line_kernel): lines that a cluster holds a cell to a thread (7648 cells),
+// without forcing; the tiled kernels in their own block shapes, outside the
+// per-sweep profile and rising sources.
+bool line_applies(const cliffs_ctx* c) {
+  return c->xrun != c->yrun && (c->xrun ? c->nx : c->ny) <= kLineCluster * kLineCells &&
+         c->sweep_kind == CLIFFS_SWEEP_TILED && c->blk_x == 128 && c->warps_y == 4 && !c->prof && !c->feed_on &&
+         !c->rise_on;
+}
+
+// `steps` steps in one launch; the state stays in the copy it is in.
+int launch_line(cliffs_ctx* c, int steps) {
+  SweepArgs A = sweep_args(c, c->xrun ? 1 : 2, true, c->cur);
+  A.srf_o = c->srf[c->cur];
+  A.xu_o = c->xu[c->cur];
+  A.yv_o = c->yv[c->cur];
+  // blocks of about kLineBlock threads: more blocks shorten a step until the
+  // cluster is at its largest
+  int blocks = 1;
+  while (blocks < kLineCluster && (A.n + blocks - 1) / blocks + 2 * kLineAgain > kLineBlock) blocks *= 2;
+  const int m = (A.n + blocks - 1) / blocks;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)((m + 2 * kLineAgain + 31) / 32 * 32));
+  cfg.stream = c->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  ++c->launches;
+  if (c->xrun)
+    CK((cudaLaunchKernelEx(&cfg, line_kernel<0, false>, A, m, steps)));
+  else if (c->scl_y)
+    CK((cudaLaunchKernelEx(&cfg, line_kernel<1, true>, A, m, steps)));
+  else
+    CK((cudaLaunchKernelEx(&cfg, line_kernel<1, false>, A, m, steps)));
+  c->sweeps += (unsigned)steps;
+  c->max_pending = false;
+  c->max_fresh = false;
   return CLIFFS_OK;
 }
 
@@ -1948,7 +1993,7 @@ static int graph_steps(cliffs_ctx* c, int nsteps, double* t, int32_t* steps_done
 int cliffs_gpu_prepare_steps(cliffs_ctx* c, int32_t nsteps) {
   if (!c || nsteps < 0) return CLIFFS_ERR_ARG;
   if (!c->have_state) return CLIFFS_ERR_STATE;
-  if (!plain_graphs_apply(c)) return CLIFFS_OK;
+  if (!plain_graphs_apply(c) || line_applies(c)) return CLIFFS_OK;
   // the graphs cliffs_gpu_step(nsteps) would replay; a fresh state's first
   // step runs alone
   const bool fresh = c->max_fresh;
@@ -2019,6 +2064,16 @@ int cliffs_gpu_step(cliffs_ctx* c, int32_t nsteps, double* t, int32_t* steps_don
   if (!c->have_state) return CLIFFS_ERR_STATE;
   if (steps_done) *steps_done = 0;
   int done = 0;
+  if (line_applies(c)) {
+    // bounded launches: a few milliseconds each
+    for (int len; done < nsteps; done += len) {
+      len = std::min(nsteps - done, 4096);
+      RET(launch_line(c, len));
+      for (int s = 0; s < len; ++s) *t = *t + c->dt;
+      if (steps_done) *steps_done = done + len;
+    }
+    return CLIFFS_OK;
+  }
   if (c->max_fresh && nsteps > 0) {
     // the first step from a fresh state folds nothing into the max-wave
     // fields; the graphs' steps all fold in the previous step's end state
