@@ -98,6 +98,9 @@ int make_map(CUtensorMap* m, const float* base, int nx, int ny, int pitch, int b
 
 }  // namespace
 
+// The tiles of whole steps (step.cuh).
+enum { STEP_LARGE = 0, STEP_SMALL = 1, STEP_TINY = 2 };
+
 struct cliffs_ctx {
   // one device allocation holding the per-grid arrays (dep, the state
   // copies, the max-wave fields, geometry, status words, worklist, edge
@@ -178,8 +181,11 @@ struct cliffs_ctx {
   bool ytile_ok = false;
   // the window maps of step_kernel (whole steps of the tiled kernels when
   // step_ok)
-  CUtensorMap w_dep, w_srf[2], w_xu[2], w_yv[2];
+  struct WindowMaps {
+    CUtensorMap dep, srf[2], xu[2], yv[2];
+  } win[2];  // StepLarge's; StepSmall's and StepTiny's
   bool step_ok = false;
+  int step_size = STEP_LARGE;  // the tile of the grid's whole steps
   int grid_sx = 0, grid_sy = 0;  // resident blocks of staged_x / staged_y
   unsigned long long stage_ns = 2000000000ull;  // limit of one stage wait
   // fast-kernel sweeps launched as programmatic dependents of the previous
@@ -509,6 +515,30 @@ __global__ void k_feed_child(int mm, int nn, int W_nx, int E_nx, int S_ny, int N
   }
 }
 
+// Tiles of a grid in whole steps.
+template <class T>
+int tiles_of(int nx, int ny) {
+  return ((nx + T::W - 1) / T::W) * ((ny + T::R - 1) / T::R);
+}
+int step_tiles(int size, int nx, int ny) {
+  return size == STEP_LARGE   ? tiles_of<StepLarge>(nx, ny)
+         : size == STEP_SMALL ? tiles_of<StepSmall>(nx, ny)
+                              : tiles_of<StepTiny>(nx, ny);
+}
+// The tile for grids of so many large, and of so many tiny tiles in all.  As
+// long as all large tiles are on the chip at once, a step lasts as long as its
+// slowest block: smaller tiles, which the phases cross in half the time, and
+// which as long as they all fit too have every row that the full rules read in
+// the window.  Measured, us per step (large, small, tiny): 256 x 256 14.0,
+// 10.8, 10.7; 400 x 400 13.5, 11.2, 11.1; 600 x 600 (1140 tiny tiles) 15.2,
+// 16.9, 13.7; 800 x 600 (1500) 17.1, 14.4, 16.4; 1201 x 903 (589 large ones)
+// 26.3, 23.9, 26.8; 1500 x 1500 (1200) 31.9, 33.8, 39.1.
+int step_size(int64_t large, int64_t tiny, int sms) {
+  return large > (int64_t)sms * StepLarge::Blocks ? STEP_LARGE
+         : tiny > (int64_t)sms * StepTiny::Blocks ? STEP_SMALL
+                                                  : STEP_TINY;
+}
+
 int check_device(int* dev) {
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) return CLIFFS_ERR_DEVICE;
@@ -830,7 +860,7 @@ PairConst pair_const(const SweepArgs& A) {
 }
 
 // The arguments of one whole step from state copy s to 1 - s.
-StepArgs step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey) {
+StepArgs step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey, int size) {
   StepArgs A;
   A.X = sweep_args(c, 1, false, s);
   A.X.hmax_in = c->hmax;
@@ -839,40 +869,41 @@ StepArgs step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey)
   A.Y = sweep_args(c, 2, false, s);
   A.Y.edges = ey;
   A.K = PairPair{pair_const(A.X), pair_const(A.Y)};
-  A.M = StepMaps{c->w_dep, c->w_srf[s], c->w_xu[s], c->w_yv[s]};
+  const auto& W = c->win[size == STEP_LARGE ? 0 : 1];
+  A.M = StepMaps{W.dep, W.srf[s], W.xu[s], W.yv[s]};
   return A;
-}
-
-dim3 step_grid(const cliffs_ctx* c) {
-  return dim3((c->nx + kStepW - 1) / kStepW, (c->ny + kStepR - 1) / kStepR);
 }
 
 // The variant for the grid's spacing: a table when an axis is not uniform,
 // else uniform spacing with or without the metric term.
-template <typename... Args>
-cudaError_t step_launch(const cliffs_ctx* c, const cudaLaunchConfig_t* cfg, Args... args) {
-  if (!c->geo_uni_x || !c->geo_uni_y) return cudaLaunchKernelEx(cfg, step_kernel<GEO_TABLE, GEO_TABLE>, args...);
-  if (c->scl_y || c->lscale) return cudaLaunchKernelEx(cfg, step_kernel<GEO_METRIC, GEO_METRIC>, args...);
-  return cudaLaunchKernelEx(cfg, step_kernel<GEO_FLAT, GEO_FLAT>, args...);
+template <class T>
+cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepArgs& A, const StepCtl& C) {
+  cfg.gridDim = dim3((c->nx + T::W - 1) / T::W, (c->ny + T::R - 1) / T::R);
+  cfg.blockDim = dim3(T::Threads);
+  if (!c->geo_uni_x || !c->geo_uni_y)
+    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_TABLE, GEO_TABLE>, A.X, A.Y, A.M, C, A.K);
+  if (c->scl_y || c->lscale)
+    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_METRIC, GEO_METRIC>, A.X, A.Y, A.M, C, A.K);
+  return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_FLAT, GEO_FLAT>, A.X, A.Y, A.M, C, A.K);
 }
 
 // One whole step on the context's stream, folding the previous step's end
 // state into the max-wave fields; ex, ey: the edge tables of a forced step.
 int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
   const int s = c->cur;
-  const StepArgs A = step_args(c, s, ex, ey);
+  const StepArgs A = step_args(c, s, ex, ey, c->step_size);
   const StepCtl C{S.wait_ns, S.extra, s};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = step_grid(c);
-  cfg.blockDim = dim3(kStepThreads);
   cfg.stream = c->stream;
   cfg.attrs = at;
   cfg.numAttrs = c->pdl ? 1 : 0;
   ++c->launches;
-  CK(step_launch(c, &cfg, A.X, A.Y, A.M, C, A.K));
+  CK(c->step_size == STEP_LARGE   ? step_launch<StepLarge>(c, cfg, A, C)
+     : c->step_size == STEP_SMALL ? step_launch<StepSmall>(c, cfg, A, C)
+                                  : step_launch<StepTiny>(c, cfg, A, C));
   c->cur = 1 - s;
   c->sweeps += 2u;
   return CLIFFS_OK;
@@ -1202,11 +1233,16 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
            !make_map(&c->m_xu16[k], c->xu[k], nx, ny, pp, 32, kYRows) &&
            !make_map(&c->m_yv16[k], c->yv[k], nx, ny, pp, 32, kYRows);
     c->ytile_ok = yt;
-    bool st = ok && c->xrun && c->yrun && !make_map(&c->w_dep, c->dep, nx, ny, pp, kStepWin, kStepRows);
-    for (int k = 0; k < 2 && st; ++k)
-      st = !make_map(&c->w_srf[k], c->srf[k], nx, ny, pp, kStepWin, kStepRows) &&
-           !make_map(&c->w_xu[k], c->xu[k], nx, ny, pp, kStepWin, kStepRows) &&
-           !make_map(&c->w_yv[k], c->yv[k], nx, ny, pp, kStepWin, kStepRows);
+    bool st = ok && c->xrun && c->yrun;
+    for (int w = 0; w < 2 && st; ++w) {
+      const int bx = w ? StepSmall::Win : StepLarge::Win, by = w ? StepSmall::Rows : StepLarge::Rows;
+      auto& W = c->win[w];
+      st = !make_map(&W.dep, c->dep, nx, ny, pp, bx, by);
+      for (int k = 0; k < 2 && st; ++k)
+        st = !make_map(&W.srf[k], c->srf[k], nx, ny, pp, bx, by) && !make_map(&W.xu[k], c->xu[k], nx, ny, pp, bx, by) &&
+             !make_map(&W.yv[k], c->yv[k], nx, ny, pp, bx, by);
+    }
+    c->step_size = step_size(step_tiles(STEP_LARGE, nx, ny), step_tiles(STEP_TINY, nx, ny), nsm);
     c->step_ok = st && cells < (1ull << 30);  // its stores take 32-bit byte offsets
     c->grid_sx = nsm * bx;
     c->grid_sy = nsm * by;
@@ -2837,6 +2873,7 @@ struct cliffs_batch {
   int* d_step_off = nullptr;  // n + 1 offsets, then n tiles across
   int step_tiles = 0;
   int step_geo = GEO_FLAT;
+  int step_size = STEP_LARGE;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
   // groups, column groups); the list of a plan's tile shape is built from them
   std::vector<int> tx, ty, lx, ly;
@@ -2990,12 +3027,19 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
     std::vector<StepArgs> sa[2];
     std::vector<int> so((size_t)n + 1, 0), sg;
     bool uniform = true, plain = true;
+    int64_t large = 0, tiny = 0;
+    for (int k = 0; k < n; ++k) {
+      large += step_tiles(STEP_LARGE, ctxs[k]->nx, ctxs[k]->ny);
+      tiny += step_tiles(STEP_TINY, ctxs[k]->nx, ctxs[k]->ny);
+    }
+    b->step_size = step_size(large, tiny, b->sms);
     for (int k = 0; k < n; ++k) {
       const cliffs_ctx* c = ctxs[k];
-      for (int q = 0; q < 2; ++q) sa[q].push_back(step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr));
-      const dim3 g = step_grid(c);
-      so[k + 1] = so[k] + (int)(g.x * g.y);
-      sg.push_back((int)g.x);
+      for (int q = 0; q < 2; ++q)
+        sa[q].push_back(step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr, b->step_size));
+      so[k + 1] = so[k] + step_tiles(b->step_size, c->nx, c->ny);
+      const int w = b->step_size == STEP_LARGE ? StepLarge::W : StepSmall::W;
+      sg.push_back((c->nx + w - 1) / w);
       uniform = uniform && c->geo_uni_x && c->geo_uni_y;
       plain = plain && !c->scl_y && !c->lscale;
     }
@@ -3102,16 +3146,26 @@ static bool batch_whole(const cliffs_batch* b) {
   return b->d_step[0] && b->plan.x_rows <= 1 && b->plan.y_groups <= 1;
 }
 
+template <class T>
+static void batch_step_launch(cliffs_batch* b, const BatchStep& B, const StepCtl& C) {
+  const unsigned g = (unsigned)b->step_tiles;
+  if (b->step_geo == GEO_FLAT)
+    batch_step_kernel<T, GEO_FLAT, GEO_FLAT><<<g, T::Threads, 0, b->stream>>>(B, C);
+  else if (b->step_geo == GEO_METRIC)
+    batch_step_kernel<T, GEO_METRIC, GEO_METRIC><<<g, T::Threads, 0, b->stream>>>(B, C);
+  else
+    batch_step_kernel<T, GEO_TABLE, GEO_TABLE><<<g, T::Threads, 0, b->stream>>>(B, C);
+}
+
 static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
   const BatchStep B{b->d_step[odd], b->d_step_off, b->d_step_off + b->ctx.size() + 1, (int)b->ctx.size()};
   const StepCtl C{S.wait_ns, S.extra, odd};
-  const unsigned g = (unsigned)b->step_tiles;
-  if (b->step_geo == GEO_FLAT)
-    batch_step_kernel<GEO_FLAT, GEO_FLAT><<<g, kStepThreads, 0, b->stream>>>(B, C);
-  else if (b->step_geo == GEO_METRIC)
-    batch_step_kernel<GEO_METRIC, GEO_METRIC><<<g, kStepThreads, 0, b->stream>>>(B, C);
+  if (b->step_size == STEP_LARGE)
+    batch_step_launch<StepLarge>(b, B, C);
+  else if (b->step_size == STEP_SMALL)
+    batch_step_launch<StepSmall>(b, B, C);
   else
-    batch_step_kernel<GEO_TABLE, GEO_TABLE><<<g, kStepThreads, 0, b->stream>>>(B, C);
+    batch_step_launch<StepTiny>(b, B, C);
   ++b->launches;
   return cudaGetLastError() == cudaSuccess ? CLIFFS_OK : CLIFFS_ERR_CUDA;
 }

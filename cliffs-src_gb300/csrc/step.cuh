@@ -3,14 +3,13 @@
 //
 // A sweep per launch moves the state through memory twice a step: 72 bytes a
 // cell, and each cell's window is loaded, classified and converted once per
-// sweep.  Here a block takes a tile of kStepW columns x kStepR rows with one
+// sweep.  Here a block takes a tile of 64 columns x 30 rows (StepLarge) with one
 // halo row on each side (the y-sweep's), brings it into shared memory with
 // tensor-map copies, sweeps its rows in place, then its columns out of the
 // swept tile straight to the other copy of the state: 44 bytes a cell, the
 // max-wave fold included.
 //
-// Both sweeps march: a thread owns two lines of a sweep (two rows kStepPair
-// apart in the x phase, two adjacent columns in the y phase) over 8 cells and
+// Both sweeps march: a thread owns two lines of a sweep (two rows 16 apart in the x phase, two adjacent columns in the y phase) over 8 cells and
 // carries the last cell and the last face's flux along, so that every celerity
 // is computed 10/8 and every face flux 9/8 times a cell (6/4 and 5/4 in
 // fast_kernel).  The two lines are the two halves of packed FP32 operations
@@ -43,22 +42,36 @@
 
 namespace cliffs {
 
-constexpr int kStepW = 64;                 // columns of a tile (32 or 64)
-constexpr int kStepThreads = 2 * kStepW;
-constexpr int kStepBlocks = 512 / kStepThreads;  // per SM: 128 registers a thread
-constexpr int kStepRows = 32;          // rows of its window
-constexpr int kStepR = kStepRows - 2;  // rows of a tile
-constexpr int kStepPair = 16;          // rows between the two lines of an x thread
-// columns of the window: one 16-byte chunk on the left, two on the right (the
-// second unused): rows of an odd number of 16-byte chunks, so that the x
-// phase's 16-byte accesses (2 rows x 4 segments a quarter warp) meet no bank
-// conflicts
-constexpr int kStepWin = kStepW + 12;
-constexpr int kStepField = kStepRows * kStepWin;  // floats of one field of the window
-constexpr uint32_t kStepBytes = 4u * kStepField * 4u;
+// A tile of W columns, in a window of ROWS rows with HALO of them on each side
+// (the y-sweep of a plain cell reads one, the full rules three); a thread of
+// either phase marches SEG cells of two lines.  INPLACE: the rows are swept in
+// place; else into fields of their own, so that the x phase's listed cells find
+// their input in the window.
+template <int W_, int ROWS_, int HALO_, int SEG_, bool INPLACE_>
+struct StepTile {
+  static constexpr int W = W_, Rows = ROWS_, Halo = HALO_, Seg = SEG_;
+  static constexpr bool InPlace = INPLACE_;
+  static constexpr int R = Rows - 2 * Halo;  // rows of the tile
+  static constexpr int Part = (R + 3) / 4;   // rows of a thread of the y phase
+  static constexpr int Pair = Rows / 2;      // rows between the two lines of an x thread
+  static constexpr int Threads = Pair * (W / Seg);
+  static constexpr int Blocks = 512 / Threads;  // per SM: 128 registers a thread
+  // columns of the window: one 16-byte chunk on the left, two on the right (the
+  // second unused): rows of an odd number of 16-byte chunks, so that the x
+  // phase's accesses (2 rows x 4 segments a quarter warp) spread over the banks
+  static constexpr int Win = W + 12;
+  static constexpr int Field = Rows * Win;             // floats of one field of the window
+  static constexpr int Out = InPlace ? 0 : 3 * Field;  // from a field of the input to the swept one
+  static constexpr int Floats = (InPlace ? 4 : 7) * Field;
+  static constexpr uint32_t Bytes = 4u * Field * 4u;   // of the window's copies
+  static_assert(W / Seg == 8 && Threads == 2 * W, "8 segments of a row, 4 parts of a column pair");
+};
+using StepLarge = StepTile<64, 32, 1, 8, true>;
+using StepSmall = StepTile<32, 16, 1, 4, false>;
+using StepTiny = StepTile<32, 16, 3, 4, false>;
 
 struct StepMaps {
-  CUtensorMap dep, srf, xu, yv;  // the input copy's fields, a kStepWin x kStepRows box
+  CUtensorMap dep, srf, xu, yv;  // the input copy's fields, a Win x Rows box
 };
 
 // ---- two FP32 lanes in a 64-bit register ---------------------------------------
@@ -264,7 +277,7 @@ __device__ __forceinline__ unsigned take_sign(unsigned mask, unsigned x) { retur
 // neighbour.  Returns false when general_cell has to decide: the cell or a
 // neighbour of it is flooded, or a remainder of water or velocity lies on land
 // with no wet cell in reach.
-__device__ __forceinline__ bool shore_cell(const RawCell<float> (&w)[5], int o, int n, const LineCtx<float>& C,
+__device__ __forceinline__ bool shore_cell(const RawCell<float>* w, int o, int n, const LineCtx<float>& C,
                                            const Geo<float>& g, const Phys<float>& p, OutCell<float>& out) {
   float H[5], E[5];
   bool wet[5];
@@ -383,75 +396,93 @@ __device__ __forceinline__ LineCtx<float> y_line(const SweepArgs& Y, int L, int 
   return C;
 }
 
-// step_y_value's full rules: the raw cells o-3 .. o+3, those outside the
-// window swept again from the step's input.
-__device__ __noinline__ OutCell<float> step_y_general(const SweepArgs& X, const SweepArgs& Y, const float* sm, int r0,
-                                                      int c0, int t, int c, bool& scan) {
-  const int o = r0 + t, L = c0 + c + 1, n = Y.n;
+// The tile cell (t, c) of the x phase from the step's input in the window.
+template <class T>
+__device__ __noinline__ OutCell<float> step_x_window(const SweepArgs& X, const float* sm, int rb, int c0, int t, int c) {
+  const int L = rb + t, i = c0 + c + 1, n = X.n;
   RawCell<float> w[7];
   bool anywet = false;
-#pragma unroll 1
+#pragma unroll
+  for (int q = 0; q < 7; ++q) {
+    const int k = i - 3 + q;
+    const float* f = sm + t * T::Win + 1 + c + q;
+    w[q] = RawCell<float>{f[0], f[T::Field], f[2 * T::Field], f[3 * T::Field], k >= 1 && k <= n};
+    anywet |= w[q].present && depth_of(w[q].s, w[q].d) > X.ph.ground;
+  }
+  float alpha = 1.f, ialpha = 1.f;
+  if (X.lscale) {
+    const float2 a = __ldg(X.lscale + (L - 1));
+    alpha = a.x;
+    ialpha = a.y;
+  }
+  LineCtx<float> C;
+  C.n = n;
+  C.wet = anywet;
+  C.eL = i == 1 ? edge_vals(X, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.eR = i == n ? edge_vals(X, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.inv_dx1 = X.inv_dx1 * ialpha;
+  C.inv_dxn1 = X.inv_dxn1 * ialpha;
+  C.scl1 = C.scln = 0.f;
+  OutCell<float> out;
+  if (shore_cell(w + 1, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, out)) return out;
+  if (!anywet) return step_x_general(X, L, i);  // does the row hold a wet cell elsewhere?
+  Geo<float> g[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) g[q] = geo_at(X, i - 1 + q, alpha, ialpha);
+  return general_cell(w, i, C, g, X.ph);
+}
+
+// The x-swept cell of row o + q - 3 beside cell (t, c) (row o = rb + t) that
+// lies outside the window: swept again from the step's input.
+__device__ __noinline__ RawCell<float> step_y_outside(const SweepArgs& X, int k, int L) {
+  const OutCell<float> x = step_x_value(X, k, L);
+  return RawCell<float>{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
+}
+
+// The y-swept value of tile cell (t, c) (row rb + t, column c0 + c + 1,
+// 1-based) from the x-swept window sm.  scan: the cell keeps a remainder of
+// water or velocity with no wet cell in reach, and whether its column holds
+// one elsewhere decides (cliffs.f:113); nothing is returned then.
+template <class T>
+__device__ __noinline__ OutCell<float> step_y_value(const SweepArgs& X, const SweepArgs& Y, const float* sm, int rb,
+                                                    int c0, int t, int c, bool& scan) {
+  const int o = rb + t, L = c0 + c + 1, n = Y.n;
+  const float ground = Y.ph.ground;
+  scan = false;
+  RawCell<float> w[7];
+  bool have[7];
+#pragma unroll
   for (int q = 0; q < 7; ++q) {
     const int k = o - 3 + q, tt = t - 3 + q;
-    RawCell<float> r{0.f, 0.f, 0.f, 0.f, false};
-    if (k >= 1 && k <= n) {
-      if (tt >= 0 && tt < kStepRows) {
-        const float* f = sm + tt * kStepWin + 4 + c;
-        r = RawCell<float>{f[0], f[kStepField], f[3 * kStepField], f[2 * kStepField], true};
-      } else {
-        const OutCell<float> x = step_x_value(X, k, L);
-        r = RawCell<float>{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
-      }
-      anywet |= depth_of(r.s, r.d) > Y.ph.ground;
+    w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
+    have[q] = k < 1 || k > n || (tt >= 0 && tt < T::Rows);
+    if (k >= 1 && k <= n && have[q]) {
+      const float* f = sm + tt * T::Win + 4 + c;
+      w[q] = RawCell<float>{f[0], f[T::Field + T::Out], f[3 * T::Field + T::Out], f[2 * T::Field + T::Out], true};
     }
-    w[q] = r;
   }
-  scan = !anywet && !(depth_of(w[3].s, w[3].d) == 0.f && w[3].u == 0.f && w[3].v == 0.f);
-  if (scan) return OutCell<float>{w[3].s, w[3].u, w[3].v};
+  // a cell two rows away and outside the window matters to a wet cell beside a
+  // land neighbour, and to a remainder on land
+  const bool rest = w[3].u == 0.f && w[3].v == 0.f && depth_of(w[3].s, w[3].d) == 0.f;
+  if (!have[1] && !rest && !(depth_of(w[2].s, w[2].d) > ground)) w[1] = step_y_outside(X, o - 2, L);
+  if (!have[5] && !rest && !(depth_of(w[4].s, w[4].d) > ground)) w[5] = step_y_outside(X, o + 2, L);
   LineCtx<float> C = y_line(Y, L, o);
+  OutCell<float> out;
+  if (shore_cell(w + 1, o, n, C, geo_at(Y, o, 1.f, 1.f), Y.ph, out)) return out;
+  // the full rules: all cells o-3 .. o+3
+#pragma unroll
+  for (int q = 0; q < 7; ++q)
+    if (!have[q] && !w[q].present) w[q] = step_y_outside(X, o - 3 + q, L);
+  bool anywet = false;
+#pragma unroll
+  for (int q = 0; q < 7; ++q) anywet |= w[q].present && depth_of(w[q].s, w[q].d) > ground;
+  scan = !anywet && !rest;
+  if (scan) return OutCell<float>{w[3].s, w[3].u, w[3].v};
   C.wet = anywet;
   Geo<float> g[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q) g[q] = geo_at(Y, o - 1 + q, 1.f, 1.f);
   return general_cell(w, o, C, g, Y.ph);
-}
-
-// The y-swept value of tile cell (t, c) (row r0 + t, column c0 + c + 1,
-// 1-based) from the x-swept window sm.  scan: the cell keeps a remainder of
-// water or velocity with no wet cell in reach, and whether its column holds
-// one elsewhere decides (cliffs.f:113); nothing is returned then.
-__device__ __noinline__ OutCell<float> step_y_value(const SweepArgs& X, const SweepArgs& Y, const float* sm, int r0,
-                                                    int c0, int t, int c, bool& scan) {
-  const int o = r0 + t, L = c0 + c + 1, n = Y.n;
-  scan = false;
-  RawCell<float> w[5];
-  bool have[5];
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    const int k = o - 2 + q, tt = t - 2 + q;
-    w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
-    have[q] = k < 1 || k > n || (tt >= 0 && tt < kStepRows);
-    if (k >= 1 && k <= n && have[q]) {
-      const float* f = sm + tt * kStepWin + 4 + c;
-      w[q] = RawCell<float>{f[0], f[kStepField], f[3 * kStepField], f[2 * kStepField], true};
-    }
-  }
-  // an outer cell outside the window matters to a wet cell beside a land
-  // neighbour, and to a remainder on land
-  if (!have[0] || !have[4]) {
-    const bool rest = w[2].u == 0.f && w[2].v == 0.f && depth_of(w[2].s, w[2].d) == 0.f;
-    const int q = have[0] ? 4 : 0, k = o - 2 + q;
-    const RawCell<float>& a = have[0] ? w[3] : w[1];
-    if (!rest && !(depth_of(a.s, a.d) > Y.ph.ground)) {
-      const OutCell<float> x = step_x_value(X, k, L);
-      const RawCell<float> r{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
-      if (have[0]) w[4] = r;
-      else w[0] = r;
-    }
-  }
-  OutCell<float> out;
-  if (shore_cell(w, o, n, y_line(Y, L, o), geo_at(Y, o, 1.f, 1.f), Y.ph, out)) return out;
-  return step_y_general(X, Y, sm, r0, c0, t, c, scan);
 }
 
 __device__ __forceinline__ void courant_status(const SweepArgs& A, float cour) {
@@ -479,31 +510,30 @@ __device__ __forceinline__ bool at_rest(unsigned near, float H, float u, float v
   return (near & 7u) == 0u && H == 0.f && u == 0.f && v == 0.f;
 }
 
-template <int GX>
-__device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst* sK, float* sm, int r0, int c0,
+template <class T, int GX>
+__device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst* sK, float* sm, int rb, int c0,
                                              uint16_t* s_list, unsigned* s_n, bool& bad) {
   const Phys<float> p = X.ph;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // a quarter warp takes 4 segments of 2 neighbouring rows; the warp, all
   // segments of its rows
-  constexpr int kPairs = 256 / kStepW;  // row pairs of a warp
   const int q4 = lane >> 3;
-  const int seg = (lane & 3) | (kStepW == 64 ? (q4 & 1) * 4 : 0);
-  const int tA = warp * kPairs + (kStepW == 64 ? q4 >> 1 : q4) * 2 + ((lane >> 2) & 1), tB = tA + kStepPair;
-  const int n = X.n, k0 = c0 + 8 * seg + 1;
-  float* rowA = sm + tA * kStepWin + 4 + 8 * seg;
-  float* rowB = rowA + kStepPair * kStepWin;
+  const int seg = (lane & 3) | (q4 & 1) * 4;
+  const int tA = warp * 4 + (q4 >> 1) * 2 + ((lane >> 2) & 1), tB = tA + T::Pair;
+  const int n = X.n, k0 = c0 + T::Seg * seg + 1;
+  float* rowA = sm + tA * T::Win + 4 + T::Seg * seg;
+  float* rowB = rowA + T::Pair * T::Win;
   // the halo cells, before a neighbouring segment's results replace them
   float hl[8], hr[8];
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
-    hl[2 * f] = rowA[f * kStepField - 1];
-    hl[2 * f + 1] = rowB[f * kStepField - 1];
-    hr[2 * f] = rowA[f * kStepField + 8];
-    hr[2 * f + 1] = rowB[f * kStepField + 8];
+    hl[2 * f] = rowA[f * T::Field - 1];
+    hl[2 * f + 1] = rowB[f * T::Field - 1];
+    hr[2 * f] = rowA[f * T::Field + T::Seg];
+    hr[2 * f + 1] = rowB[f * T::Field + T::Seg];
   }
-  __syncwarp();
-  const int LA = r0 + tA, LB = r0 + tB;  // 1-based rows
+  if (T::InPlace) __syncwarp();
+  const int LA = rb + tA, LB = rb + tB;  // 1-based rows
   const bool swA = LA >= X.lo && LA <= X.hi && k0 <= n, swB = LB >= X.lo && LB <= X.hi && k0 <= n;
   float cour = 0.f;
   if (swA || swB) {
@@ -527,7 +557,7 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
     float cmA = 0.f, cmB = 0.f;       // the largest |u| + c of each line (times dt/(fm+fp) with GEO_TABLE)
     f2 chk = 0ull;                    // 0 * results: NaN when one is not finite
     // every cell of the segment interior, on swept rows
-    const bool inner = swA && swB && k0 >= 2 && k0 + 7 <= n - 1;
+    const bool inner = swA && swB && k0 >= 2 && k0 + T::Seg - 1 <= n - 1;
     March m;
     auto flags = [&](const Cell2& c) {
       const unsigned a = wet_sign(c.H[0], p), b = wet_sign(c.H[1], p);
@@ -569,38 +599,43 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
       f2 ou, ov, cn;
       update2<GX & GEO_DFPM>(m, b.v, qP, qQ, gk, p.ginv, K, os, ou, ov, cn);
       flags(b);
-      float *const fA = rowA + i, *const fB = rowB + i;
+      float *const fA = rowA + T::Out + i, *const fB = rowB + T::Out + i;
       if ((okA & okB & 7u) == 7u && inner && fminf(lo2(cn), hi2(cn)) > 0.f) {
-        fA[kStepField] = os[0];
-        fA[2 * kStepField] = lo2(ou);
-        fA[3 * kStepField] = lo2(ov);
-        fB[kStepField] = os[1];
-        fB[2 * kStepField] = hi2(ou);
-        fB[3 * kStepField] = hi2(ov);
+        fA[T::Field] = os[0];
+        fA[2 * T::Field] = lo2(ou);
+        fA[3 * T::Field] = lo2(ov);
+        fB[T::Field] = os[1];
+        fB[2 * T::Field] = hi2(ou);
+        fB[3 * T::Field] = hi2(ov);
         chk = fma2(pk(os[0], os[1]), 0ull, fma2(ou, 0ull, fma2(ov, 0ull, chk)));
       } else {
         const int k = k0 + i;
         const bool in = k >= 2 && k <= n - 1;
         const bool pA = in && swA && (okA & 7u) == 7u && lo2(cn) > 0.f;
         const bool pB = in && swB && (okB & 7u) == 7u && hi2(cn) > 0.f;
-        if (pA) {
-          fA[kStepField] = os[0];
-          fA[2 * kStepField] = lo2(ou);
-          fA[3 * kStepField] = lo2(ov);
+        // rows that are not swept and land at rest keep their input, which
+        // is in place or copied; the others are listed
+        const bool kA = !swA || at_rest(wetA, m.j.H[0], lo2(m.j.u), lo2(m.j.v));
+        const bool kB = !swB || at_rest(wetB, m.j.H[1], hi2(m.j.u), hi2(m.j.v));
+        const bool wA = pA || (!T::InPlace && kA), wB = pB || (!T::InPlace && kB);
+        const float s0 = pA ? os[0] : m.j.s[0], u0 = pA ? lo2(ou) : lo2(m.j.u), v0 = pA ? lo2(ov) : lo2(m.j.v);
+        const float s1 = pB ? os[1] : m.j.s[1], u1 = pB ? hi2(ou) : hi2(m.j.u), v1 = pB ? hi2(ov) : hi2(m.j.v);
+        if (wA) {
+          fA[T::Field] = s0;
+          fA[2 * T::Field] = u0;
+          fA[3 * T::Field] = v0;
         }
-        if (pB) {
-          fB[kStepField] = os[1];
-          fB[2 * kStepField] = hi2(ou);
-          fB[3 * kStepField] = hi2(ov);
+        if (wB) {
+          fB[T::Field] = s1;
+          fB[2 * T::Field] = u1;
+          fB[3 * T::Field] = v1;
         }
-        // a finite sum of the stored values (0 where none is)
-        const float z = (pA ? os[0] + lo2(ou) + lo2(ov) : 0.f) * 0.f + (pB ? os[1] + hi2(ou) + hi2(ov) : 0.f) * 0.f;
+        // a finite sum of the results (0 where none is)
+        const float z = (pA ? s0 + u0 + v0 : 0.f) * 0.f + (pB ? s1 + u1 + v1 : 0.f) * 0.f;
         bad = bad || z != z;
-        const bool lA = !pA && swA && !at_rest(wetA, m.j.H[0], lo2(m.j.u), lo2(m.j.v));
-        const bool lB = !pB && swB && !at_rest(wetB, m.j.H[1], hi2(m.j.u), hi2(m.j.v));
         if (k <= n) {
-          restA |= (lA ? 1u : 0u) << i;
-          restB |= (lB ? 1u : 0u) << i;
+          restA |= (pA || kA ? 0u : 1u) << i;
+          restB |= (pB || kB ? 0u : 1u) << i;
         }
       }
       float a = add_rn(fabsf(lo2(m.j.u)), lo2(m.j.c)), c = add_rn(fabsf(hi2(m.j.u)), hi2(m.j.c));
@@ -622,12 +657,12 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
       Two t;
       t.d[0] = *reinterpret_cast<const float2*>(rowA + i);
       t.d[1] = *reinterpret_cast<const float2*>(rowB + i);
-      t.s[0] = *reinterpret_cast<const float2*>(rowA + kStepField + i);
-      t.s[1] = *reinterpret_cast<const float2*>(rowB + kStepField + i);
-      t.u[0] = *reinterpret_cast<const float2*>(rowA + 2 * kStepField + i);
-      t.u[1] = *reinterpret_cast<const float2*>(rowB + 2 * kStepField + i);
-      t.v[0] = *reinterpret_cast<const float2*>(rowA + 3 * kStepField + i);
-      t.v[1] = *reinterpret_cast<const float2*>(rowB + 3 * kStepField + i);
+      t.s[0] = *reinterpret_cast<const float2*>(rowA + T::Field + i);
+      t.s[1] = *reinterpret_cast<const float2*>(rowB + T::Field + i);
+      t.u[0] = *reinterpret_cast<const float2*>(rowA + 2 * T::Field + i);
+      t.u[1] = *reinterpret_cast<const float2*>(rowB + 2 * T::Field + i);
+      t.v[0] = *reinterpret_cast<const float2*>(rowA + 3 * T::Field + i);
+      t.v[1] = *reinterpret_cast<const float2*>(rowB + 3 * T::Field + i);
       return t;
     };
     auto first = [&](const Two& t) {
@@ -649,7 +684,7 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
       take(j, inv, qP, qQ);
     }
 #pragma unroll 1
-    for (int i = 0; i < 6; i += 2) {
+    for (int i = 0; i < T::Seg - 2; i += 2) {
       const Two t = load(i + 2);
       const Cell2 c = first(t);
       advance(b, i);
@@ -657,43 +692,52 @@ __device__ __forceinline__ void step_x_phase(const SweepArgs& X, const PairConst
       advance(c, i + 1);
     }
     const Cell2 h = make_cell2<true>(p, K, hr[0], hr[1], hr[2], hr[3], hr[4], hr[5], hr[6], hr[7]);
-    advance(b, 6);
-    advance(h, 7);
+    advance(b, T::Seg - 2);
+    advance(h, T::Seg - 1);
     bad = bad || (swA && lo2(chk) != lo2(chk)) || (swB && hi2(chk) != hi2(chk));
-    list_push(restA, tA * kStepW + 8 * seg, s_list, s_n);
-    list_push(restB, tB * kStepW + 8 * seg, s_list, s_n);
+    list_push(restA, tA * T::W + T::Seg * seg, s_list, s_n);
+    list_push(restB, tB * T::W + T::Seg * seg, s_list, s_n);
     if (GX != GEO_TABLE) {
       cmA *= -lo2(g.ndtx);
       cmB *= -hi2(g.ndtx);
     }
     cour = fmaxf(swA ? cmA : 0.f, swB ? cmB : 0.f);
+  } else if (!T::InPlace) {
+#pragma unroll
+    for (int f = 1; f < 4; ++f)
+#pragma unroll
+      for (int i = 0; i < T::Seg; ++i) {
+        rowA[f * T::Field + T::Out + i] = rowA[f * T::Field + i];
+        rowB[f * T::Field + T::Out + i] = rowB[f * T::Field + i];
+      }
   }
   courant_status(X, cour);
 }
 
 // ---- the y phase ------------------------------------------------------------------
 
-template <int GY>
-__device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst* sK, const float* sm, int r0, int c0,
+template <class T, int GY>
+__device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst* sK, const float* sm, int rb, int c0,
                                              uint16_t* s_list, unsigned* s_n, bool& bad) {
   const Phys<float> p = Y.ph;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int part = kStepW == 64 ? warp : 2 * warp + (lane >> 4);  // of four, 8 rows each
-  const int c = 2 * (kStepW == 64 ? lane : lane & 15), L = c0 + c + 1, n = Y.n;
-  const int t0 = 1 + 8 * part;
-  const int rows = min(min(8, kStepR - 8 * part), n - (r0 + t0) + 1);  // output rows of this thread
+  const int part = T::W == 64 ? warp : 2 * warp + (lane >> 4);  // of four, Part rows each
+  const int c = 2 * (T::W == 64 ? lane : lane & 15), L = c0 + c + 1, n = Y.n;
+  const int t0 = T::Halo + T::Part * part;
+  const int rows = min(min(T::Part, T::R - T::Part * part), n - (rb + t0) + 1);  // output rows of this thread
   float cour = 0.f;
   if (rows > 0 && L <= Y.nlines) {
     const PairConst K = load_const(sK);
     const bool sw0 = L >= Y.lo && L <= Y.hi, sw1 = L + 1 >= Y.lo && L + 1 <= Y.hi;
     // every cell interior, on swept columns
-    const bool inner = sw0 && sw1 && r0 + t0 >= 2 && r0 + t0 + rows - 1 <= n - 1;
+    const bool inner = sw0 && sw1 && rb + t0 >= 2 && rb + t0 + rows - 1 <= n - 1;
     unsigned rest = 0u;  // listed cells: bit 2i + k, row t0 + i and column c + k
-    const float* at = sm + (t0 - 1) * kStepWin + 4 + c;
+    const float* at = sm + (t0 - 1) * T::Win + 4 + c;
     auto load = [&](const float* f) {
-      const float2 d = *reinterpret_cast<const float2*>(f), s = *reinterpret_cast<const float2*>(f + kStepField);
-      const float2 x = *reinterpret_cast<const float2*>(f + 2 * kStepField);
-      const float2 y = *reinterpret_cast<const float2*>(f + 3 * kStepField);
+      const float2 d = *reinterpret_cast<const float2*>(f);
+      const float2 s = *reinterpret_cast<const float2*>(f + T::Field + T::Out);
+      const float2 x = *reinterpret_cast<const float2*>(f + 2 * T::Field + T::Out);
+      const float2 y = *reinterpret_cast<const float2*>(f + 3 * T::Field + T::Out);
       return make_cell2(p, K, d.x, d.y, s.x, s.y, y.x, y.y, x.x, x.y);
     };
     Cell2 b;  // the cell after m.j, made ready while m.j is finished
@@ -729,22 +773,22 @@ __device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst
     m.va = 0ull;
     flags(m.j);
     {
-      const Cell2 j = load(at + kStepWin);
-      b = load(at + 2 * kStepWin);
+      const Cell2 j = load(at + T::Win);
+      b = load(at + 2 * T::Win);
       f2 inv, qP, qQ;
-      face(j, r0 + t0, inv, qP, qQ);
+      face(j, rb + t0, inv, qP, qQ);
       take(j, inv, qP, qQ);
       flags(j);
     }
-    at += 2 * kStepWin;
+    at += 2 * T::Win;
     // byte offset of the output pair (a field is below 4 GB)
-    uint32_t q = ((uint32_t)(r0 + t0 - 1) * (uint32_t)Y.pitch + (uint32_t)(L - 1)) * 4u;
+    uint32_t q = ((uint32_t)(rb + t0 - 1) * (uint32_t)Y.pitch + (uint32_t)(L - 1)) * 4u;
     char *const ps = reinterpret_cast<char*>(Y.srf_o), *const px = reinterpret_cast<char*>(Y.xu_o),
                *const py = reinterpret_cast<char*>(Y.yv_o);
 #pragma unroll 2
     for (int i = 0; i < rows; ++i, q += 4u * (uint32_t)Y.pitch) {
-      const int o = r0 + t0 + i;  // the row finished here
-      at += kStepWin;
+      const int o = rb + t0 + i;  // the row finished here
+      at += T::Win;
       // past the window's last row in a tile's last round: not used, within
       // the block's shared memory
       const Cell2 next = load(at);
@@ -806,7 +850,7 @@ __device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst
       unsigned w = atomicAdd(s_n, (unsigned)__popc(rest));
       for (; rest; rest &= rest - 1u) {
         const int b = __ffs(rest) - 1;
-        s_list[w++] = (uint16_t)((t0 + (b >> 1)) * kStepW + c + (b & 1));
+        s_list[w++] = (uint16_t)((t0 + (b >> 1)) * T::W + c + (b & 1));
       }
     }
     cour = fmaxf(sw0 ? cm0 : 0.f, sw1 ? cm1 : 0.f);
@@ -818,9 +862,11 @@ __device__ __forceinline__ void step_y_phase(const SweepArgs& Y, const PairConst
 
 // ---- the step ---------------------------------------------------------------------
 
+template <class T>
 struct StepShared {
-  __align__(128) float win[4 * kStepField];  // dep, srf, xu, yv: [row + 1 - r0][col + 4 - c0]
-  uint16_t list[kStepRows * kStepW];         // listed cells: window row * kStepW + tile column
+  // dep, srf, xu, yv (and the swept srf, xu, yv): [row + Halo - r0][col + 4 - c0]
+  __align__(128) float win[T::Floats];
+  uint16_t list[T::Rows * T::W];             // listed cells: window row * W + tile column
   unsigned n[2];                             // their number, x phase and y phase
   unsigned scans;
   PairConst k[2];                            // x and y axis
@@ -830,44 +876,49 @@ struct StepShared {
 // The max-wave fold of the step's input (cliffs_main.f:347-355) over the rows
 // of the window that the calling warp sweeps: loads issued before the wait for
 // the window's copies.
+template <class T>
 struct Fold {
-  float4 h[4], v[4];
+  static constexpr int N = T::W / 16;
+  float4 h[N], v[N];
 };
 
 // Fold item k of a lane: window row and tile column (a float4).
+template <class T>
 __device__ __forceinline__ void fold_item(int k, int& t, int& c) {
-  constexpr int kPairs = 256 / kStepW, kVecs = kStepW / 4;
+  constexpr int kVecs = T::W / 4;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = (32 * k + lane) / kVecs;  // of the warp's 2 * kPairs rows
-  t = warp * kPairs + r % kPairs + (r / kPairs) * kStepPair;
+  const int r = (32 * k + lane) / kVecs;  // of the warp's 8 rows
+  t = warp * 4 + r % 4 + (r / 4) * T::Pair;
   c = (lane % kVecs) * 4;
 }
 
-__device__ __forceinline__ bool fold_cell(const SweepArgs& X, int r0, int c0, int t, int c, size_t& q) {
-  const int row = r0 + t - 1;  // 0-based
+template <class T>
+__device__ __forceinline__ bool fold_cell(const SweepArgs& X, int rb, int c0, int t, int c, size_t& q) {
+  const int row = rb + t - 1;  // 0-based
   q = (size_t)row * (size_t)X.pitch + (size_t)(c0 + c);
-  return t >= 1 && t <= kStepR && row < X.nlines && c0 + c < X.n;
+  return t >= T::Halo && t < T::Halo + T::R && row < X.nlines && c0 + c < X.n;
 }
 
-template <int GX, int GY>
+template <class T, int GX, int GY>
 __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y, const StepMaps& M, int r0, int c0,
-                                          const StepCtl& C, StepShared& S) {
+                                          const StepCtl& C, StepShared<T>& S) {
   const int tid = threadIdx.x;
+  const int rb = r0 + 1 - T::Halo;  // the 1-based row of window row 0
   if (tid == 0) {
-    mbar_expect_tx(&S.bar, kStepBytes + C.extra);
-    tma_load_2d(S.win, &M.dep, &S.bar, c0 - 4, r0 - 1);
-    tma_load_2d(S.win + kStepField, &M.srf, &S.bar, c0 - 4, r0 - 1);
-    tma_load_2d(S.win + 2 * kStepField, &M.xu, &S.bar, c0 - 4, r0 - 1);
-    tma_load_2d(S.win + 3 * kStepField, &M.yv, &S.bar, c0 - 4, r0 - 1);
+    mbar_expect_tx(&S.bar, T::Bytes + C.extra);
+    tma_load_2d(S.win, &M.dep, &S.bar, c0 - 4, rb - 1);
+    tma_load_2d(S.win + T::Field, &M.srf, &S.bar, c0 - 4, rb - 1);
+    tma_load_2d(S.win + 2 * T::Field, &M.xu, &S.bar, c0 - 4, rb - 1);
+    tma_load_2d(S.win + 3 * T::Field, &M.yv, &S.bar, c0 - 4, rb - 1);
   }
-  Fold F;
+  Fold<T> F;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < Fold<T>::N; ++k) {
     int t, c;
     size_t q;
-    fold_item(k, t, c);
+    fold_item<T>(k, t, c);
     F.h[k] = F.v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (fold_cell(X, r0, c0, t, c, q)) {
+    if (fold_cell<T>(X, rb, c0, t, c, q)) {
       F.h[k] = __ldg(reinterpret_cast<const float4*>(X.hmax_in + q));
       F.v[k] = __ldg(reinterpret_cast<const float4*>(X.velmax_in + q));
     }
@@ -881,15 +932,15 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
     return;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
+  for (int k = 0; k < Fold<T>::N; ++k) {
     int t, c;
     size_t q;
-    fold_item(k, t, c);
-    if (!fold_cell(X, r0, c0, t, c, q)) continue;
-    const float* f = S.win + t * kStepWin + 4 + c;
-    const float4 d = *reinterpret_cast<const float4*>(f), s = *reinterpret_cast<const float4*>(f + kStepField);
-    const float4 x = *reinterpret_cast<const float4*>(f + 2 * kStepField);
-    const float4 y = *reinterpret_cast<const float4*>(f + 3 * kStepField);
+    fold_item<T>(k, t, c);
+    if (!fold_cell<T>(X, rb, c0, t, c, q)) continue;
+    const float* f = S.win + t * T::Win + 4 + c;
+    const float4 d = *reinterpret_cast<const float4*>(f), s = *reinterpret_cast<const float4*>(f + T::Field);
+    const float4 x = *reinterpret_cast<const float4*>(f + 2 * T::Field);
+    const float4 y = *reinterpret_cast<const float4*>(f + 3 * T::Field);
     F.h[k].x = fmaxf(F.h[k].x, eta_of(s.x, d.x));
     F.h[k].y = fmaxf(F.h[k].y, eta_of(s.y, d.y));
     F.h[k].z = fmaxf(F.h[k].z, eta_of(s.z, d.z));
@@ -903,35 +954,36 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
   }
   __syncwarp();  // the warp's rows are read before they are swept in place
   bool bad = false;
-  step_x_phase<GX>(X, &S.k[0], S.win, r0, c0, S.list, &S.n[0], bad);
+  step_x_phase<T, GX>(X, &S.k[0], S.win, rb, c0, S.list, &S.n[0], bad);
   __syncthreads();
   const unsigned cx = S.n[0];
   if (cx) {
-    for (unsigned i = tid; i < cx; i += kStepThreads) {
-      const int t = S.list[i] / kStepW, c = S.list[i] % kStepW;
-      const OutCell<float> r = step_x_value(X, r0 + t, c0 + c + 1);
-      float* f = S.win + t * kStepWin + 4 + c;
-      f[kStepField] = r.s;
-      f[2 * kStepField] = r.u;
-      f[3 * kStepField] = r.v;
+    for (unsigned i = tid; i < cx; i += T::Threads) {
+      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
+      const OutCell<float> r = T::InPlace ? step_x_value(X, rb + t, c0 + c + 1)
+                                          : step_x_window<T>(X, S.win, rb, c0, t, c);
+      float* f = S.win + T::Out + t * T::Win + 4 + c;
+      f[T::Field] = r.s;
+      f[2 * T::Field] = r.u;
+      f[3 * T::Field] = r.v;
       bad = bad || !isfinite(r.s + r.u + r.v);
     }
     __syncthreads();
   }
-  step_y_phase<GY>(Y, &S.k[1], S.win, r0, c0, S.list, &S.n[1], bad);
+  step_y_phase<T, GY>(Y, &S.k[1], S.win, rb, c0, S.list, &S.n[1], bad);
   __syncthreads();
   const unsigned cy = S.n[1];
   if (cy) {
-    for (unsigned i = tid; i < cy; i += kStepThreads) {
-      const int t = S.list[i] / kStepW, c = S.list[i] % kStepW;
+    for (unsigned i = tid; i < cy; i += T::Threads) {
+      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
       bool scan;
-      const OutCell<float> r = step_y_value(X, Y, S.win, r0, c0, t, c, scan);
+      const OutCell<float> r = step_y_value<T>(X, Y, S.win, rb, c0, t, c, scan);
       if (scan) {
         S.list[i] |= 0x8000u;
         S.scans = 1u;
         continue;
       }
-      const size_t q = (size_t)(r0 + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
+      const size_t q = (size_t)(rb + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
       Y.srf_o[q] = r.s;
       Y.xu_o[q] = r.v;
       Y.yv_o[q] = r.u;
@@ -947,19 +999,19 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
       for (unsigned i = 0; i < cy; ++i) {
         const unsigned ent = S.list[i];
         if (!(ent & 0x8000u)) continue;
-        const int t = (int)(ent & 0x7fffu) / kStepW, c = (int)(ent & 0x7fffu) % kStepW;
+        const int t = (int)(ent & 0x7fffu) / T::W, c = (int)(ent & 0x7fffu) % T::W;
         if (c != col) {
           col = c;
           wet = false;
-          for (int j = 0; j < Y.n && !wet; j += kStepThreads)
+          for (int j = 0; j < Y.n && !wet; j += T::Threads)
             wet = __syncthreads_or(j + tid < Y.n && step_x_wet(X, j + tid + 1, c0 + c + 1));
         }
         if (tid == 0) {
-          const float* f = S.win + t * kStepWin + 4 + c;
-          const size_t q = (size_t)(r0 + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
-          Y.srf_o[q] = wet ? state_from_depth(0.f, f[0]) : f[kStepField];
-          Y.xu_o[q] = wet ? 0.f : f[2 * kStepField];
-          Y.yv_o[q] = wet ? 0.f : f[3 * kStepField];
+          const float* f = S.win + t * T::Win + 4 + c;
+          const size_t q = (size_t)(rb + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
+          Y.srf_o[q] = wet ? state_from_depth(0.f, f[0]) : f[T::Field + T::Out];
+          Y.xu_o[q] = wet ? 0.f : f[2 * T::Field + T::Out];
+          Y.yv_o[q] = wet ? 0.f : f[3 * T::Field + T::Out];
         }
       }
     }
@@ -967,14 +1019,14 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
   if (bad) atomicOr(X.status, ST_NAN);
 }
 
-// Tiles in bands of kStepR rows, the last band first when `flip` is set: a
+// Tiles in bands of R rows, the last band first when `flip` is set: a
 // step starts on the rows that the one before it wrote last, which are still
 // in L2.
-template <int GX, int GY>
-__global__ void __launch_bounds__(kStepThreads, kStepBlocks)
+template <class T, int GX, int GY>
+__global__ void __launch_bounds__(T::Threads, T::Blocks)
     step_kernel(const __grid_constant__ SweepArgs X, const __grid_constant__ SweepArgs Y,
                 const __grid_constant__ StepMaps M, const StepCtl C, const __grid_constant__ PairPair K) {
-  __shared__ StepShared S;
+  __shared__ StepShared<T> S;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     mbar_init(&S.bar, 1);
@@ -986,7 +1038,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepBlocks)
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int by = C.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
-  step_tile<GX, GY>(X, Y, M, by * kStepR, (int)blockIdx.x * kStepW, C, S);
+  step_tile<T, GX, GY>(X, Y, M, by * T::R, (int)blockIdx.x * T::W, C, S);
 }
 
 // One whole step of many grids (batch.cuh): a block per tile of the list of
@@ -1007,9 +1059,9 @@ struct BatchStep {
   int n;
 };
 
-template <int GX, int GY>
-__global__ void __launch_bounds__(kStepThreads, kStepBlocks) batch_step_kernel(const BatchStep B, const StepCtl C) {
-  __shared__ StepShared S;
+template <class T, int GX, int GY>
+__global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const BatchStep B, const StepCtl C) {
+  __shared__ StepShared<T> S;
   __shared__ SweepArgs sA[2];
   const int tid = threadIdx.x;
   // every other step takes the tiles last to first, as step_kernel its bands
@@ -1019,7 +1071,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepBlocks) batch_step_kernel(c
   const int local = tile - __ldg(B.off + k), g = __ldg(B.gx + k);
   static_assert(sizeof(SweepArgs) % 8 == 0 && sizeof(PairPair) % 8 == 0, "copied in 8-byte words");
   const auto copy = [&](void* to, const void* from, int bytes) {
-    for (int w = tid; w < bytes / 8; w += kStepThreads)
+    for (int w = tid; w < bytes / 8; w += T::Threads)
       reinterpret_cast<unsigned long long*>(to)[w] = __ldg(reinterpret_cast<const unsigned long long*>(from) + w);
   };
   copy(&sA[0], &A->X, sizeof(SweepArgs));
@@ -1031,7 +1083,7 @@ __global__ void __launch_bounds__(kStepThreads, kStepBlocks) batch_step_kernel(c
     fence_mbar_init();
   }
   __syncthreads();
-  step_tile<GX, GY>(sA[0], sA[1], A->M, local / g * kStepR, local % g * kStepW, C, S);
+  step_tile<T, GX, GY>(sA[0], sA[1], A->M, local / g * T::R, local % g * T::W, C, S);
 }
 
 }  // namespace cliffs

@@ -2,8 +2,9 @@
 two-dimensional grid) against a launch per sweep (CLIFFS_SWEEP_DIRECT):
 bit-identical states, max-wave fields and status.
 
-Grids around the kernel's tile (64 columns x 30 rows), as small as 3 cells
-across, in plane, spherical and stretched coordinates; on each a rough sea
+Grids around the kernel's tiles, as small as 3 cells across and large enough
+for each of its three tiles (64 columns x 30 rows on large grids, 32 x 14 and
+32 x 10 on smaller ones), in plane, spherical and stretched coordinates; on each a rough sea
 floor with islands and ponds, so that every kind of cell (plain, shoreline,
 flooded, drying, land at rest, line ends) lies in tiles' middles, edges and
 corners; odd and even step counts (a call's last odd step runs a sweep at a
@@ -55,7 +56,10 @@ def _same(a, b):
 
 @pytest.mark.parametrize("nx,ny,metric", [
     (3, 3, "plane"), (4, 95, "plane"), (130, 3, "plane"), (63, 29, "plane"), (64, 30, "plane"), (65, 31, "plane"),
-    (66, 62, "sphere"), (127, 33, "stretched"), (129, 61, "sphere"), (200, 91, "stretched"), (257, 130, "plane")])
+    (66, 62, "sphere"), (127, 33, "stretched"), (129, 61, "sphere"), (200, 91, "stretched"), (257, 130, "plane"),
+    (31, 11, "plane"), (33, 21, "sphere"), (97, 41, "stretched"),
+    (1290, 311, "plane"), (1279, 323, "sphere"), (1665, 309, "stretched"),  # 32 x 14 tiles
+    (1601, 751, "plane"), (1663, 749, "sphere"), (1665, 781, "stretched")])  # 64 x 30 tiles
 def test_whole_steps_match_sweeps(nx, ny, metric):
     c = _case(nx, ny, metric, nx * 1000 + ny)
     a, b = _grid(c, cg.TILED), _grid(c, cg.DIRECT)
@@ -91,7 +95,7 @@ def test_contexts_in_turn():
                                      ("plane", "stretched", "sphere")])
 def test_batched_whole_steps_match_sweeps(metrics):
     """Uneven grids in one batch, by steps of odd and even length."""
-    sizes = [(3, 40), (65, 31), (190, 97)]
+    sizes = [(3, 40), (65, 31), (190, 97 if metrics[2] == "plane" else 2100)]
     cs = [_case(nx, ny, m, nx) for (nx, ny), m in zip(sizes, metrics)]
     a, b = [_grid(c, cg.TILED) for c in cs], [_grid(c, cg.DIRECT) for c in cs]
     batch = pkg.Batch(a)
