@@ -186,6 +186,8 @@ struct cliffs_ctx {
   } win[2];  // StepLarge's; StepSmall's and StepTiny's
   bool step_ok = false;
   int step_size = STEP_LARGE;  // the tile of the grid's whole steps
+  int* step_order = nullptr;   // its tiles with the coasts first (nullptr: by bands), and the coasts' number
+  int step_coast = 0;
   int grid_sx = 0, grid_sy = 0;  // resident blocks of staged_x / staged_y
   unsigned long long stage_ns = 2000000000ull;  // limit of one stage wait
   // fast-kernel sweeps launched as programmatic dependents of the previous
@@ -539,6 +541,31 @@ int step_size(int64_t large, int64_t tiny, int sms) {
                                                   : STEP_TINY;
 }
 
+// Whether coasts go first among so many tiles: up to six times what the chip
+// holds at once.  Beyond, the end of a step is a small part of it, and tiles
+// taken out of their bands cost more in L2, and places that are not the block's
+// own more registers (us per step, bands and coasts first: 4320 x 2160, 8 times,
+// 90.4 and 91.8; 2048 x 2048, 3.6 times, 47.0 and 45.0; 1003 x 777 18.3 and
+// 16.1; 600 x 600 13.7 and 13.2).
+bool coasts_first(int64_t tiles, int size, int sms) {
+  return tiles <= 6ll * sms * (size == STEP_LARGE ? StepLarge::Blocks : StepSmall::Blocks);
+}
+
+// Flags of the tiles that hold a coast.
+void tile_coasts(int size, int tiles, int nx, int ny, int pitch, const float* dep, uint8_t* flags, cudaStream_t st) {
+  if (size == STEP_LARGE)
+    k_tile_coast<StepLarge><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+  else if (size == STEP_SMALL)
+    k_tile_coast<StepSmall><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+  else
+    k_tile_coast<StepTiny><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+}
+
+int device_sms(int dev) {
+  int n = 0;
+  return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 1;
+}
+
 int check_device(int* dev) {
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) return CLIFFS_ERR_DEVICE;
@@ -876,15 +903,17 @@ StepArgs step_args(const cliffs_ctx* c, int s, const float* ex, const float* ey,
 
 // The variant for the grid's spacing: a table when an axis is not uniform,
 // else uniform spacing with or without the metric term.
-template <class T>
+template <class T, bool ORDERED>
 cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepArgs& A, const StepCtl& C) {
-  cfg.gridDim = dim3((c->nx + T::W - 1) / T::W, (c->ny + T::R - 1) / T::R);
+  const unsigned gx = (unsigned)((c->nx + T::W - 1) / T::W), gy = (unsigned)((c->ny + T::R - 1) / T::R);
+  cfg.gridDim = ORDERED ? dim3(gx * gy) : dim3(gx, gy);
   cfg.blockDim = dim3(T::Threads);
+  const int* o = c->step_order;
   if (!c->geo_uni_x || !c->geo_uni_y)
-    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_TABLE, GEO_TABLE>, A.X, A.Y, A.M, C, A.K);
+    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_TABLE, GEO_TABLE, ORDERED>, A.X, A.Y, A.M, C, A.K, o);
   if (c->scl_y || c->lscale)
-    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_METRIC, GEO_METRIC>, A.X, A.Y, A.M, C, A.K);
-  return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_FLAT, GEO_FLAT>, A.X, A.Y, A.M, C, A.K);
+    return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_METRIC, GEO_METRIC, ORDERED>, A.X, A.Y, A.M, C, A.K, o);
+  return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_FLAT, GEO_FLAT, ORDERED>, A.X, A.Y, A.M, C, A.K, o);
 }
 
 // One whole step on the context's stream, folding the previous step's end
@@ -892,7 +921,7 @@ cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepA
 int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
   const int s = c->cur;
   const StepArgs A = step_args(c, s, ex, ey, c->step_size);
-  const StepCtl C{S.wait_ns, S.extra, s};
+  const StepCtl C{S.wait_ns, S.extra, s, c->step_coast};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -901,9 +930,10 @@ int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl&
   cfg.attrs = at;
   cfg.numAttrs = c->pdl ? 1 : 0;
   ++c->launches;
-  CK(c->step_size == STEP_LARGE   ? step_launch<StepLarge>(c, cfg, A, C)
-     : c->step_size == STEP_SMALL ? step_launch<StepSmall>(c, cfg, A, C)
-                                  : step_launch<StepTiny>(c, cfg, A, C));
+  CK(c->step_size == STEP_SMALL  ? (step_launch<StepSmall, true>(c, cfg, A, C))
+     : c->step_size == STEP_TINY ? (step_launch<StepTiny, true>(c, cfg, A, C))
+     : c->step_order             ? (step_launch<StepLarge, true>(c, cfg, A, C))
+                                 : (step_launch<StepLarge, false>(c, cfg, A, C)));
   c->cur = 1 - s;
   c->sweeps += 2u;
   return CLIFFS_OK;
@@ -1096,6 +1126,10 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
   if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   c->stream = c->own;
   const size_t n64 = (size_t)c->nx * c->ny;
+  const int sms = device_sms(dev);
+  c->step_size = step_size(step_tiles(STEP_LARGE, c->nx, c->ny), step_tiles(STEP_TINY, c->nx, c->ny), sms);
+  const int tiles = step_tiles(c->step_size, c->nx, c->ny);
+  uint8_t* tile_flags = nullptr;
   auto layout = [&](char* base) {
     size_t off = 0;
     carve(base, off, &c->dep, cells);
@@ -1118,6 +1152,8 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     carve(base, off, &c->cnt, 2);
     carve(base, off, &c->dep64, n64);
     carve(base, off, &c->xfer, 3 * n64);
+    carve(base, off, &c->step_order, (size_t)tiles + 1);
+    carve(base, off, &tile_flags, (size_t)tiles);
     return off;
   };
   if (dalloc(&c->arena, layout(nullptr))) return fail(CLIFFS_ERR_NOMEM);
@@ -1130,6 +1166,12 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     return fail(CLIFFS_ERR_CUDA);
   ++c->launches;
   k_dep_from64<<<grid2(c->pitch, c->ny), 128, 0, c->stream>>>(c->nx, c->ny, c->pitch, c->dep64, c->dep);
+  const bool ordered = c->xrun && c->yrun && coasts_first(tiles, c->step_size, sms);
+  if (ordered) {  // the order of whole steps' tiles
+    c->launches += 2;
+    tile_coasts(c->step_size, tiles, c->nx, c->ny, c->pitch, c->dep, tile_flags, c->stream);
+    k_tile_order<<<1, 1024, 0, c->stream>>>(tiles, tile_flags, c->step_order, c->step_order + tiles);
+  }
   if (cudaGetLastError() != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   // geometry tables
   auto build_geo = [&](int n, const double* s, std::vector<float4>& geo, float& i1, float& in1) {
@@ -1189,9 +1231,13 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     if (cudaMemcpyAsync(lo, span.data(), span.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->status, 0, 2 * sizeof(unsigned), c->stream) != cudaSuccess ||
         cudaMemsetAsync(c->cnt, 0, 2 * sizeof(uint32_t), c->stream) != cudaSuccess ||
+        (ordered &&
+         cudaMemcpyAsync(&c->step_coast, c->step_order + tiles, sizeof(int), cudaMemcpyDeviceToHost, c->stream) !=
+             cudaSuccess) ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
       return fail(CLIFFS_ERR_CUDA);
   }
+  if (!ordered) c->step_order = nullptr;
   if (!d->row_scale) c->lscale = nullptr;  // (its arena slot stays unused)
   if (!zeta_nonzero) c->scl_y = nullptr;
   // the staged sweep kernels: tensor maps of the y-sweep's fields and the
@@ -1242,7 +1288,6 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
         st = !make_map(&W.srf[k], c->srf[k], nx, ny, pp, bx, by) && !make_map(&W.xu[k], c->xu[k], nx, ny, pp, bx, by) &&
              !make_map(&W.yv[k], c->yv[k], nx, ny, pp, bx, by);
     }
-    c->step_size = step_size(step_tiles(STEP_LARGE, nx, ny), step_tiles(STEP_TINY, nx, ny), nsm);
     c->step_ok = st && cells < (1ull << 30);  // its stores take 32-bit byte offsets
     c->grid_sx = nsm * bx;
     c->grid_sy = nsm * by;
@@ -2870,8 +2915,8 @@ struct cliffs_batch {
   // plans: every scenario's arguments for the steps from its state copy cur
   // ([0]) and back to it ([1]), the tile list, and the variant
   StepArgs* d_step[2] = {nullptr, nullptr};
-  int* d_step_off = nullptr;  // n + 1 offsets, then n tiles across
-  int step_tiles = 0;
+  int4* d_step_order = nullptr;
+  int step_tiles = 0, step_coast = 0;
   int step_geo = GEO_FLAT;
   int step_size = STEP_LARGE;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
@@ -2940,7 +2985,7 @@ static void batch_free(cliffs_batch* b) {
   if (b->d_ymaps) cudaFree(b->d_ymaps);
   for (StepArgs* a : b->d_step)
     if (a) cudaFree(a);
-  if (b->d_step_off) cudaFree(b->d_step_off);
+  if (b->d_step_order) cudaFree(b->d_step_order);
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -3025,7 +3070,7 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
   for (int k = 0; k < n; ++k) whole = whole && ctxs[k]->step_ok;
   if (whole) {
     std::vector<StepArgs> sa[2];
-    std::vector<int> so((size_t)n + 1, 0), sg;
+    std::vector<int4> order;
     bool uniform = true, plain = true;
     int64_t large = 0, tiny = 0;
     for (int k = 0; k < n; ++k) {
@@ -3037,20 +3082,45 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
       const cliffs_ctx* c = ctxs[k];
       for (int q = 0; q < 2; ++q)
         sa[q].push_back(step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr, b->step_size));
-      so[k + 1] = so[k] + step_tiles(b->step_size, c->nx, c->ny);
+      const int t = step_tiles(b->step_size, c->nx, c->ny);
       const int w = b->step_size == STEP_LARGE ? StepLarge::W : StepSmall::W;
-      sg.push_back((c->nx + w - 1) / w);
+      const int r = b->step_size == STEP_LARGE ? StepLarge::R : b->step_size == STEP_SMALL ? StepSmall::R : StepTiny::R;
+      const int across = (c->nx + w - 1) / w;
+      for (int q = 0; q < t; ++q) order.push_back(make_int4(k, q / across * r, q % across * w, 0));
       uniform = uniform && c->geo_uni_x && c->geo_uni_y;
       plain = plain && !c->scl_y && !c->lscale;
     }
     b->step_geo = !uniform ? GEO_TABLE : plain ? GEO_FLAT : GEO_METRIC;
-    b->step_tiles = so[n];
-    so.insert(so.end(), sg.begin(), sg.end());
-    if (dalloc(&b->d_step[0], (size_t)n) || dalloc(&b->d_step[1], (size_t)n) || dalloc(&b->d_step_off, so.size()))
+    b->step_tiles = (int)order.size();
+    if (coasts_first(b->step_tiles, b->step_size, b->sms)) {  // coasts first, then the others
+      uint8_t* d_flags = nullptr;
+      std::vector<uint8_t> flags(order.size());
+      if (dalloc(&d_flags, flags.size())) return fail(CLIFFS_ERR_NOMEM);
+      int t0 = 0;
+      for (int k = 0; k < n; ++k) {
+        const cliffs_ctx* c = ctxs[k];
+        const int t = step_tiles(b->step_size, c->nx, c->ny);
+        tile_coasts(b->step_size, t, c->nx, c->ny, c->pitch, c->dep, d_flags + t0, b->stream);
+        t0 += t;
+      }
+      const bool got = cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, b->stream) ==
+                           cudaSuccess &&
+                       cudaStreamSynchronize(b->stream) == cudaSuccess;
+      cudaFree(d_flags);
+      if (!got) return fail(CLIFFS_ERR_CUDA);
+      std::vector<int4> sorted;
+      for (int pass = 0; pass < 2; ++pass) {
+        for (size_t q = 0; q < order.size(); ++q)
+          if ((flags[q] != 0) == (pass == 0)) sorted.push_back(order[q]);
+        if (pass == 0) b->step_coast = (int)sorted.size();
+      }
+      order.swap(sorted);
+    }
+    if (dalloc(&b->d_step[0], (size_t)n) || dalloc(&b->d_step[1], (size_t)n) || dalloc(&b->d_step_order, order.size()))
       return fail(CLIFFS_ERR_NOMEM);
     if (cudaMemcpy(b->d_step[0], sa[0].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
         cudaMemcpy(b->d_step[1], sa[1].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
-        cudaMemcpy(b->d_step_off, so.data(), so.size() * sizeof(int), cudaMemcpyHostToDevice))
+        cudaMemcpy(b->d_step_order, order.data(), order.size() * sizeof(int4), cudaMemcpyHostToDevice))
       return fail(CLIFFS_ERR_CUDA);
   }
   b->plan.mode = b->max_ctas > 0 ? CLIFFS_BATCH_PERSISTENT : CLIFFS_BATCH_GRAPH;
@@ -3158,8 +3228,8 @@ static void batch_step_launch(cliffs_batch* b, const BatchStep& B, const StepCtl
 }
 
 static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
-  const BatchStep B{b->d_step[odd], b->d_step_off, b->d_step_off + b->ctx.size() + 1, (int)b->ctx.size()};
-  const StepCtl C{S.wait_ns, S.extra, odd};
+  const BatchStep B{b->d_step[odd], b->d_step_order};
+  const StepCtl C{S.wait_ns, S.extra, odd, b->step_coast};
   if (b->step_size == STEP_LARGE)
     batch_step_launch<StepLarge>(b, B, C);
   else if (b->step_size == STEP_SMALL)

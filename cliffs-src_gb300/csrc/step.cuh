@@ -37,7 +37,6 @@
 // SM 50.8 us (spills); tiles of 32 columns 48.9 us; the max-wave update on the
 // outputs, in the y phase, 49.5 us.
 #pragma once
-#include "batch.cuh"
 #include "staged.cuh"
 
 namespace cliffs {
@@ -149,7 +148,8 @@ struct PairPair {
 struct StepCtl {
   unsigned long long wait_ns;  // limit of the window's wait
   unsigned extra;              // bytes it waits for beyond its copies: 0, except in the timeout self-test
-  int flip;                    // bands last to first
+  int flip;                    // tiles beyond the first `coast` last to first, or bands
+  int coast;                   // tiles at the front of the order that go first in every step
 };
 
 // rsqrtf for arguments that are not subnormal (celerities: g * max(H, ground);
@@ -1019,13 +1019,71 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
   if (bad) atomicOr(X.status, ST_NAN);
 }
 
-// Tiles in bands of R rows, the last band first when `flip` is set: a
+// The order of a grid's tiles: those that hold a coast first, as their listed
+// cells make them last longer (a step ends with its slowest block, which is to
+// start early); the others band by band, every other step last to first: a
 // step starts on the rows that the one before it wrote last, which are still
-// in L2.
-template <class T, int GX, int GY>
+// in L2.  The coast is that of the depth at the context's creation: the order
+// changes no result.
+__device__ __forceinline__ int tile_at(const StepCtl& C, int id, int tiles) {
+  return C.flip && id >= C.coast ? tiles - 1 - (id - C.coast) : id;
+}
+
+// Whether a tile or a cell beside it holds land and sea.
+template <class T>
+__global__ void k_tile_coast(int nx, int ny, int pitch, const float* __restrict__ dep, uint8_t* flags) {
+  const int tx = (int)blockIdx.x % ((nx + T::W - 1) / T::W), ty = (int)blockIdx.x / ((nx + T::W - 1) / T::W);
+  bool land = false, sea = false;
+  for (int i = threadIdx.x; i < (T::W + 2) * (T::R + 2); i += blockDim.x) {
+    const int x = tx * T::W - 1 + i % (T::W + 2), y = ty * T::R - 1 + i / (T::W + 2);
+    if (x < 0 || x >= nx || y < 0 || y >= ny) continue;
+    const bool l = dep[(size_t)y * pitch + x] < 0.f;
+    land = land || l;
+    sea = sea || !l;
+  }
+  land = __syncthreads_or(land);
+  sea = __syncthreads_or(sea);
+  if (threadIdx.x == 0) flags[blockIdx.x] = land && sea;
+}
+
+// order: the tiles with a flag, then the others, each in their order; count:
+// those with one.  One block of 1024 threads.
+__global__ void k_tile_order(int tiles, const uint8_t* __restrict__ flags, int* order, int* count) {
+  __shared__ int s_warp[32], s_base;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int base = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int i0 = 0; i0 < tiles; i0 += 1024) {
+      const int i = i0 + tid;
+      const bool take = i < tiles && (flags[i] != 0) == (pass == 0);
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (lane == 0) s_warp[warp] = __popc(m);
+      __syncthreads();
+      if (tid == 0) {
+        int sum = base;
+        for (int w = 0; w < 32; ++w) {
+          const int c = s_warp[w];
+          s_warp[w] = sum;
+          sum += c;
+        }
+        s_base = sum;
+      }
+      __syncthreads();
+      if (take) order[s_warp[warp] + __popc(m & ((1u << lane) - 1u))] = i;
+      base = s_base;
+      __syncthreads();
+    }
+    if (pass == 0 && tid == 0) *count = base;
+  }
+}
+
+// ORDERED: a one-dimensional grid, the tiles from the order; else a grid of
+// tiles, by bands.
+template <class T, int GX, int GY, bool ORDERED>
 __global__ void __launch_bounds__(T::Threads, T::Blocks)
     step_kernel(const __grid_constant__ SweepArgs X, const __grid_constant__ SweepArgs Y,
-                const __grid_constant__ StepMaps M, const StepCtl C, const __grid_constant__ PairPair K) {
+                const __grid_constant__ StepMaps M, const StepCtl C, const __grid_constant__ PairPair K,
+                const int* __restrict__ order) {
   __shared__ StepShared<T> S;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
@@ -1035,17 +1093,26 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
     S.k[1] = K.y;
     fence_mbar_init();
   }
+  int bx, by;
+  if (ORDERED) {  // written once, before the context's first launch: read ahead
+    const int gx = (X.n + T::W - 1) / T::W;
+    const int tile = __ldg(order + tile_at(C, (int)blockIdx.x, (int)gridDim.x));
+    bx = tile % gx;
+    by = tile / gx;
+  } else {
+    bx = (int)blockIdx.x;
+    by = C.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+  }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int by = C.flip ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
-  step_tile<T, GX, GY>(X, Y, M, by * T::R, (int)blockIdx.x * T::W, C, S);
+  step_tile<T, GX, GY>(X, Y, M, by * T::R, bx * T::W, C, S);
 }
 
 // One whole step of many grids (batch.cuh): a block per tile of the list of
-// all scenarios' tiles, the scenario found by bisection, its arguments staged
-// in shared memory and its tensor maps read from device memory.  24 scenarios
-// of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with its uploads
-// and maxima: 7.0 ms, from 12.2 with a launch per sweep phase.
+// all scenarios' tiles (coasts first, as above), the scenario's arguments
+// staged in shared memory and its tensor maps read from device memory.  24
+// scenarios of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with
+// its uploads and maxima: 7.0 ms, from 12.2 with a launch per sweep phase.
 struct StepArgs {
   SweepArgs X, Y;
   PairPair K;
@@ -1054,9 +1121,7 @@ struct StepArgs {
 
 struct BatchStep {
   const StepArgs* args;  // per scenario, for the state copy that the step reads
-  const int* off;        // first tile of a scenario; [n] the total
-  const int* gx;         // tiles across a scenario
-  int n;
+  const int4* order;     // scenario, first row and first column of each tile
 };
 
 template <class T, int GX, int GY>
@@ -1064,11 +1129,8 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const
   __shared__ StepShared<T> S;
   __shared__ SweepArgs sA[2];
   const int tid = threadIdx.x;
-  // every other step takes the tiles last to first, as step_kernel its bands
-  const int tile = C.flip ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-  const int k = batch_scenario(B.off, B.n, tile);
-  const StepArgs* A = B.args + k;
-  const int local = tile - __ldg(B.off + k), g = __ldg(B.gx + k);
+  const int4 at = __ldg(B.order + tile_at(C, (int)blockIdx.x, (int)gridDim.x));
+  const StepArgs* A = B.args + at.x;
   static_assert(sizeof(SweepArgs) % 8 == 0 && sizeof(PairPair) % 8 == 0, "copied in 8-byte words");
   const auto copy = [&](void* to, const void* from, int bytes) {
     for (int w = tid; w < bytes / 8; w += T::Threads)
@@ -1083,7 +1145,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const
     fence_mbar_init();
   }
   __syncthreads();
-  step_tile<T, GX, GY>(sA[0], sA[1], A->M, local / g * T::R, local % g * T::W, C, S);
+  step_tile<T, GX, GY>(sA[0], sA[1], A->M, at.y, at.z, C, S);
 }
 
 }  // namespace cliffs
