@@ -14,45 +14,65 @@
 // tensor-core product (im2col x W^T, bias and ReLU in the epilogue).  A level
 // with fewer output channels (the map's one, or 8) is below the tensor
 // cores' narrowest tile and runs as a direct convolution (k_dec_conv).
-// Backward: the output gradient in BF16 (k_to_bf16); the weight and bias
-// gradients by k_dec_dw (per chunk of pixels, FP32 sums of BF16 products
-// read straight from the level input, then summed over the chunks); the
-// input gradient by k_dec_dx (FP32 sums of BF16 products over the taps and
-// the 2x2 upsampled cells).  The direct kernels keep the weights in shared
-// memory as FP32, [tap][input channel][output channel], with CO >= Cout
-// output channels (zeros past Cout), and every sum runs in a fixed order, so
-// training is deterministic.
+// Backward: the map's gradient in BF16 (k_to_bf16); per level the weight and
+// bias gradients by k_dec_dw (k_dec_dw1 for the map's level; per chunk of input
+// cells, FP32 sums of the output gradient over the pixels that a cell reaches
+// through a tap, times the cell, then summed over the chunks) and the input
+// gradient by k_dec_dx (k_dec_dx1; FP32 sums of BF16 products over the taps and
+// the 2x2 upsampled cells), in BF16 rows that are the next level's output
+// gradient.  The convolution and the input gradient keep the weights in shared
+// memory as FP32.  Every sum runs in a fixed order, so training is deterministic.
 #pragma once
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdint>
 
 namespace cliffs_nn {
 
+// Two FP32 values in a register pair and Blackwell's packed operations on
+// them: each half rounds as the scalar operation does.
+using fpair = unsigned long long;
+__device__ __forceinline__ fpair pair_of(uint32_t lo, uint32_t hi) {
+  return (fpair)hi << 32 | lo;
+}
+__device__ __forceinline__ fpair pair_add(fpair a, fpair b) {
+  fpair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ void pair_fma(fpair& acc, fpair a, fpair b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float pair_lo(fpair a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float pair_hi(fpair a) { return __uint_as_float((uint32_t)(a >> 32)); }
+// Two BF16 values as FP32.
+__device__ __forceinline__ fpair pair_bf16(uint32_t w) { return pair_of(w << 16, w & 0xffff0000u); }
+
 // im2col of the 2x upsampled input: row p = (b, Y, X) of the output grid
 // (side 2S), column k = tap * Cin + c < 9 Cin, columns up to kp zero.  The
 // upsampled cell (Y', X') = (Y + ty - 1, X + tx - 1) reads input cell
-// (Y' / 2, X' / 2); outside [0, 2S) it is zero padding.  dst [P][kp].  Block
-// (32, 8): eight pixels, each thread 8 columns at a time (one tap, 8
-// channels: C and kp are multiples of 8), one 16-byte load and store.  Pixel
-// indices are 32-bit (B (2S)^2 < 2^31).
-__global__ void k_im2col_up(int B, int S, int C, const __nv_bfloat16* __restrict__ x, int kp, __nv_bfloat16* dst) {
-  const int S2 = 2 * S, img = S2 * S2;
-  const int p = blockIdx.x * 8 + threadIdx.y;
-  if (p >= B * img) return;
+// (Y' / 2, X' / 2); outside [0, 2S) it is zero padding.  dst [P][kp].  A thread
+// per 8 columns (one tap, 8 channels: C and kp are multiples of 8), one 16-byte
+// load and store, so that every lane works whatever kp is: a warp per pixel left
+// 28 of 32 lanes idle in every second round of the surrogate's 36 groups and took
+// 171 us at a batch of 512 (302 MB written), this 105.  Pixel indices are 32-bit
+// (B (2S)^2 < 2^31).
+__global__ void __launch_bounds__(256) k_im2col_up(int B, int S, int C, const __nv_bfloat16* __restrict__ x, int kp,
+                                                   __nv_bfloat16* dst) {
+  const unsigned S2 = 2 * S, img = S2 * S2, per = kp / 8;
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;  // fewer than 18 map cells B < 2^32
+  const int p = t / per, k = 8 * (t % per);
+  if (p >= (int)(B * img)) return;
   const int b = p / img, r = p % img, Y = r / S2, X = r % S2;
-  uint4* out = reinterpret_cast<uint4*>(dst + (size_t)p * kp);
-  for (int kq = threadIdx.x; kq < kp / 8; kq += 32) {
-    const int k = 8 * kq;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (k < 9 * C) {
-      const int tap = k / C, c = k % C;
-      const int Yu = Y + tap / 3 - 1, Xu = X + tap % 3 - 1;
-      if (Yu >= 0 && Yu < S2 && Xu >= 0 && Xu < S2)
-        v = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * S + (Yu >> 1)) * S + (Xu >> 1)) * C + c));
-    }
-    out[kq] = v;
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (k < 9 * C) {
+    const int tap = k / C, c = k % C;
+    const int Yu = Y + tap / 3 - 1, Xu = X + tap % 3 - 1;
+    if (Yu >= 0 && Yu < 2 * S && Xu >= 0 && Xu < 2 * S)
+      v = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * S + (Yu >> 1)) * S + (Xu >> 1)) * C + c));
   }
+  reinterpret_cast<uint4*>(dst)[t] = v;
 }
 
 // The decoder's input: ReLU of the latent columns [col0, col0 + n) of the
@@ -106,7 +126,17 @@ __global__ void __launch_bounds__(32 * kStrands) k_reduce_wgrad(int rows, int co
   float s = 0.f;
   if (in) {
     const int r = k / cols, c = k % cols;
-    for (int z = strand; z < splits; z += kStrands) s += part[((size_t)z * rows + r) * ldp + c];
+    const float* at = part + (size_t)r * ldp + c;
+    const size_t split = (size_t)rows * ldp;
+    int z = strand;
+    for (; z + 7 * kStrands < splits; z += 8 * kStrands) {  // 8 loads in flight, added in order
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = __ldg(at + (size_t)(z + i * kStrands) * split);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += v[i];
+    }
+    for (; z < splits; z += kStrands) s += __ldg(at + (size_t)z * split);
   }
   sh[strand][lane] = s;
   __syncthreads();
@@ -118,16 +148,17 @@ __global__ void __launch_bounds__(32 * kStrands) k_reduce_wgrad(int rows, int co
   }
 }
 
-// FP32 to BF16, n values.
+// FP32 to BF16, n values, four a thread (both arrays 16-byte aligned).
 __global__ void k_to_bf16(int n, const float* __restrict__ src, __nv_bfloat16* dst) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) dst[t] = __float2bfloat16(src[t]);
-}
-
-// Input channels per thread of the direct kernels: G x CO FP32 sums.
-template <int CO>
-__host__ __device__ constexpr int dec_group() {
-  return CO == 1 ? 8 : CO == 8 ? 4 : CO == 16 ? 2 : 1;
+  const int t = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (t + 3 < n) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(src + t));
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(dst + t) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  } else {
+    for (int i = t; i < n; ++i) dst[i] = __float2bfloat16(src[i]);
+  }
 }
 
 // The 8 BF16 values of a 16-byte load as FP32.
@@ -140,249 +171,556 @@ __device__ __forceinline__ void unpack8(const uint4 q, float (&v)[8]) {
   }
 }
 
-// G consecutive BF16 values (G = 1, 2, 4 or 8; 2G-byte aligned) as FP32.
-template <int G>
-__device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float (&v)[G]) {
-  if constexpr (G == 8) {
-    float t[8];
-    unpack8(__ldg(reinterpret_cast<const uint4*>(p)), t);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = t[i];
-  } else if constexpr (G == 4) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
-    v[0] = __uint_as_float(q.x << 16);
-    v[1] = __uint_as_float(q.x & 0xffff0000u);
-    v[2] = __uint_as_float(q.y << 16);
-    v[3] = __uint_as_float(q.y & 0xffff0000u);
-  } else if constexpr (G == 2) {
-    const uint32_t q = __ldg(reinterpret_cast<const unsigned int*>(p));
-    v[0] = __uint_as_float(q << 16);
-    v[1] = __uint_as_float(q & 0xffff0000u);
-  } else {
-    v[0] = __bfloat162float(p[0]);
-  }
-}
-
 // The weights w [co][kp] (BF16, columns k = tap * C + c) into shared memory
-// as FP32 [9C][CO], zero past co.  The whole block calls it.
-template <int CO>
-__device__ __forceinline__ void stage_weights(float* sw, int C, int co, const __nv_bfloat16* __restrict__ w, int kp) {
+// as FP32, [tap][C][co] or (CLAST) [tap][co][C].  The whole block calls it; true
+// if every weight is finite.
+template <bool CLAST>
+__device__ __forceinline__ bool stage_weights(float* sw, int C, int co, const __nv_bfloat16* __restrict__ w, int kp) {
   const int K = 9 * C;
-  for (int t = threadIdx.x; t < K * CO; t += blockDim.x) {
-    const int k = t / CO, o = t % CO;
-    sw[t] = o < co ? __bfloat162float(w[(size_t)o * kp + k]) : 0.f;
+  bool finite = true;
+  for (int t = threadIdx.x; t < K * co; t += blockDim.x) {
+    const int o = CLAST ? t / C % co : t % co, k = CLAST ? t / (C * co) * C + t % C : t / co;
+    const float v = __bfloat162float(w[(size_t)o * kp + k]);
+    finite = finite && isfinite(v);
+    sw[t] = v;
   }
-  __syncthreads();
+  return __syncthreads_and(finite);
 }
 
-// Direct forward convolution of a level with co <= CO output channels (CO =
-// 1 or 8): one thread per output pixel p = (b, Y, X) of the 2S x 2S grid,
-// FP32 sums over the taps (in order) and the input channels, bias added;
-// then either ReLU and a BF16 row of co values (out16, NHWC) or the FP32
-// value of the one-channel map (out32).  C a multiple of 8.  Dynamic shared
-// memory: 9 C CO floats.
-template <int CO>
-__global__ void __launch_bounds__(256) k_dec_conv(int B, int S, int C, int co, const __nv_bfloat16* __restrict__ x,
-                                                  const __nv_bfloat16* __restrict__ w, int kp,
-                                                  const float* __restrict__ bias, __nv_bfloat16* out16, float* out32) {
-  extern __shared__ float sw[];
-  stage_weights<CO>(sw, C, co, w, kp);
-  const int S2 = 2 * S, img = S2 * S2;
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= B * img) return;
-  const int b = p / img, r = p % img;
-  const int Y = r / S2, X = r % S2;
-  float acc[CO];
+// Direct forward convolution of a level with CO = 1 or 8 output channels: a
+// thread per input cell (b, y0, x0), whose 2 x 2 output pixels share the
+// weights' reads and, upsampled from 3 x 3 input cells, most of the inputs'.
+// Per pixel FP32 sums over the taps (in order) and the input channels, bias
+// added; then either ReLU and a BF16 row of CO values (out16, NHWC) or the FP32
+// value of the one-channel map (out32).  A tap in the zero padding adds
+// products with 0, which leave a sum as it is; with weights that are not
+// finite (GUARD) it is passed over.  C a multiple of 8.  Dynamic shared memory:
+// 9 C CO floats.  Bound by the FP32 issue (36 C CO products a cell, two to an
+// instruction for CO = 8).  A thread per pixel read the weights four times as
+// often: at a batch of 512, 212 us for the map's level and 170 us for the
+// 8-channel one, against 69 and 107 here
+template <int CO, bool GUARD>
+__device__ __forceinline__ void conv_cell(int S, int C, int b, int y0, int x0, const __nv_bfloat16* __restrict__ x,
+                                          const float* sw, const float* __restrict__ bias, __nv_bfloat16* out16,
+                                          float* out32) {
+  constexpr int NP = CO == 8 ? 4 : 1;
+  const int S2 = 2 * S;
+  fpair acc2[4][NP];
+  float acc[4];
 #pragma unroll
-  for (int o = 0; o < CO; ++o) acc[o] = 0.f;
+  for (int i = 0; i < 4; ++i) {
+    acc[i] = 0.f;
+#pragma unroll
+    for (int o = 0; o < NP; ++o) acc2[i][o] = 0;
+  }
+#pragma unroll
   for (int tap = 0; tap < 9; ++tap) {
-    const int Yu = Y + tap / 3 - 1, Xu = X + tap % 3 - 1;
-    if (Yu < 0 || Yu >= S2 || Xu < 0 || Xu >= S2) continue;
-    const __nv_bfloat16* xr = x + (((size_t)b * S + (Yu >> 1)) * S + (Xu >> 1)) * C;
-    const float* wt = sw + tap * C * CO;
+    const int ty = tap / 3, tx = tap % 3;
+#pragma unroll 1
     for (int c8 = 0; c8 < C; c8 += 8) {
-      float xv[8];
-      load_bf16<8>(xr + c8, xv);
+      uint4 v[4];  // pixel (a, e) = i reads input cell (y0 + dy, x0 + dx) through the tap
+      bool in[4];
 #pragma unroll
-      for (int g = 0; g < 8; ++g)
-#pragma unroll
-        for (int o = 0; o < CO; ++o) acc[o] = fmaf(xv[g], wt[(c8 + g) * CO + o], acc[o]);
-    }
-  }
-  if (out16) {
-#pragma unroll
-    for (int o = 0; o < CO; ++o)
-      if (o < co) out16[(size_t)p * co + o] = __float2bfloat16(fmaxf(acc[o] + bias[o], 0.f));
-  } else {
-    out32[p] = acc[0] + bias[0];
-  }
-}
-
-// Partial weight and bias gradients of a level over one chunk of output
-// pixels (block z: pixels [z chunk, (z+1) chunk)).  dW[o][k] is the sum over
-// pixels p of dz[p][o] times the im2col value of column k = tap * C + c at p,
-// read from the level input x (B, S, S, C) through the 2x upsampling and the
-// zero padding; db[o] the sum of dz[p][o].  The 9C/G groups of G input
-// channels of one tap are spread over blockIdx.y, KGb = min(9C/G, blockDim)
-// groups per block; thread (slot s, group kg) owns the G channels
-// c0 = (kg % (C/G)) G .. of tap kg / (C/G) and all CO outputs, and takes
-// every NS-th pixel of each staged run of kStage pixels (NS = blockDim / KGb
-// slots); the slots' sums are then added in slot order.  dz holds BF16 rows
-// of ldz values (co used).  part [blocks][co][9C], part_b [blocks][co]
-// (from blockIdx.y = 0).  Dynamic shared memory: dec_dw_smem<CO>(C) bytes.
-constexpr int kStage = 128;
-template <int CO>
-__host__ __device__ constexpr size_t dec_dw_smem(int C) {
-  return (size_t)kStage * CO * 4 + (size_t)kStage * 8 + (size_t)9 * C * CO * 4;
-}
-template <int CO>
-__global__ void __launch_bounds__(256) k_dec_dw(int B, int S, int C, int co, const __nv_bfloat16* __restrict__ dz,
-                                                int ldz, const __nv_bfloat16* __restrict__ x, int chunk,
-                                                float* part, float* part_b) {
-  constexpr int G = dec_group<CO>();
-  extern __shared__ float sm[];
-  float* sdz = sm;                                          // [kStage][CO]
-  int2* spix = reinterpret_cast<int2*>(sdz + kStage * CO);  // (b S, Y << 16 | X); Y = -1 past the end
-  float* sacc = reinterpret_cast<float*>(spix + kStage);    // [9C][CO]
-  const int K = 9 * C, KG = K / G, KGb = min(KG, (int)blockDim.x), NS = (int)blockDim.x / KGb;
-  const int t = threadIdx.x;
-  const int kg = (int)blockIdx.y * KGb + t % KGb, slot = t / KGb;
-  const bool worker = slot < NS && kg < KG;
-  const int tap = kg / (C / G), c0 = (kg % (C / G)) * G;
-  const int dy = tap / 3 - 1, dxo = tap % 3 - 1;
-  const int S2 = 2 * S, img = S2 * S2, P = B * img;
-  const int p0 = blockIdx.x * chunk;
-  float acc[G][CO];
-#pragma unroll
-  for (int g = 0; g < G; ++g)
-#pragma unroll
-    for (int o = 0; o < CO; ++o) acc[g][o] = 0.f;
-  float bsum = 0.f;
-  for (int r0 = 0; r0 < chunk; r0 += kStage) {
-    __syncthreads();  // the previous run is consumed
-    for (int i = t; i < kStage * CO; i += blockDim.x) {
-      const int j = i / CO, o = i % CO;
-      const int p = p0 + r0 + j;
-      sdz[i] = (r0 + j < chunk && p < P && o < co) ? __bfloat162float(dz[(size_t)p * ldz + o]) : 0.f;
-    }
-    for (int j = t; j < kStage; j += blockDim.x) {
-      const int p = p0 + r0 + j;
-      int2 v = make_int2(0, -4 * 65536);  // row -4: every tap outside the grid
-      if (r0 + j < chunk && p < P) {
-        const int b = p / img, r = p % img;
-        v = make_int2(b * S, (r / S2) << 16 | (r % S2));
-      }
-      spix[j] = v;
-    }
-    __syncthreads();
-    if (t < co)
-      for (int j = 0; j < kStage; ++j) bsum += sdz[j * CO + t];
-    if (worker) {
-      for (int j = slot; j < kStage; j += NS) {
-        const int2 v = spix[j];
-        const int Yu = (v.y >> 16) + dy, Xu = (v.y & 0xffff) + dxo;
-        if (Yu < 0 || Yu >= S2 || Xu < 0 || Xu >= S2) continue;
-        float xv[G];
-        load_bf16<G>(x + ((size_t)(v.x + (Yu >> 1)) * S + (Xu >> 1)) * C + c0, xv);
-        const float* d = sdz + j * CO;
-#pragma unroll
-        for (int o = 0; o < CO; ++o) {
-          const float dv = d[o];
-#pragma unroll
-          for (int g = 0; g < G; ++g) acc[g][o] = fmaf(dv, xv[g], acc[g][o]);
+      for (int i = 0; i < 4; ++i) {
+        const int a = i >> 1, e = i & 1;
+        const int yy = y0 + (a + ty + 1) / 2 - 1, xx = x0 + (e + tx + 1) / 2 - 1;
+        if (e == 1 && tx != 0 && tx != 2) {
+          v[i] = v[i - 1], in[i] = in[i - 1];  // the cell of the pixel to the left
+        } else if (a == 1 && ty == 1) {
+          v[i] = v[i - 2], in[i] = in[i - 2];  // of the pixel above
+        } else {
+          v[i] = make_uint4(0u, 0u, 0u, 0u);
+          in[i] = yy >= 0 && yy < S && xx >= 0 && xx < S;
+          if (in[i]) v[i] = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * S + yy) * S + xx) * C + c8));
         }
       }
-    }
-  }
-  // the slots' sums, added in slot order
-  for (int i = t; i < K * CO; i += blockDim.x) sacc[i] = 0.f;
-  for (int s = 0; s < NS; ++s) {
-    __syncthreads();
-    if (worker && slot == s)
+      const float* wt = sw + (tap * C + c8) * CO;
+      if constexpr (CO == 8) {
 #pragma unroll
-      for (int g = 0; g < G; ++g)
+        for (int g = 0; g < 8; ++g) {
+          const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(wt + g * 8);
+          const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(wt + g * 8 + 4);
 #pragma unroll
-        for (int o = 0; o < CO; ++o) sacc[(kg * G + g) * CO + o] += acc[g][o];
-  }
-  __syncthreads();
-  const int kb = (int)blockIdx.y * KGb * G, kn = min(K - kb, KGb * G);  // this block's columns
-  for (int i = t; i < co * kn; i += blockDim.x) {
-    const int o = i / kn, k = kb + i % kn;
-    part[((size_t)blockIdx.x * co + o) * K + k] = sacc[k * CO + o];
-  }
-  if (blockIdx.y == 0 && t < co) part_b[(size_t)blockIdx.x * co + t] = bsum;
-}
-
-// Gradient of the level input x (B, S, S, C) from the output gradient dz
-// (B, 2S, 2S pixels of ldz BF16 values, co used) and the weights w [co][kp]:
-// the 3x3 correlation transposed, summed over the 2x2 cells each input cell
-// was copied to.  One thread per input cell and group of G channels, the
-// cell varying fastest (a warp reads the same weights), FP32 sums in a fixed
-// order.  dz rows of ldz values are 16-byte aligned when co > 1 (co a
-// multiple of 8).  mask (optional): x's own values, the ReLU derivative
-// applied (x > 0).  Sample b's S*S*C values go to dx + b * ld + col0.
-// Dynamic shared memory: 9 C CO floats.
-template <int CO>
-__global__ void __launch_bounds__(256) k_dec_dx(int B, int S, int C, int co, const __nv_bfloat16* __restrict__ dz,
-                                                int ldz, const __nv_bfloat16* __restrict__ w, int kp,
-                                                const __nv_bfloat16* __restrict__ mask, float* dx, int ld,
-                                                int col0) {
-  constexpr int G = dec_group<CO>();
-  extern __shared__ float sw[];
-  stage_weights<CO>(sw, C, co, w, kp);
-  const int ncell = B * S * S;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncell * (C / G)) return;
-  const int c0 = (t / ncell) * G;
-  const int q = t % ncell;  // input cell
-  const int x0 = q % S, y0 = (q / S) % S, b = q / (S * S);
-  const int S2 = 2 * S;
-  const int nq = co / 8;  // 16-byte loads of a dz row (co > 1)
-  float acc[G];
-#pragma unroll
-  for (int g = 0; g < G; ++g) acc[g] = 0.f;
-  for (int a = 0; a < 2; ++a)
-    for (int e = 0; e < 2; ++e) {
-      const int Yu = 2 * y0 + a, Xu = 2 * x0 + e;  // the upsampled cell
-      for (int ty = 0; ty < 3; ++ty) {
-        const int Y = Yu - (ty - 1);  // output row that read (Yu, Xu) through tap ty
-        if (Y < 0 || Y >= S2) continue;
-        for (int tx = 0; tx < 3; ++tx) {
-          const int X = Xu - (tx - 1);
-          if (X < 0 || X >= S2) continue;
-          const __nv_bfloat16* g = dz + (((size_t)b * S2 + Y) * S2 + X) * ldz;
-          float dv[CO];
-          if constexpr (CO == 1) {
-            dv[0] = __bfloat162float(g[0]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < CO / 8; ++i) {
-              float t8[8];
-              if (i < nq) {
-                unpack8(__ldg(reinterpret_cast<const uint4*>(g) + i), t8);
-              } else {
-#pragma unroll
-                for (int h = 0; h < 8; ++h) t8[h] = 0.f;
-              }
-#pragma unroll
-              for (int h = 0; h < 8; ++h) dv[8 * i + h] = t8[h];
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t q = g < 2 ? v[i].x : g < 4 ? v[i].y : g < 6 ? v[i].z : v[i].w;
+            const uint32_t f = g & 1 ? q & 0xffff0000u : q << 16;
+            const fpair d = pair_of(f, f);
+            if (!GUARD || in[i]) {
+              pair_fma(acc2[i][0], d, w0.x);
+              pair_fma(acc2[i][1], d, w0.y);
+              pair_fma(acc2[i][2], d, w1.x);
+              pair_fma(acc2[i][3], d, w1.y);
             }
           }
-          const float* wt = sw + ((ty * 3 + tx) * C + c0) * CO;
+        }
+      } else {
+        const float4 w0 = *reinterpret_cast<const float4*>(wt), w1 = *reinterpret_cast<const float4*>(wt + 4);
+        const float f[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-          for (int gg = 0; gg < G; ++gg)
+        for (int i = 0; i < 4; ++i) {
+          float xv[8];
+          unpack8(v[i], xv);
+          if (!GUARD || in[i]) {
 #pragma unroll
-            for (int o = 0; o < CO; ++o) acc[gg] = fmaf(dv[o], wt[gg * CO + o], acc[gg]);
+            for (int g = 0; g < 8; ++g) acc[i] = fmaf(xv[g], f[g], acc[i]);
+          }
         }
       }
     }
-  const size_t i0 = (size_t)q * C + c0;  // index of the first channel in x
-  float* out = dx + (size_t)b * ld + col0 + (i0 - (size_t)b * S * S * C);
+  }
 #pragma unroll
-  for (int gg = 0; gg < G; ++gg) {
-    float v = acc[gg];
-    if (mask && !(__bfloat162float(mask[i0 + gg]) > 0.f)) v = 0.f;
-    out[gg] = v;
+  for (int a = 0; a < 2; ++a) {
+    const size_t p = ((size_t)b * S2 + 2 * y0 + a) * S2 + 2 * x0;
+    if constexpr (CO == 8) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        uint32_t w[4];
+#pragma unroll
+        for (int o = 0; o < 4; ++o) {
+          const fpair r = acc2[2 * a + e][o];
+          const __nv_bfloat162 h = __floats2bfloat162_rn(fmaxf(pair_lo(r) + bias[2 * o], 0.f),
+                                                         fmaxf(pair_hi(r) + bias[2 * o + 1], 0.f));
+          w[o] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(out16 + (p + e) * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    } else {
+      *reinterpret_cast<float2*>(out32 + p) = make_float2(acc[2 * a] + bias[0], acc[2 * a + 1] + bias[0]);
+    }
+  }
+}
+template <int CO>
+__global__ void __launch_bounds__(256) k_dec_conv(int B, int S, int C, const __nv_bfloat16* __restrict__ x,
+                                                  const __nv_bfloat16* __restrict__ w, int kp,
+                                                  const float* __restrict__ bias, __nv_bfloat16* out16, float* out32) {
+  extern __shared__ __align__(16) float sw[];
+  const bool finite = stage_weights<false>(sw, C, CO, w, kp);
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= B * S * S) return;
+  const int b = q / (S * S), y0 = (q / S) % S, x0 = q % S;
+  if (finite)
+    conv_cell<CO, false>(S, C, b, y0, x0, x, sw, bias, out16, out32);
+  else
+    conv_cell<CO, true>(S, C, b, y0, x0, x, sw, bias, out16, out32);
+}
+
+// The weight gradients of a level are sums over the input cells.  The 2x upsampling
+// makes four upsampled cells of an input cell (y0, x0), and through tap (ty, tx)
+// these are read by the four output pixels in rows 2 y0 + 1 - ty, 2 y0 + 2 - ty
+// and columns 2 x0 + 1 - tx, 2 x0 + 2 - tx.  So with D[tap][o] the sum of the
+// output gradient over those four pixels (inside the grid),
+//   dW[o][tap][c] = sum over cells of D[tap][o] x[c]
+//   db[o]         = sum over cells of D[centre][o]
+// a quarter of the products of the sums over output pixels, and the nine D of a
+// cell come from one window of 4 x 4 pixels.
+
+// The 8 gradients o0 .. o0 + 7 of pixel (Y, X), as FP32 pairs; 0 outside.
+__device__ __forceinline__ void dz_pixel(const __nv_bfloat16* __restrict__ dz, int b, int S2, int Y, int X, int co,
+                                         int o0, fpair (&v)[4]) {
+  uint4 q = make_uint4(0u, 0u, 0u, 0u);
+  if (Y >= 0 && Y < S2 && X >= 0 && X < S2)
+    q = __ldg(reinterpret_cast<const uint4*>(dz + (((size_t)b * S2 + Y) * S2 + X) * co + o0));
+  v[0] = pair_bf16(q.x);
+  v[1] = pair_bf16(q.y);
+  v[2] = pair_bf16(q.z);
+  v[3] = pair_bf16(q.w);
+}
+
+// Columns X .. X + N + 1 of row Y of the one-channel gradient, 0 outside; X odd,
+// N even: the N in the middle are read in pairs.
+template <int N>
+__device__ __forceinline__ void dz_row(const __nv_bfloat16* __restrict__ dz, int b, int S2, int Y, int X,
+                                       float (&v)[N + 2]) {
+#pragma unroll
+  for (int j = 0; j < N + 2; ++j) v[j] = 0.f;
+  if (Y < 0 || Y >= S2) return;
+  const __nv_bfloat16* r = dz + ((size_t)b * S2 + Y) * S2;
+  if (X >= 0) v[0] = __bfloat162float(r[X]);
+#pragma unroll
+  for (int j = 1; j < N + 1; j += 2)
+    if (X + j < S2) {
+      const uint32_t q = __ldg(reinterpret_cast<const unsigned int*>(r + X + j));
+      v[j] = __uint_as_float(q << 16);
+      v[j + 1] = __uint_as_float(q & 0xffff0000u);
+    }
+  if (X + N + 1 < S2) v[N + 1] = __bfloat162float(r[X + N + 1]);
+}
+
+// Partial weight and bias gradients of a level with co (a multiple of 8) output
+// channels over one chunk of input cells (block z: cells [z chunk, (z+1) chunk)).
+// Per run of STAGE cells the block puts D and x as FP32 into shared memory, a row
+// of STAGE + 4 floats for each of the 9 co (tap, o) and of its channels, and
+// multiplies them: thread (slot, mm, nn) holds the 8 x 4 sums of rows mm + i mt
+// and channels nn + j nb (mt = 9 co / 8; neighbouring threads read neighbouring
+// rows, in other banks), and takes every NS-th group of 4 cells, two cells to a
+// packed product.  12 16-byte reads of shared memory feed 128 products.  The
+// slots' sums are then added in slot order.  Channels beyond 4 nb go to further
+// blockIdx.y.  part [blocks][co][9C], part_b [blocks][co] (from blockIdx.y = 0).
+// At a batch of 512, 32 -> 16 and 16 -> 8 channels took 322 and 323 us with a
+// thread per column that walked the output pixels; 75 each here, most
+// of it staging and the reads of shared memory (604 M products each).
+constexpr int kDwTiles = 512;    // most threads of a slot
+constexpr int kDwThreads = 160;  // threads wanted in a block: at 128 registers, three blocks an SM
+constexpr int dw_stage(int co) { return co <= 8 ? 128 : 64; }
+struct DwPlan {  // of co output and C input channels
+  int nb, slots, threads, smem;
+};
+inline DwPlan dw_plan(int co, int C) {
+  const int mt = 9 * co / 8, stage = dw_stage(co);
+  DwPlan p;
+  p.nb = std::min(C / 4, kDwTiles / mt) & ~1;  // at least 2 (mt <= 72): whole groups of 8 channels
+  p.slots = std::max(1, std::min(stage / 4, kDwThreads / (mt * p.nb)));
+  p.threads = (mt * p.nb * p.slots + 31) / 32 * 32;
+  p.smem = std::max((9 * co + 4 * p.nb) * (stage + 4), p.slots > 1 ? mt * p.nb * 33 : 0) * 4 + co * 4;
+  return p;
+}
+template <int STAGE>
+__global__ void __launch_bounds__(kDwTiles) k_dec_dw(int cells, int S, int C, int co, int nb, int slots,
+                                                     const __nv_bfloat16* __restrict__ dz,
+                                                     const __nv_bfloat16* __restrict__ x, int chunk, float* part,
+                                                     float* part_b) {
+  constexpr int LD = STAGE + 4;
+  extern __shared__ __align__(16) float sm[];
+  const int M = 9 * co, mt = M / 8, T = mt * nb, S2 = 2 * S;
+  const int cb = blockIdx.y * 4 * nb, cn = min(4 * nb, C - cb), nl = cn / 4;  // this block's channels
+  float* sb = sm;                    // [co] bias sums
+  float* sd = sm + co;               // [M][LD]
+  float* sx = sd + (size_t)M * LD;   // [cn][LD]
+  const int t = threadIdx.x, slot = t / T, tt = t % T, mm = tt % mt, nn = tt / mt;
+  const bool worker = slot < slots && nn < nl;
+  const int q0 = blockIdx.x * chunk, n = min(chunk, cells - q0);
+  fpair acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  for (int o = t; o < co; o += blockDim.x) sb[o] = 0.f;
+  for (int r0 = 0; r0 < n; r0 += STAGE) {
+    __syncthreads();  // the previous run is consumed
+    const int nd = STAGE * (co / 8), all = nd + STAGE * (cn / 8);
+    for (int k = t; k < all; k += blockDim.x) {
+      const bool isd = k < nd;
+      const int j = k % STAGE, g = 8 * ((isd ? k : k - nd) / STAGE);  // cell, first of 8 channels
+      const int q = q0 + r0 + j;
+      const bool in = r0 + j < n;
+      if (isd) {
+        const int b = q / (S * S), y0 = (q / S) % S, x0 = q % S;
+        float* to = sd + (size_t)g * LD + j;
+        fpair h[3][4];  // sums of neighbouring columns, the row above
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          fpair p[4][4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            dz_pixel(dz, b, S2, in ? 2 * y0 - 1 + r : -1, 2 * x0 - 1 + e, co, g, p[e]);
+#pragma unroll
+          for (int e = 0; e < 3; ++e)
+#pragma unroll
+            for (int o = 0; o < 4; ++o) {
+              const fpair s = pair_add(p[e][o], p[e + 1][o]);
+              if (r > 0) {
+                const fpair d = pair_add(h[e][o], s);  // tap (3 - r, 2 - e)
+                float* at = to + (size_t)((3 * (3 - r) + 2 - e) * co + 2 * o) * LD;
+                at[0] = pair_lo(d);
+                at[LD] = pair_hi(d);
+              }
+              h[e][o] = s;
+            }
+        }
+      } else {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (in) v = __ldg(reinterpret_cast<const uint4*>(x + (size_t)q * C + cb + g));
+        float f[8];
+        unpack8(v, f);
+        float* to = sx + (size_t)g * LD + j;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) to[i * LD] = f[i];
+      }
+    }
+    __syncthreads();
+    if (blockIdx.y == 0)  // db: the centre tap's sums, a warp per channel
+      for (int o = t >> 5; o < co; o += blockDim.x >> 5) {
+        const float* d = sd + (size_t)(4 * co + o) * LD;
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < STAGE; j += 32) s += d[j + (t & 31)];
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+        if ((t & 31) == 0) sb[o] += s;
+      }
+    if (worker) {
+      const float* d0 = sd + (size_t)mm * LD;
+      const float* x0 = sx + (size_t)nn * LD;
+#pragma unroll 1
+      for (int k = 4 * slot; k < STAGE; k += 4 * slots) {
+        ulonglong2 xv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xv[j] = *reinterpret_cast<const ulonglong2*>(x0 + (size_t)j * nl * LD + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(d0 + (size_t)i * mt * LD + k);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            pair_fma(acc[i][j], d.x, xv[j].x);
+            pair_fma(acc[i][j], d.y, xv[j].y);
+          }
+        }
+      }
+    }
+  }
+  float v[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) v[k] = pair_lo(acc[k / 4][k % 4]) + pair_hi(acc[k / 4][k % 4]);
+  __syncthreads();
+  if (blockIdx.y == 0)
+    for (int o = t; o < co; o += blockDim.x) part_b[(size_t)blockIdx.x * co + o] = sb[o];
+  if (slots > 1) {  // added in slot order
+    float* sacc = sd + tt * 33;
+    for (int s = 0; s < slots; ++s) {
+      if (worker && slot == s)
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+          if (s > 0) v[k] += sacc[k];
+          sacc[k] = v[k];
+        }
+      __syncthreads();
+    }
+  }
+  if (worker && slot == slots - 1)
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      const int row = mm + k / 4 * mt, c = cb + nn + k % 4 * nl;
+      part[((size_t)blockIdx.x * co + row % co) * 9 * C + row / co * C + c] = v[k];
+    }
+}
+
+// The same for one output channel (the map's level): a thread per input cell of
+// the chunk, stepping by the block, and the 8 channels from 8 blockIdx.y; its 72
+// sums stay in registers, then the block's are added in a fixed order.  278 us at
+// a batch of 512 before, 55 here (151 M products; loads of pairs and single values).
+constexpr int kDw1Threads = 160;
+__global__ void __launch_bounds__(kDw1Threads) k_dec_dw1(int cells, int S, int C, const __nv_bfloat16* __restrict__ dz,
+                                                         const __nv_bfloat16* __restrict__ x, int chunk, float* part,
+                                                         float* part_b) {
+  __shared__ float red[kDw1Threads / 32][73];
+  const int S2 = 2 * S, cb = 8 * blockIdx.y;
+  const int q0 = blockIdx.x * chunk, q1 = min(q0 + chunk, cells);
+  float acc[73];  // [tap][channel], then the bias
+#pragma unroll
+  for (int k = 0; k < 73; ++k) acc[k] = 0.f;
+  for (int q = q0 + threadIdx.x; q < q1; q += kDw1Threads) {
+    const int b = q / (S * S), y0 = (q / S) % S, x0 = q % S;
+    float xv[8];
+    unpack8(__ldg(reinterpret_cast<const uint4*>(x + (size_t)q * C + cb)), xv);
+    float p[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) dz_row<2>(dz, b, S2, 2 * y0 - 1 + r, 2 * x0 - 1, p[r]);
+#pragma unroll
+    for (int ty = 0; ty < 3; ++ty)
+#pragma unroll
+      for (int tx = 0; tx < 3; ++tx) {
+        const int r = 2 - ty, e = 2 - tx;
+        const float d = (p[r][e] + p[r][e + 1]) + (p[r + 1][e] + p[r + 1][e + 1]);
+        if (ty == 1 && tx == 1) acc[72] += d;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) acc[(ty * 3 + tx) * 8 + g] = fmaf(d, xv[g], acc[(ty * 3 + tx) * 8 + g]);
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < 73; ++k) {
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], w);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = acc[k];
+  }
+  __syncthreads();
+  const int k = threadIdx.x;
+  if (k < 73) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kDw1Threads / 32; ++w) s += red[w][k];
+    if (k < 72)
+      part[(size_t)blockIdx.x * 9 * C + k / 8 * C + cb + k % 8] = s;
+    else if (blockIdx.y == 0)
+      part_b[blockIdx.x] = s;
+  }
+}
+
+// Writes the gradients of 8 channels of an input cell: the ReLU derivative
+// applied (mask: x's own values, x > 0), as a BF16 row (the output gradient of
+// the level above) or as FP32.
+__device__ __forceinline__ void dx_store(const float (&v)[8], const __nv_bfloat16* mask, size_t at, size_t to,
+                                         __nv_bfloat16* dx16, float* dx32) {
+  float m[8], r[8];
+  unpack8(__ldg(reinterpret_cast<const uint4*>(mask + at)), m);
+#pragma unroll
+  for (int g = 0; g < 8; ++g) r[g] = m[g] > 0.f ? v[g] : 0.f;
+  if (dx16) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(r[2 * i], r[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(dx16 + at) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+#pragma unroll
+    for (int g = 0; g < 8; ++g) dx32[to + g] = r[g];
+  }
+}
+
+// Gradient of the level input x (B, S, S, C) from the output gradient dz (B, 2S,
+// 2S pixels of co BF16 values) and the weights w [co][kp], with x's ReLU
+// derivative: BF16 rows (dx16), or FP32 with sample b's S S C values at dx32 +
+// b ld + col0.  The 3x3 correlation transposed, summed over the 2x2 upsampled
+// cells of each input cell: FP32 sums over (cell, tap, o) in order, a channel
+// each (the sums over D above would round otherwise, and what is rounded here
+// goes through every layer below).  A thread takes two cells, one below the
+// other, so that neighbouring lanes read neighbouring pixels, and G channels (16,
+// or 8 where C is no multiple of 16): 16 bytes of weights from shared memory serve
+// 8 products.  A pixel in the zero padding adds products with 0, which leave a sum
+// as it is; with weights that are not finite (GUARD) it is passed over.  Dynamic
+// shared memory: 9 C co floats, [tap][o][c].  36 C co products a cell, 65 us of
+// FP32 issue at a batch of 512 for 32 <- 16 and for 16 <- 8 channels; these took
+// 432 and 230 us with a cell and 2 or 4 channels a thread, 165 and 144 here.  Two
+// cells side by side: 187 and 141; 8 channels: 190 and 156; four cells: 185 and 142;
+// packed products: 157 each, the copies into pairs costing what they save.
+constexpr int kDxThreads = 128, kDxCells = 2;
+template <int G, bool GUARD>
+__device__ __forceinline__ void dx_cells(int S, int C, int co, int b, int y0, int x0, int c0,
+                                         const __nv_bfloat16* __restrict__ dz, const float* sw, float (&acc)[kDxCells][G]) {
+  const int S2 = 2 * S;
+#pragma unroll 1
+  for (int ae = 0; ae < 4; ++ae) {
+    const int Yu = 2 * y0 + (ae >> 1), Xu = 2 * x0 + (ae & 1);  // the upsampled cell
+#pragma unroll 1
+    for (int ty = 0; ty < 3; ++ty) {
+      const int Y = Yu - (ty - 1);  // output row that read it through tap ty
+#pragma unroll
+      for (int tx = 0; tx < 3; ++tx) {
+        const int X = Xu - (tx - 1);
+        const __nv_bfloat16* px = dz + (((ptrdiff_t)b * S2 + Y) * S2 + X) * co;
+        bool in[kDxCells];
+#pragma unroll
+        for (int m = 0; m < kDxCells; ++m) in[m] = Y + 2 * m >= 0 && Y + 2 * m < S2 && X >= 0 && X < S2;
+        const float* wt = sw + (ty * 3 + tx) * co * C + c0;
+#pragma unroll 1
+        for (int o8 = 0; o8 < co; o8 += 8) {
+          uint4 q[kDxCells];
+#pragma unroll
+          for (int m = 0; m < kDxCells; ++m) {
+            q[m] = make_uint4(0u, 0u, 0u, 0u);
+            if (in[m]) q[m] = __ldg(reinterpret_cast<const uint4*>(px + (ptrdiff_t)(2 * m) * S2 * co + o8));
+          }
+#pragma unroll
+          for (int o = 0; o < 8; ++o) {
+            const float4* wp = reinterpret_cast<const float4*>(wt + (o8 + o) * C);
+            float f[G];
+#pragma unroll
+            for (int k = 0; k < G / 4; ++k) {
+              const float4 v = wp[k];
+              f[4 * k] = v.x, f[4 * k + 1] = v.y, f[4 * k + 2] = v.z, f[4 * k + 3] = v.w;
+            }
+#pragma unroll
+            for (int m = 0; m < kDxCells; ++m) {
+              const uint32_t h = o < 2 ? q[m].x : o < 4 ? q[m].y : o < 6 ? q[m].z : q[m].w;
+              const float d = __uint_as_float(o & 1 ? h & 0xffff0000u : h << 16);
+              if (!GUARD || in[m]) {
+#pragma unroll
+                for (int k = 0; k < G; ++k) acc[m][k] = fmaf(d, f[k], acc[m][k]);
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+}
+template <int G>
+__global__ void __launch_bounds__(kDxThreads) k_dec_dx(int B, int S, int C, int co,
+                                                       const __nv_bfloat16* __restrict__ dz,
+                                                       const __nv_bfloat16* __restrict__ w, int kp,
+                                                       const __nv_bfloat16* __restrict__ x, __nv_bfloat16* dx16,
+                                                       float* dx32, int ld, int col0) {
+  extern __shared__ __align__(16) float sw[];
+  const bool finite = stage_weights<true>(sw, C, co, w, kp);
+  const int pr = (S + kDxCells - 1) / kDxCells, runs = B * S * pr;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= runs * (C / G)) return;
+  const int c0 = t / runs * G, u = t % runs;
+  const int x0 = u % S, y0 = (u / S) % pr * kDxCells, b = u / (pr * S);
+  float acc[kDxCells][G];
+#pragma unroll
+  for (int m = 0; m < kDxCells; ++m)
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc[m][g] = 0.f;
+  if (finite)
+    dx_cells<G, false>(S, C, co, b, y0, x0, c0, dz, sw, acc);
+  else
+    dx_cells<G, true>(S, C, co, b, y0, x0, c0, dz, sw, acc);
+#pragma unroll
+  for (int m = 0; m < kDxCells; ++m) {
+    if (y0 + m >= S) break;
+    const size_t cell = (size_t)(y0 + m) * S + x0;
+#pragma unroll
+    for (int h = 0; h < G; h += 8) {
+      float v[8];
+#pragma unroll
+      for (int g = 0; g < 8; ++g) v[g] = acc[m][h + g];
+      dx_store(v, x, ((size_t)b * S * S + cell) * C + c0 + h, (size_t)b * ld + col0 + cell * C + c0 + h, dx16, dx32);
+    }
+  }
+}
+
+// The same for one output channel (the map's level), the window of 4 x 6 pixels
+// in registers: 105 us at a batch of 512 before, 58 here (two cells and 128 threads: with 256 one block of 158 registers an SM, 92).
+template <bool GUARD>
+__device__ __forceinline__ void dx1_cells(int S, int y0, int x0, const float (&p)[4][6], const float* wt, int C,
+                                          fpair (&acc)[2][4]) {
+#pragma unroll
+  for (int ae = 0; ae < 4; ++ae)
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+      const int r = (ae >> 1) - tap / 3 + 2, e = (ae & 1) - tap % 3 + 2;  // row, column in the window
+      const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(wt + tap * C);
+      const ulonglong2 f0 = wp[0], f1 = wp[1];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const uint32_t h = __float_as_uint(p[r][e + 2 * m]);
+        const fpair d = pair_of(h, h);
+        const int Y = 2 * y0 - 1 + r, X = 2 * x0 - 1 + e + 2 * m;
+        if (!GUARD || (Y >= 0 && Y < 2 * S && X >= 0 && X < 2 * S)) {
+          pair_fma(acc[m][0], d, f0.x);
+          pair_fma(acc[m][1], d, f0.y);
+          pair_fma(acc[m][2], d, f1.x);
+          pair_fma(acc[m][3], d, f1.y);
+        }
+      }
+    }
+}
+__global__ void __launch_bounds__(kDxThreads, 4) k_dec_dx1(int B, int S, int C, const __nv_bfloat16* __restrict__ dz,
+                                                 const __nv_bfloat16* __restrict__ w, int kp,
+                                                 const __nv_bfloat16* __restrict__ x, __nv_bfloat16* dx16) {
+  extern __shared__ __align__(16) float sw[];
+  const bool finite = stage_weights<true>(sw, C, 1, w, kp);
+  const int pr = (S + 1) / 2, runs = B * S * pr, S2 = 2 * S;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= runs * (C / 8)) return;
+  const int c0 = t / runs * 8, u = t % runs;
+  const int x0 = u % pr * 2, y0 = (u / pr) % S, b = u / (pr * S);
+  float p[4][6];
+  fpair acc[2][4] = {};
+#pragma unroll
+  for (int r = 0; r < 4; ++r) dz_row<4>(dz, b, S2, 2 * y0 - 1 + r, 2 * x0 - 1, p[r]);
+  if (finite)
+    dx1_cells<false>(S, y0, x0, p, sw + c0, C, acc);
+  else
+    dx1_cells<true>(S, y0, x0, p, sw + c0, C, acc);
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    float v[8];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) v[2 * g] = pair_lo(acc[m][g]), v[2 * g + 1] = pair_hi(acc[m][g]);
+    if (x0 + m < S) dx_store(v, x, (((size_t)b * S + y0) * S + x0 + m) * C + c0, 0, dx16, nullptr);
   }
 }
 

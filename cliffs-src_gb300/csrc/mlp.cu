@@ -268,9 +268,8 @@ struct cliffs_mlp {
   bf16* X[3] = {nullptr, nullptr, nullptr};  // decoder level inputs, NHWC
   float* map = nullptr;                      // [cap][side2]
   bf16* col = nullptr;                       // im2col [P][kp]
-  float* dzf = nullptr;  // a level's output gradient, FP32 [P][Cout]
-  bf16* dzb = nullptr;   // ... in BF16 [P][pad16(Cout)]
-  float* dxf = nullptr;  // a level's input gradient (levels 1, 2)
+  float* dzf = nullptr;  // the map's gradient, FP32
+  bf16* dzb[2] = {};     // a level's output gradient, BF16 [P][Cout], and the next one's
   float* wpart = nullptr;  // partials of a weight gradient over chunks of pixels
   float* cpart = nullptr;  // partials of a bias gradient over chunks of pixels
   float* part2 = nullptr;  // map loss partial sums
@@ -284,12 +283,12 @@ constexpr int kLossBlocks = 64;
 constexpr int kMapLossBlocks = 1024;  // the map loss: B x side^2 values
 
 void free_decoder(cliffs_mlp* m) {
-  void* p[] = {m->X[0], m->X[1], m->X[2], m->map, m->col, m->dzf, m->dzb, m->dxf, m->wpart, m->cpart, m->part2};
+  void* p[] = {m->X[0], m->X[1], m->X[2], m->map, m->col, m->dzf, m->dzb[0], m->dzb[1], m->wpart, m->cpart, m->part2};
   for (void* q : p)
     if (q) cudaFree(q);
   m->X[0] = m->X[1] = m->X[2] = nullptr;
-  m->col = m->dzb = nullptr;
-  m->map = m->dzf = m->dxf = m->wpart = m->cpart = m->part2 = nullptr;
+  m->col = m->dzb[0] = m->dzb[1] = nullptr;
+  m->map = m->dzf = m->wpart = m->cpart = m->part2 = nullptr;
 }
 
 void free_all(cliffs_mlp* m) {
@@ -330,18 +329,16 @@ Level level(const cliffs_mlp* m, int l) {
   v.kp = pad16(v.K);
   return v;
 }
-constexpr int kDwChunk = 512;  // least output pixels per partial of a decoder weight gradient
-
-// Output pixels per partial of a level's weight gradient (P pixels) (a multiple of
-// kStage; at most ~2048 partials), and the number of partials.
-int dw_chunk(long long P) {
-  const long long c = std::max<long long>(kDwChunk, ((P + 2047) / 2048 + kStage - 1) / kStage * kStage);
-  return (int)c;
+// Input cells per partial of a level's weight gradient (cells in all): at most
+// kDwPartials partials, three blocks on each of 152 SMs, so that they run at once;
+// their number and size do not depend on the device.
+constexpr int kDwChunk = 256, kDwPartials = 456;
+int dw_chunk(long long cells) {
+  return (int)std::max<long long>(kDwChunk, (cells + 64ll * kDwPartials - 1) / (64ll * kDwPartials) * 64);
 }
-int dw_blocks(long long P) { return (int)((P + dw_chunk(P) - 1) / dw_chunk(P)); }
-
-// The direct kernels' output-channel class: CO >= cout of 1, 8, 16, 32, 64.
-int co_class(int cout) { return cout <= 1 ? 1 : cout <= 8 ? 8 : cout <= 16 ? 16 : cout <= 32 ? 32 : 64; }
+int dw_blocks(long long cells) { return (int)((cells + dw_chunk(cells) - 1) / dw_chunk(cells)); }
+// Most partials of any batch with at most this many cells.
+size_t dw_most(long long cells) { return std::min<long long>(kDwPartials, (cells + kDwChunk - 1) / kDwChunk); }
 
 // Activation buffers for batches up to cap.
 int ensure_cap(cliffs_mlp* m, int cap) {
@@ -369,21 +366,19 @@ int ensure_cap(cliffs_mlp* m, int cap) {
     return CLIFFS_ERR_NOMEM;
   if (m->d.map_side > 0) {
     free_decoder(m);
-    size_t col = 0, dz = 0, dzp = 0, dx = 0, wp = 0, bp = 0;
+    size_t col = 0, dzp = 0, wp = 0, bp = 0;
     for (int l = 0; l < 3; ++l) {
       const Level v = level(m, l);
       const size_t P = (size_t)cap * 4 * v.S * v.S;
       if (v.cout >= 16) col = std::max(col, P * v.kp);  // im2col of the tensor-core levels
-      dz = std::max(dz, P * v.cout);
       dzp = std::max(dzp, P * v.cout);
-      if (l > 0) dx = std::max(dx, (size_t)cap * v.S * v.S * v.cin);
-      wp = std::max(wp, (size_t)dw_blocks((long long)P) * v.cout * v.K);
-      bp = std::max(bp, (size_t)dw_blocks((long long)P) * v.cout);
+      wp = std::max(wp, dw_most((long long)P / 4) * v.cout * v.K);
+      bp = std::max(bp, dw_most((long long)P / 4) * v.cout);
       if (dalloc(&m->X[l], (size_t)cap * v.S * v.S * v.cin)) return CLIFFS_ERR_NOMEM;
     }
     if (dalloc(&m->map, (size_t)cap * m->side2) || dalloc(&m->col, col) ||
-        dalloc(&m->dzf, std::max(dz, dx)) || dalloc(&m->dzb, dzp) ||
-        dalloc(&m->dxf, std::max(dz, dx)) || dalloc(&m->wpart, wp) || dalloc(&m->cpart, bp) ||
+        dalloc(&m->dzf, (size_t)cap * m->side2) || dalloc(&m->dzb[0], dzp) ||
+        dalloc(&m->dzb[1], dzp) || dalloc(&m->wpart, wp) || dalloc(&m->cpart, bp) ||
         dalloc(&m->part2, kMapLossBlocks))
       return CLIFFS_ERR_NOMEM;
   }
@@ -466,33 +461,57 @@ void smem_limit(Kernel* k, size_t bytes) {
 
 template <int CO>
 void dec_conv_launch(cliffs_mlp* m, int B, const Level& v, const Layer& y, bf16* out16, float* out32) {
-  const long long P = (long long)B * 4 * v.S * v.S;
   const size_t sh = (size_t)9 * v.cin * CO * 4;
   smem_limit(k_dec_conv<CO>, sh);
-  k_dec_conv<CO><<<blocks256(P), 256, sh, m->stream>>>(B, v.S, v.cin, v.cout, m->X[v.lvl], y.W, y.kp, y.b, out16,
-                                                       out32);
+  k_dec_conv<CO><<<blocks256((long long)B * v.S * v.S), 256, sh, m->stream>>>(B, v.S, v.cin, m->X[v.lvl], y.W, y.kp,
+                                                                             y.b, out16, out32);
 }
 
-template <int CO>
-void dec_dw_launch(cliffs_mlp* m, int B, const Level& v) {
-  constexpr int G = dec_group<CO>();
-  const long long P = (long long)B * 4 * v.S * v.S;
-  const int KG = v.K / G, KGb = std::min(KG, 256), threads = KGb * std::max(1, 256 / KGb);
-  const size_t sh = dec_dw_smem<CO>(v.cin);
-  smem_limit(k_dec_dw<CO>, sh);
-  const dim3 grid(dw_blocks(P), (KG + KGb - 1) / KGb);
-  k_dec_dw<CO><<<grid, threads, sh, m->stream>>>(B, v.S, v.cin, v.cout, m->dzb, v.cout, m->X[v.lvl],
-                                                 dw_chunk(P), m->wpart, m->cpart);
+// Partials of a level's weight and bias gradients from its output gradient dz.
+void dec_dw_launch(cliffs_mlp* m, int B, const Level& v, const bf16* dz) {
+  const int cells = B * v.S * v.S, chunk = dw_chunk(cells), nb = dw_blocks(cells);
+  const bf16* x = m->X[v.lvl];
+  if (v.cout == 1) {
+    k_dec_dw1<<<dim3(nb, v.cin / 8), kDw1Threads, 0, m->stream>>>(cells, v.S, v.cin, dz, x, chunk, m->wpart,
+                                                                  m->cpart);
+    return;
+  }
+  const DwPlan p = dw_plan(v.cout, v.cin);
+  const dim3 grid(nb, (v.cin / 4 + p.nb - 1) / p.nb);
+  auto go = [&](auto kernel) {
+    smem_limit(kernel, p.smem);
+    kernel<<<grid, p.threads, p.smem, m->stream>>>(cells, v.S, v.cin, v.cout, p.nb, p.slots, dz, x, chunk, m->wpart,
+                                                   m->cpart);
+  };
+  if (dw_stage(v.cout) == 128)
+    go(k_dec_dw<128>);
+  else
+    go(k_dec_dw<64>);
 }
 
-template <int CO>
-void dec_dx_launch(cliffs_mlp* m, int B, const Level& v, const Layer& y, float* dx, int ld, int col0) {
-  constexpr int G = dec_group<CO>();
-  const long long n = (long long)B * v.S * v.S * (v.cin / G);
-  const size_t sh = (size_t)9 * v.cin * CO * 4;
-  smem_limit(k_dec_dx<CO>, sh);
-  k_dec_dx<CO><<<blocks256(n), 256, sh, m->stream>>>(B, v.S, v.cin, v.cout, m->dzb, v.cout, y.W, y.kp,
-                                                     m->X[v.lvl], dx, ld, col0);
+// Its input gradient: the next level's output gradient (dx16), or FP32 rows of ld
+// values from column col0 (dx32).
+void dec_dx_launch(cliffs_mlp* m, int B, const Level& v, const Layer& y, const bf16* dz, bf16* dx16, float* dx32,
+                   int ld, int col0) {
+  const size_t sh = (size_t)9 * v.cin * v.cout * 4;
+  const bf16* x = m->X[v.lvl];
+  auto blocks = [&](int cells, int channels) {  // a thread takes so many of each
+    const long long n = (long long)B * v.S * ((v.S + cells - 1) / cells) * (v.cin / channels);
+    return (unsigned)((n + kDxThreads - 1) / kDxThreads);
+  };
+  if (v.cout == 1) {
+    k_dec_dx1<<<blocks(2, 8), kDxThreads, sh, m->stream>>>(B, v.S, v.cin, dz, y.W, y.kp, x, dx16);
+    return;
+  }
+  auto go = [&](auto kernel, int channels) {
+    smem_limit(kernel, sh);
+    kernel<<<blocks(kDxCells, channels), kDxThreads, sh, m->stream>>>(B, v.S, v.cin, v.cout, dz, y.W, y.kp, x, dx16,
+                                                                      dx32, ld, col0);
+  };
+  if (v.cin % 16 == 0)
+    go(k_dec_dx<16>, 16);
+  else
+    go(k_dec_dx<8>, 8);
 }
 
 // The map decoder's forward pass for rows [0, B): latent columns of out -> map.
@@ -514,7 +533,7 @@ void decoder_forward(cliffs_mlp* m, int B) {
       continue;
     }
     const int P = B * 4 * v.S * v.S;
-    k_im2col_up<<<(P + 7) / 8, dim3(32, 8), 0, m->stream>>>(B, v.S, v.cin, m->X[l], v.kp, m->col);
+    k_im2col_up<<<blocks256((long long)P * (v.kp / 8)), 256, 0, m->stream>>>(B, v.S, v.cin, m->X[l], v.kp, m->col);
     ++m->launches;
     Epi e{};
     e.bias = y.b;
@@ -534,38 +553,26 @@ void decoder_forward(cliffs_mlp* m, int B) {
 // the gradients of the decoder's weights and biases, and the latent's into
 // dyf columns [n_out, n_total).
 void decoder_backward(cliffs_mlp* m, int B) {
+  k_to_bf16<<<blocks256(((long long)B * m->side2 + 3) / 4), 256, 0, m->stream>>>(B * m->side2, m->dzf, m->dzb[0]);
+  ++m->launches;
   for (int l = 2; l >= 0; --l) {
     const Level v = level(m, l);
     Layer& y = m->L[m->nd + l];
-    const int P = B * 4 * v.S * v.S;
-    // the output gradient in BF16 rows of cout values (ReLU masks applied by
-    // the level above's input gradient)
-    k_to_bf16<<<blocks256((long long)P * v.cout), 256, 0, m->stream>>>(P * v.cout, m->dzf, m->dzb);
-    // weight and bias gradients: partial sums over chunks of pixels, then
+    const bf16* dz = m->dzb[l & 1];  // BF16 rows of cout values, the ReLU mask applied
+    // weight and bias gradients: partial sums over chunks of cells, then
     // over the chunks in order
-    switch (co_class(v.cout)) {
-      case 1: dec_dw_launch<1>(m, B, v); break;
-      case 8: dec_dw_launch<8>(m, B, v); break;
-      case 16: dec_dw_launch<16>(m, B, v); break;
-      case 32: dec_dw_launch<32>(m, B, v); break;
-      default: dec_dw_launch<64>(m, B, v); break;
-    }
-    const int nb = dw_blocks(P);
+    dec_dw_launch(m, B, v, dz);
+    const int nb = dw_blocks((long long)B * v.S * v.S);
     k_reduce_wgrad<<<(v.cout * v.K + 31) / 32, 32 * kStrands, 0, m->stream>>>(v.cout, v.K, v.K, nb, m->wpart, y.gw);
     k_reduce_wgrad<<<(v.cout + 31) / 32, 32 * kStrands, 0, m->stream>>>(1, v.cout, v.cout, nb, m->cpart, y.gb);
-    // input gradient, masked by the level input's ReLU; level 0's goes to
-    // the latent columns of the dense output gradient
-    float* dx = l > 0 ? m->dxf : m->dyf;
-    const int ld = l > 0 ? v.S * v.S * v.cin : m->n_total, col0 = l > 0 ? 0 : m->d.n_out;
-    switch (co_class(v.cout)) {
-      case 1: dec_dx_launch<1>(m, B, v, y, dx, ld, col0); break;
-      case 8: dec_dx_launch<8>(m, B, v, y, dx, ld, col0); break;
-      case 16: dec_dx_launch<16>(m, B, v, y, dx, ld, col0); break;
-      case 32: dec_dx_launch<32>(m, B, v, y, dx, ld, col0); break;
-      default: dec_dx_launch<64>(m, B, v, y, dx, ld, col0); break;
-    }
-    m->launches += 5;
-    if (l > 0) std::swap(m->dzf, m->dxf);  // the input gradient is the next level's output gradient
+    // input gradient, masked by the level input's ReLU: the output gradient of
+    // the level above it; level 0's goes to the latent columns of the dense
+    // output gradient
+    if (l > 0)
+      dec_dx_launch(m, B, v, y, dz, m->dzb[(l - 1) & 1], nullptr, 0, 0);
+    else
+      dec_dx_launch(m, B, v, y, dz, nullptr, m->dyf, m->n_total, m->d.n_out);
+    m->launches += 4;
   }
 }
 
