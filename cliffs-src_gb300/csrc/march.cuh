@@ -400,8 +400,8 @@ CL_HD OutCell<R> general_cell(const RawCell<R> w[7], int o, const LineCtx<R>& L,
   auto update = [&](int t, const Geo<R>& g, R& cn) -> OutCell<R> {
     const CellState<R>& j = fm[t];
     const CellState<R> mir{-j.u, j.c, j.e, j.d, j.v, j.H};
-    const CellState<R>& a = ew[t - 1] ? fm[t - 1] : mir;
-    const CellState<R>& b = ew[t + 1] ? fm[t + 1] : mir;
+    const CellState<R> a = ew[t - 1] ? fm[t - 1] : mir;
+    const CellState<R> b = ew[t + 1] ? fm[t + 1] : mir;
     R FPl, FQl, FPr, FQr;
     face_flux(a.u, a.c, a.e, j.u, j.c, j.e, p, FPl, FQl);
     face_flux(j.u, j.c, j.e, b.u, b.c, b.e, p, FPr, FQr);

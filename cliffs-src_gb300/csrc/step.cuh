@@ -432,57 +432,112 @@ __device__ __noinline__ OutCell<float> step_x_window(const SweepArgs& X, const f
   return general_cell(w, i, C, g, X.ph);
 }
 
-// The x-swept cell of row o + q - 3 beside cell (t, c) (row o = rb + t) that
-// lies outside the window: swept again from the step's input.
+// The x-swept cell (row k, column L) outside the window: swept again from the
+// step's input.
 __device__ __noinline__ RawCell<float> step_y_outside(const SweepArgs& X, int k, int L) {
   const OutCell<float> x = step_x_value(X, k, L);
   return RawCell<float>{__ldg(X.dep + cidx<0>(k, L, X.pitch)), x.s, x.v, x.u, true};
 }
 
-// The y-swept value of tile cell (t, c) (row rb + t, column c0 + c + 1,
-// 1-based) from the x-swept window sm.  scan: the cell keeps a remainder of
-// water or velocity with no wet cell in reach, and whether its column holds
-// one elsewhere decides (cliffs.f:113); nothing is returned then.
+// The x-swept cell (t, c) of the window sm, as the y-sweep reads it.
 template <class T>
-__device__ __noinline__ OutCell<float> step_y_value(const SweepArgs& X, const SweepArgs& Y, const float* sm, int rb,
-                                                    int c0, int t, int c, bool& scan) {
+__device__ __forceinline__ RawCell<float> step_y_raw(const float* sm, int t, int c) {
+  const float* f = sm + t * T::Win + 4 + c;
+  return RawCell<float>{f[0], f[T::Field + T::Out], f[3 * T::Field + T::Out], f[2 * T::Field + T::Out], true};
+}
+
+struct YValue {
+  OutCell<float> out;
+  int state;  // 0: out holds; 1: step_y_full has to decide; 2: the column's wet scan has to
+};
+
+// The y-swept value of tile cell (t, c) (row rb + t, column c0 + c + 1, 1-based)
+// from the x-swept window sm, unless a flooded cell, a remainder on land or a
+// cell outside the window has a say in it (state 1).
+template <class T>
+__device__ __noinline__ YValue step_y_shore(const SweepArgs& Y, const float* sm, int rb, int c0, int t, int c) {
   const int o = rb + t, L = c0 + c + 1, n = Y.n;
   const float ground = Y.ph.ground;
-  scan = false;
+  RawCell<float> w[5];
+  bool have[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const int k = o - 2 + q, tt = t - 2 + q;
+    w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
+    have[q] = k < 1 || k > n || (tt >= 0 && tt < T::Rows);
+    if (k >= 1 && k <= n && have[q]) w[q] = step_y_raw<T>(sm, tt, c);
+  }
+  YValue r;
+  r.out = OutCell<float>{0.f, 0.f, 0.f};
+  // a cell two rows away and outside the window matters to a wet cell beside a
+  // land neighbour, and to a remainder on land
+  const bool rest = w[2].u == 0.f && w[2].v == 0.f && depth_of(w[2].s, w[2].d) == 0.f;
+  r.state = 1;
+  if (!have[0] && !rest && !(depth_of(w[1].s, w[1].d) > ground)) return r;
+  if (!have[4] && !rest && !(depth_of(w[3].s, w[3].d) > ground)) return r;
+  const LineCtx<float> C = y_line(Y, L, o);
+  r.state = shore_cell(w, o, n, C, geo_at(Y, o, 1.f, 1.f), Y.ph, r.out) ? 0 : 1;
+  return r;
+}
+
+// The same by all the rules, from cells o-3 .. o+3, by two lanes: at most two of
+// the cells lie outside the window, on one side of it, and each lane sweeps one of
+// them again (one lane sweeping both, the few blocks with a flooded cell in their
+// first or last rows ended 4 to 9 us after the others and held up the step).  Both
+// lanes have the value.  The whole warp calls it; on: the pair has a cell.
+template <class T>
+__device__ __noinline__ YValue step_y_full(const SweepArgs& X, const SweepArgs& Y, const float* sm, int rb, int c0,
+                                           bool on, int t, int c) {
+  static_assert(T::Halo >= 1 && (T::Halo >= 3 || T::R >= 4), "at most two cells outside");
+  const int o = rb + t, L = c0 + c + 1, n = Y.n, odd = (int)(threadIdx.x & 1);
+  const float ground = Y.ph.ground;
+  // above the window: rows t - 3, t - 2; below: t + 2, t + 3
+  const bool above = t < 3;
+  RawCell<float> mine{0.f, 0.f, 0.f, 0.f, false};
+  if (T::Halo < 3) {
+    const int tt = above ? t - 3 + odd : t + 2 + odd, k = rb + tt;
+    if (on && (tt < 0 || tt >= T::Rows) && k >= 1 && k <= n) mine = step_y_outside(X, k, L);
+    __syncwarp();
+  }
+  LineCtx<float> C = y_line(Y, L, o);
+  Geo<float> g[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) g[q] = geo_at(Y, o - 1 + q, 1.f, 1.f);
   RawCell<float> w[7];
-  bool have[7];
 #pragma unroll
   for (int q = 0; q < 7; ++q) {
     const int k = o - 3 + q, tt = t - 3 + q;
     w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
-    have[q] = k < 1 || k > n || (tt >= 0 && tt < T::Rows);
-    if (k >= 1 && k <= n && have[q]) {
-      const float* f = sm + tt * T::Win + 4 + c;
-      w[q] = RawCell<float>{f[0], f[T::Field + T::Out], f[3 * T::Field + T::Out], f[2 * T::Field + T::Out], true};
-    }
+    if (k >= 1 && k <= n && tt >= 0 && tt < T::Rows) w[q] = step_y_raw<T>(sm, tt, c);
   }
-  // a cell two rows away and outside the window matters to a wet cell beside a
-  // land neighbour, and to a remainder on land
-  const bool rest = w[3].u == 0.f && w[3].v == 0.f && depth_of(w[3].s, w[3].d) == 0.f;
-  if (!have[1] && !rest && !(depth_of(w[2].s, w[2].d) > ground)) w[1] = step_y_outside(X, o - 2, L);
-  if (!have[5] && !rest && !(depth_of(w[4].s, w[4].d) > ground)) w[5] = step_y_outside(X, o + 2, L);
-  LineCtx<float> C = y_line(Y, L, o);
-  OutCell<float> out;
-  if (shore_cell(w + 1, o, n, C, geo_at(Y, o, 1.f, 1.f), Y.ph, out)) return out;
-  // the full rules: all cells o-3 .. o+3
-#pragma unroll
-  for (int q = 0; q < 7; ++q)
-    if (!have[q] && !w[q].present) w[q] = step_y_outside(X, o - 3 + q, L);
+  if (T::Halo < 3) {
+    RawCell<float> its;
+    its.d = __shfl_xor_sync(0xffffffffu, mine.d, 1);
+    its.s = __shfl_xor_sync(0xffffffffu, mine.s, 1);
+    its.u = __shfl_xor_sync(0xffffffffu, mine.u, 1);
+    its.v = __shfl_xor_sync(0xffffffffu, mine.v, 1);
+    its.present = __shfl_xor_sync(0xffffffffu, (int)mine.present, 1);
+    const RawCell<float> first = odd ? its : mine, second = odd ? mine : its;
+    if (above && first.present) w[0] = first;
+    if (above && second.present) w[1] = second;
+    if (!above && first.present) w[5] = first;
+    if (!above && second.present) w[6] = second;
+  }
   bool anywet = false;
 #pragma unroll
   for (int q = 0; q < 7; ++q) anywet |= w[q].present && depth_of(w[q].s, w[q].d) > ground;
-  scan = !anywet && !rest;
-  if (scan) return OutCell<float>{w[3].s, w[3].u, w[3].v};
+  YValue r;
+  r.out = OutCell<float>{w[3].s, w[3].u, w[3].v};
+  r.state = 0;
+  if (!on) return r;
+  const bool rest = w[3].u == 0.f && w[3].v == 0.f && depth_of(w[3].s, w[3].d) == 0.f;
+  if (!anywet && !rest) {  // whether its column holds a wet cell elsewhere decides (cliffs.f:113)
+    r.state = 2;
+    return r;
+  }
   C.wet = anywet;
-  Geo<float> g[3];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) g[q] = geo_at(Y, o - 1 + q, 1.f, 1.f);
-  return general_cell(w, o, C, g, Y.ph);
+  r.out = general_cell(w, o, C, g, Y.ph);
+  return r;
 }
 
 __device__ __forceinline__ void courant_status(const SweepArgs& A, float cour) {
@@ -868,7 +923,7 @@ struct StepShared {
   __align__(128) float win[T::Floats];
   uint16_t list[T::Rows * T::W];             // listed cells: window row * W + tile column
   unsigned n[2];                             // their number, x phase and y phase
-  unsigned scans;
+  unsigned full, scans;                      // cells left for step_y_full, and of these for the column scan
   PairConst k[2];                            // x and y axis
   __align__(8) uint64_t bar;
 };
@@ -974,22 +1029,44 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
   __syncthreads();
   const unsigned cy = S.n[1];
   if (cy) {
-    for (unsigned i = tid; i < cy; i += T::Threads) {
-      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
-      bool scan;
-      const OutCell<float> r = step_y_value<T>(X, Y, S.win, rb, c0, t, c, scan);
-      if (scan) {
-        S.list[i] |= 0x8000u;
-        S.scans = 1u;
-        continue;
-      }
+    const auto store = [&](int t, int c, const OutCell<float>& r) {
       const size_t q = (size_t)(rb + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
       Y.srf_o[q] = r.s;
       Y.xu_o[q] = r.v;
       Y.yv_o[q] = r.u;
       bad = bad || !isfinite(r.s + r.u + r.v);
+    };
+    for (unsigned i = tid; i < cy; i += T::Threads) {
+      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
+      const YValue r = step_y_shore<T>(Y, S.win, rb, c0, t, c);
+      if (r.state) {
+        S.list[i] |= 0x4000u;
+        S.full = 1u;
+      } else {
+        store(t, c, r.out);
+      }
     }
     __syncthreads();
+    if (S.full) {  // a pair of lanes each
+      const int lane = tid & 31;
+      for (unsigned base = (unsigned)(tid >> 5) * 16u; base < cy; base += T::Threads / 2) {
+        const unsigned i = base + (unsigned)(lane >> 1);
+        const unsigned ent = i < cy ? S.list[i] : 0u;
+        const bool on = (ent & 0x4000u) != 0u;
+        if (!__any_sync(0xffffffffu, on)) continue;
+        const int t = on ? (int)(ent & 0x3fffu) / T::W : T::Halo, c = (int)(ent & 0x3fffu) % T::W;
+        const YValue r = step_y_full<T>(X, Y, S.win, rb, c0, on, t, c);
+        if (on && !(lane & 1)) {
+          if (r.state == 2) {
+            S.list[i] = (uint16_t)((ent & 0x3fffu) | 0x8000u);
+            S.scans = 1u;
+          } else {
+            store(t, c, r.out);
+          }
+        }
+      }
+      __syncthreads();
+    }
     if (S.scans) {
       // remainders on land: zeroed when the x-swept column holds a wet cell
       // anywhere, else left as they are; the block looks through the column
@@ -1088,7 +1165,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     mbar_init(&S.bar, 1);
-    S.n[0] = S.n[1] = S.scans = 0u;
+    S.n[0] = S.n[1] = S.full = S.scans = 0u;
     S.k[0] = K.x;
     S.k[1] = K.y;
     fence_mbar_init();
@@ -1141,7 +1218,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const
   copy(S.k, &A->K, sizeof(PairPair));
   if (tid == 0) {
     mbar_init(&S.bar, 1);
-    S.n[0] = S.n[1] = S.scans = 0u;
+    S.n[0] = S.n[1] = S.full = S.scans = 0u;
     fence_mbar_init();
   }
   __syncthreads();
