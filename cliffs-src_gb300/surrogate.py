@@ -117,7 +117,7 @@ class MLP:
 
     def get(self, layer, which):
         r, c = self.shape(layer)
-        a = np.zeros((r, c) if which in (0, 2) else (r,), np.float32)
+        a = np.empty((r, c) if which in (0, 2) else (r,), np.float32)  # all of it written
         cg._chk(self.L.cliffs_mlp_get(self.h, layer, which, a.ctypes.data_as(_fp), a.size), "mlp_get")
         return a
 
@@ -131,7 +131,7 @@ class MLP:
 
     def predict(self, x):
         x = _f32(x)
-        y = np.zeros((x.shape[0], self.n_y), np.float32)
+        y = np.empty((x.shape[0], self.n_y), np.float32)  # all of it written: 16 MB of maps take 0.28 ms to clear
         cg._chk(self.L.cliffs_mlp_predict(self.h, x.shape[0], x.ctypes.data_as(_fp), y.ctypes.data_as(_fp)),
                 "mlp_predict")
         return y
