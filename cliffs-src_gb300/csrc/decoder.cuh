@@ -198,7 +198,8 @@ __device__ __forceinline__ bool stage_weights(float* sw, int C, int co, const __
 // 9 C CO floats.  Bound by the FP32 issue (36 C CO products a cell, two to an
 // instruction for CO = 8).  A thread per pixel read the weights four times as
 // often: at a batch of 512, 212 us for the map's level and 170 us for the
-// 8-channel one, against 69 and 107 here
+// 8-channel one, against 51 and 107 here (the map's
+// level with 8 channels unpacks each of the nine cells once; unpacked at every tap 69)
 template <int CO, bool GUARD>
 __device__ __forceinline__ void conv_cell(int S, int C, int b, int y0, int x0, const __nv_bfloat16* __restrict__ x,
                                           const float* sw, const float* __restrict__ bias, __nv_bfloat16* out16,
@@ -212,6 +213,30 @@ __device__ __forceinline__ void conv_cell(int S, int C, int b, int y0, int x0, c
     acc[i] = 0.f;
 #pragma unroll
     for (int o = 0; o < NP; ++o) acc2[i][o] = 0;
+  }
+  if (CO == 1 && !GUARD && C == 8) {  // all taps of the nine cells, each unpacked once
+    float xv[9][8];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int yy = y0 + k / 3 - 1, xx = x0 + k % 3 - 1;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (yy >= 0 && yy < S && xx >= 0 && xx < S)
+        v = __ldg(reinterpret_cast<const uint4*>(x) + ((size_t)b * S + yy) * S + xx);
+      unpack8(v, xv[k]);
+    }
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+      const float4 w0 = *reinterpret_cast<const float4*>(sw + 8 * tap);
+      const float4 w1 = *reinterpret_cast<const float4*>(sw + 8 * tap + 4);
+      const float f[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = ((i >> 1) + tap / 3 + 1) / 2 * 3 + ((i & 1) + tap % 3 + 1) / 2;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) acc[i] = fmaf(xv[k][g], f[g], acc[i]);
+      }
+    }
+    C = 0;  // done
   }
 #pragma unroll
   for (int tap = 0; tap < 9; ++tap) {
