@@ -2,8 +2,8 @@
 //
 // An ensemble of independent runs (one source scenario per grid, grids of
 // uneven size) has the same work per step as one run of the ensemble's total
-// size, but each grid alone fills only part of the GPU and pays two launches
-// per step.  Here every scenario's sweep is cut into the same tiles the
+// size, but each grid alone fills only part of the GPU and pays its own
+// launches.  Here every scenario's sweep is cut into the same tiles the
 // single-grid kernels use (sweep_tile: 128 threads, 512 cells of a row in the
 // x-sweep, 32 columns x 16 rows in the y-sweep), the tiles of all scenarios
 // form one flat list per sweep direction, and a block maps a list index to its

@@ -531,10 +531,11 @@ int step_tiles(int size, int nx, int ny) {
 // long as all large tiles are on the chip at once, a step lasts as long as its
 // slowest block: smaller tiles, which the phases cross in half the time, and
 // which as long as they all fit too have every row that the full rules read in
-// the window.  Measured, us per step (large, small, tiny): 256 x 256 14.0,
-// 10.8, 10.7; 400 x 400 13.5, 11.2, 11.1; 600 x 600 (1140 tiny tiles) 15.2,
-// 16.9, 13.7; 800 x 600 (1500) 17.1, 14.4, 16.4; 1201 x 903 (589 large ones)
-// 26.3, 23.9, 26.8; 1500 x 1500 (1200) 31.9, 33.8, 39.1.
+// the window.  Measured, us per step (small, tiny): 160 x 120 10.1, 9.6; 256 x
+// 256 10.1, 9.5; 400 x 400 10.6, 10.9; 500 x 560 12.1, 11.4; 600 x 600 (1140
+// tiny tiles) 14.7, 12.0.  With the first version of the kernel (large, small,
+// tiny): 600 x 600 15.2, 16.9, 13.7; 800 x 600 (1500) 17.1, 14.4, 16.4; 1201 x
+// 903 (589 large ones) 26.3, 23.9, 26.8; 1500 x 1500 (1200) 31.9, 33.8, 39.1.
 int step_size(int64_t large, int64_t tiny, int sms) {
   return large > (int64_t)sms * StepLarge::Blocks ? STEP_LARGE
          : tiny > (int64_t)sms * StepTiny::Blocks ? STEP_SMALL

@@ -22,7 +22,7 @@
 // cells of each neighbour again, so that only the state crosses blocks.
 //
 // Results are the bits of the sweep kernels' (the same functions on the same
-// values).  2000 cells: 0.63 us a step, from 6.0 with a launch per sweep,
+// values).  2000 cells: 1.0 us a step, from 6.0 with a launch per sweep,
 // replayed from graphs; bound by the latency of the three barriers and of the
 // chain between them.
 #pragma once

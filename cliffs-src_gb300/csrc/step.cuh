@@ -3,39 +3,47 @@
 //
 // A sweep per launch moves the state through memory twice a step: 72 bytes a
 // cell, and each cell's window is loaded, classified and converted once per
-// sweep.  Here a block takes a tile of 64 columns x 30 rows (StepLarge) with one
-// halo row on each side (the y-sweep's), brings it into shared memory with
-// tensor-map copies, sweeps its rows in place, then its columns out of the
-// swept tile straight to the other copy of the state: 44 bytes a cell, the
-// max-wave fold included.
+// sweep.  Here a block takes a tile of 64 columns x 30 rows (StepLarge; smaller
+// ones on smaller grids) with one halo row on each side (the y-sweep's), brings
+// it into shared memory with tensor-map copies, sweeps its rows in place, then
+// its columns out of the swept tile straight to the other copy of the state: 44
+// bytes a cell, the max-wave fold included.
 //
-// Both sweeps march: a thread owns two lines of a sweep (two rows 16 apart in the x phase, two adjacent columns in the y phase) over 8 cells and
-// carries the last cell and the last face's flux along, so that every celerity
-// is computed 10/8 and every face flux 9/8 times a cell (6/4 and 5/4 in
-// fast_kernel).  The two lines are the two halves of packed FP32 operations
+// Both sweeps march: a thread owns two lines of a sweep (two rows half a window
+// apart in the x phase, two adjacent columns in the y phase) over 8 cells (4 in
+// the smaller tiles) and carries the last cell and the last face's flux along,
+// so that every celerity is computed 10/8 and every face flux 9/8 times a cell
+// (6/4 and 5/4 in fast_kernel).  The two lines are the two halves of packed FP32 operations
 // (add/sub/mul/fma.rn.f32x2): the same roundings as march.cuh's scalar ones,
 // at half the issue slots.
 //
 // Classification.  As in sweep.cuh, a cell takes the plain update when it is
 // interior and it and its neighbours are wet and subcritical; every other cell
 // is left out of the thread's stores and, unless it is dry land at rest, put
-// on the block's list, which the whole block finishes through the full rules
-// after the phase (shore_cell for the most part: no cell is flooded; else
-// general_cell).  The x phase's listed cells are evaluated on the step's input
-// in global memory; the y phase's on the x-swept tile.
+// on the block's list, which the whole block finishes after the phase: by
+// shore_cell where no cell is flooded, else by all the rules (general_cell).
+// The x phase's listed cells are evaluated on the step's input, in the window
+// or, where the rows are swept in place, in global memory; the y phase's on the
+// x-swept tile.  Tiles with a coast in them take longest and go first.
 //
 // Measured (us per step, replayed from graphs, against a launch per sweep;
-// the same state bits): 2048 x 2048 shelf 46.5 from 68.6; 4320 x 2160 sphere
-// 89.8 from 144.2; 600 x 600 15.4 from 18.4; 256 x 256 14.5 from 15.7.  On the
-// shelf 204 thread instructions a cell (400 in the two sweeps), 39 bytes a cell
-// to and from DRAM, 16 warps an SM at 128 registers and 0.54 instructions an
-// SM sub-core and cycle while it is busy: what bounds it is the latency of the
-// march and of the window's copies, then the end of the grid, whose last
-// blocks leave SMs idle for an eighth of the step.  The same march on one line
-// a thread in scalar operations (64 registers, 32 warps) issued 271
-// instructions a cell at 0.70 and took 50.6 us; 96 registers and 5 blocks an
-// SM 50.8 us (spills); tiles of 32 columns 48.9 us; the max-wave update on the
-// outputs, in the y phase, 49.5 us.
+// the same state bits): 4320 x 2160 sphere 89 from 144; 2048 x 2048 shelf 44.2
+// from 68.6; 1500 x 1500 28.4 from 41.0; 1201 x 903 stretched 21.1 from 29.3;
+// 1003 x 777 15.5 from 21.8; 600 x 600 12.1 from 18.4; 256 x 256 9.5 from 15.1.
+// On the shelf 204 thread instructions a cell (400 in the two sweeps), 39 bytes
+// a cell to and from DRAM, 16 warps an SM at 128 registers and 0.54
+// instructions an SM sub-core and cycle while it is busy: what bounds it is the
+// latency of the march and of the window's copies.  A small grid's step is the
+// time of its slowest block: on 256 x 256 (64 threads an SM) 0.95 us for the
+// window, 1.5 for the x phase, 1.8 for a coast's listed cells, 1.2 for the y
+// phase and 1.2 to 3.5 for its listed cells; the code of the listed cells is
+// cold in every launch, which is about a quarter of that.
+//
+// Tried on the shelf, from 46.5 us: the same march on one line a thread in
+// scalar operations (64 registers, 32 warps) issued 271 instructions a cell at
+// 0.70 and took 50.6; 96 registers and 5 blocks an SM 50.8 (spills); tiles of
+// 32 columns 48.9; the max-wave update on the outputs, in the y phase, 49.5;
+// later windows prefetched into L2 46.6.
 #pragma once
 #include "staged.cuh"
 
@@ -1189,7 +1197,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
 // all scenarios' tiles (coasts first, as above), the scenario's arguments
 // staged in shared memory and its tensor maps read from device memory.  24
 // scenarios of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with
-// its uploads and maxima: 7.0 ms, from 12.2 with a launch per sweep phase.
+// its uploads and maxima: 6.7 ms, from 12.2 with a launch per sweep phase.
 struct StepArgs {
   SweepArgs X, Y;
   PairPair K;

@@ -1,5 +1,6 @@
-// ytile.cuh -- the y-sweep of a two-dimensional step with its tile staged in
-// shared memory by the bulk-copy (TMA) engine, in and out.
+// ytile.cuh -- the y-sweep of a two-dimensional step that runs a launch per
+// sweep (whole steps run step_kernel, step.cuh), with its tile staged in shared
+// memory by the bulk-copy (TMA) engine, in and out.
 //
 // fast_kernel's y-sweep loads its window with 24 scalar loads a thread (6
 // rows of 4 fields, lanes along the row) and stores 12 scalars, each with its

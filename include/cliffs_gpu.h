@@ -271,7 +271,8 @@ void cliffs_gpu_host_free(void *p);
  * Returns CLIFFS_ERR_NAN or CLIFFS_ERR_TIMEOUT when the matching bit is set,
  * else CLIFFS_WARN_CFL when CLIFFS_ST_CFL is.
  * The Courant check has no counterpart in the reference, whose dt is fixed by
- * the user (allabout.f:55) and never checked.  Every sweep evaluates
+ * the user (allabout.f:55) and never checked.  Every sweep (of a launch of its
+ * own or of a whole step's) evaluates
  * (|u|+c) dt / ((dx(m-1)+dx(m))/2) along its lines on the state it reads
  * (row spacing scaled by cos(lat) on a spherical grid), reduced per warp by a
  * vote and, where a number exceeds 1, a warp max reduction; VTCS-2 is stable
@@ -283,9 +284,9 @@ int cliffs_gpu_courant(cliffs_ctx *ctx, double *courant);
 /* Block until queued work on the context's stream is done. */
 int cliffs_gpu_sync(cliffs_ctx *ctx);
 
-/* Kernel timing: when enabled, step() brackets every sweep (its two kernel
- * launches) with CUDA events; read returns the mean duration (ms) of x- and
- * y-sweeps and their counts since the last reset. */
+/* Kernel timing: when enabled, step() launches every sweep by itself (no whole
+ * steps in one kernel) and brackets it with CUDA events; read returns the mean
+ * duration (ms) of x- and y-sweeps and their counts since the last reset. */
 int cliffs_gpu_profile(cliffs_ctx *ctx, int32_t enable);
 int cliffs_gpu_profile_read(cliffs_ctx *ctx, double *x_ms, int64_t *x_count,
                             double *y_ms, int64_t *y_count);
@@ -393,10 +394,11 @@ int cliffs_gpu_sweep_noalloc_status(void *stream, uint32_t *flags, uint32_t *lis
  * No reference counterpart: the reference runs one grid per process.  A batch
  * steps many independent contexts (one source scenario each, grids of any
  * size) together: every scenario's sweeps are cut into the single-grid
- * kernels' tiles, the tiles of all scenarios form one list per sweep
- * direction, and either one cooperative launch covers many steps (blocks meet
- * at a grid barrier between the x and y phases) or one launch per phase and
- * step covers every scenario, replayed from a CUDA graph.  Results are
+ * kernels' tiles, the tiles of all scenarios form one list (of whole steps or
+ * per sweep direction), and either one cooperative launch covers many steps
+ * (blocks meet at a grid barrier between the x and y phases) or one launch per
+ * step (a phase, where a scenario does not take whole steps) covers every
+ * scenario, replayed from a CUDA graph.  Results are
  * bit-identical to stepping the contexts one by one with cliffs_gpu_step.
  * Contexts must be 2-D, hold a state, have no boundary forcing, and live on
  * the current device; a source still rising (cliffs_gpu_add_source) is
