@@ -52,27 +52,29 @@ __device__ __forceinline__ fpair pair_bf16(uint32_t w) { return pair_of(w << 16,
 // im2col of the 2x upsampled input: row p = (b, Y, X) of the output grid
 // (side 2S), column k = tap * Cin + c < 9 Cin, columns up to kp zero.  The
 // upsampled cell (Y', X') = (Y + ty - 1, X + tx - 1) reads input cell
-// (Y' / 2, X' / 2); outside [0, 2S) it is zero padding.  dst [P][kp].  A thread
-// per 8 columns (one tap, 8 channels: C and kp are multiples of 8), one 16-byte
-// load and store, so that every lane works whatever kp is: a warp per pixel left
-// 28 of 32 lanes idle in every second round of the surrogate's 36 groups and took
-// 171 us at a batch of 512 (302 MB written), this 105.  Pixel indices are 32-bit
-// (B (2S)^2 < 2^31).
-__global__ void __launch_bounds__(256) k_im2col_up(int B, int S, int C, const __nv_bfloat16* __restrict__ x, int kp,
+// (Y' / 2, X' / 2); outside [0, 2S) it is zero padding.  dst [P][kp].  A block
+// per (b, Y); a thread keeps its 8 columns (one tap, 8 channels: C and kp are
+// multiples of 8) and walks along X, one 16-byte load and store a pixel, so that
+// the divisions are done once.  Blocks of im2col_threads(kp).  302 MB written at a
+// batch of 512: a warp per pixel, 28 of 32 lanes idle in every second round of the
+// surrogate's 36 groups, took 171 us, a thread per 8 columns 95, this 56.
+__host__ __device__ constexpr int im2col_threads(int kp) { return 256 / (kp / 8) * (kp / 8); }
+__global__ void __launch_bounds__(256) k_im2col_up(int S, int C, const __nv_bfloat16* __restrict__ x, int kp,
                                                    __nv_bfloat16* dst) {
-  const unsigned S2 = 2 * S, img = S2 * S2, per = kp / 8;
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;  // fewer than 18 map cells B < 2^32
-  const int p = t / per, k = 8 * (t % per);
-  if (p >= (int)(B * img)) return;
-  const int b = p / img, r = p % img, Y = r / S2, X = r % S2;
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (k < 9 * C) {
-    const int tap = k / C, c = k % C;
-    const int Yu = Y + tap / 3 - 1, Xu = X + tap % 3 - 1;
-    if (Yu >= 0 && Yu < 2 * S && Xu >= 0 && Xu < 2 * S)
-      v = __ldg(reinterpret_cast<const uint4*>(x + (((size_t)b * S + (Yu >> 1)) * S + (Xu >> 1)) * C + c));
+  const int S2 = 2 * S, per = kp / 8, step = (int)blockDim.x / per;
+  const int b = blockIdx.x / S2, Y = blockIdx.x % S2;
+  const int g = (int)threadIdx.x % per, tap = 8 * g / C, c = 8 * g % C;
+  const int Yu = Y + tap / 3 - 1, dx = tap % 3 - 1;
+  const bool row = tap < 9 && Yu >= 0 && Yu < S2;
+  const __nv_bfloat16* src = x + (((size_t)b * S + (row ? Yu >> 1 : 0)) * S) * C + c;
+  uint4* out = reinterpret_cast<uint4*>(dst) + (size_t)blockIdx.x * S2 * per + g;
+#pragma unroll 4
+  for (int X = (int)threadIdx.x / per; X < S2; X += step) {
+    const int Xu = X + dx;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (row && Xu >= 0 && Xu < S2) v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(Xu >> 1) * C));
+    out[(size_t)X * per] = v;
   }
-  reinterpret_cast<uint4*>(dst)[t] = v;
 }
 
 // The decoder's input: ReLU of the latent columns [col0, col0 + n) of the

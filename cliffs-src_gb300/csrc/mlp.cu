@@ -533,7 +533,7 @@ void decoder_forward(cliffs_mlp* m, int B) {
       continue;
     }
     const int P = B * 4 * v.S * v.S;
-    k_im2col_up<<<blocks256((long long)P * (v.kp / 8)), 256, 0, m->stream>>>(B, v.S, v.cin, m->X[l], v.kp, m->col);
+    k_im2col_up<<<B * 2 * v.S, im2col_threads(v.kp), 0, m->stream>>>(v.S, v.cin, m->X[l], v.kp, m->col);
     ++m->launches;
     Epi e{};
     e.bias = y.b;
