@@ -431,17 +431,24 @@ bool gemm_tc_launch(cliffs_mlp* m, int M, int N, int K, const bf16* A, int lda, 
 // C = A B^T.  Products of at least 128 rows, 16 columns and a reduction of
 // 64 whose operands suit the tensor-memory path (16-byte aligned rows,
 // 128-byte aligned bases) run as gemm_tc, with the widest tile of 16, 64 or
-// 128 columns that N fills; the others (small batches, the first layer's 9
-// inputs) run as gemm_tn.
+// 128 columns that N fills and that gives each SM a block (kGemmFill), else 16;
+// the others (small batches, the first layer's 9 inputs) run as gemm_tn.  A
+// block's time is the chain of its slices, whatever the tile's width: 512 x 512
+// with a reduction of 512 took 12.3 us in 16 blocks of 128 columns, 9.7 in 32
+// of 64 and 7.8 in 128 of 16; 4096 x 512 12.4 us in 128 blocks of 128, 10.8 in
+// 256 of 64.
+constexpr int kGemmFill = 152;
 void gemm(cliffs_mlp* m, int M, int N, int K, const bf16* A, int lda, const bf16* B, int ldb, const Epi& e) {
   // every tensor-map box lies within its operand's extent: M >= 128 rows,
   // K >= 64, and a tile width of at most N (16, 64 or 128)
   const bool tc_ok = M >= umma::BM && N >= 16 && K >= umma::BK && lda % 8 == 0 && ldb % 8 == 0 &&
                      ((uintptr_t)A % 128) == 0 && ((uintptr_t)B % 128) == 0;
   if (tc_ok) {
-    const bool launched = N >= 128  ? gemm_tc_launch<128>(m, M, N, K, A, lda, B, ldb, e)
-                          : N >= 64 ? gemm_tc_launch<64>(m, M, N, K, A, lda, B, ldb, e)
-                                    : gemm_tc_launch<16>(m, M, N, K, A, lda, B, ldb, e);
+    const auto blocks = [&](int bn) { return (long long)((M + umma::BM - 1) / umma::BM) * ((N + bn - 1) / bn); };
+    const bool launched =
+        N >= 128 && blocks(128) >= kGemmFill ? gemm_tc_launch<128>(m, M, N, K, A, lda, B, ldb, e)
+        : N >= 64 && blocks(64) >= kGemmFill ? gemm_tc_launch<64>(m, M, N, K, A, lda, B, ldb, e)
+                                             : gemm_tc_launch<16>(m, M, N, K, A, lda, B, ldb, e);
     if (!launched) m->tc_failed = true;  // reported by the call (CLIFFS_ERR_CUDA)
     return;
   }
