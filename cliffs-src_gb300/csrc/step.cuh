@@ -355,7 +355,8 @@ __device__ __noinline__ OutCell<float> step_x_value(const SweepArgs& X, int L, i
     w[t] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
     if (k >= 1 && k <= n) {
       const size_t q = cidx<0>(L, k, X.pitch);
-      w[t] = RawCell<float>{__ldg(X.dep + q), __ldg(X.srf + q), __ldg(X.xu + q), __ldg(X.yv + q), true};
+      w[t] = RawCell<float>{__ldg(X.dep + q), ld_state<false>(X.srf + q), ld_state<false>(X.xu + q),
+                            ld_state<false>(X.yv + q), true};
     }
   }
   if (!swept) return OutCell<float>{w[2].s, w[2].u, w[2].v};  // a row that is not swept
@@ -384,7 +385,7 @@ __device__ __forceinline__ bool step_x_wet(const SweepArgs& X, int L, int i) {
   for (int k = max(i - 1, 1); k <= min(i + 1, X.n); ++k) {
     const size_t q = cidx<0>(L, k, X.pitch);
     const float d = __ldg(X.dep + q);
-    any = any || depth_of(__ldg(X.srf + q), d) > X.ph.ground;
+    any = any || depth_of(ld_state<false>(X.srf + q), d) > X.ph.ground;
     if (k == i) dq = d;
   }
   return any && depth_of(step_x_value(X, L, i).s, dq) > X.ph.ground;
@@ -982,8 +983,8 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
     fold_item<T>(k, t, c);
     F.h[k] = F.v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (fold_cell<T>(X, rb, c0, t, c, q)) {
-      F.h[k] = __ldg(reinterpret_cast<const float4*>(X.hmax_in + q));
-      F.v[k] = __ldg(reinterpret_cast<const float4*>(X.velmax_in + q));
+      F.h[k] = ld_state4<false>(X.hmax_in + q);
+      F.v[k] = ld_state4<false>(X.velmax_in + q);
     }
   }
   const bool ok = mbar_wait_ns(&S.bar, 0u, C.wait_ns);

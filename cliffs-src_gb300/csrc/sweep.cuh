@@ -65,18 +65,22 @@ struct SweepArgs {
 
 enum : unsigned { ST_NAN = 1u, ST_CFL = 4u };
 
-// Loads of the state fields (surface, u, v, max-wave).  A sweep kernel reads
-// the fields another launch wrote, through the read-only path (COH = false).
-// The batched persistent kernel (batch.cuh) reads fields that other blocks of
-// the same launch wrote before a grid barrier: those loads go to L2
-// (COH = true), where the writes are, not to a possibly stale L1 line.
+// Loads of the state fields (surface, u, v, max-wave): plain ones (COH =
+// false), never through the read-only path (__ldg), which is for data that
+// stays as it is for the kernel's whole life: a launch may start while the
+// steps before it still write these fields (griddepcontrol.wait orders plain
+// loads after those writes), and a kernel stores to some of them itself.  The
+// batched persistent kernel (batch.cuh) reads fields that other blocks of the
+// same launch wrote before a grid barrier: those loads go to L2 (COH = true),
+// where the writes are, not to a possibly stale L1 line.  Depth, geometry and
+// tile lists do not change while a context steps: they are read with __ldg.
 template <bool COH>
 __device__ __forceinline__ float ld_state(const float* p) {
-  return COH ? __ldcg(p) : __ldg(p);
+  return COH ? __ldcg(p) : *p;
 }
 template <bool COH>
 __device__ __forceinline__ float4 ld_state4(const float* p) {
-  return COH ? __ldcg(reinterpret_cast<const float4*>(p)) : __ldg(reinterpret_cast<const float4*>(p));
+  return COH ? __ldcg(reinterpret_cast<const float4*>(p)) : *reinterpret_cast<const float4*>(p);
 }
 
 template <int DIR>
