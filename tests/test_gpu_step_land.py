@@ -1,0 +1,58 @@
+"""Whole steps in one kernel on land that keeps a remainder: velocities left on
+cells whose row and column hold no water stay as they are (cliffs.f:113), step
+after step, and every such cell has its column looked through.  The same bits as
+a launch per sweep (CLIFFS_SWEEP_DIRECT), and no slower than one."""
+import importlib
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+pkg = importlib.import_module("cliffs-src_gb300")
+cg = pkg.cliffs_gpu
+
+
+def _grids(nx, ny, columns):
+    """Water in the low quarter, land elsewhere, a velocity on the high quarter's columns."""
+    d = np.full((ny, nx), -5.0)
+    d[: ny // 2, : nx // 2] = 20.0
+    h = np.maximum(d, 0.0)
+    u = np.zeros((ny, nx))
+    u[ny // 2 + 8:, nx // 2 + 8: nx // 2 + 8 + columns] = 0.1
+    u[ny // 2 + 8::3, nx // 4] = 0.2  # and one column whose remainders the next y-sweep clears
+    out = []
+    for kind in (cg.TILED, cg.DIRECT):
+        g = pkg.GpuGrid(d, dx=np.full(nx - 1, 100.0), dy=np.full(ny - 1, 100.0), ground=0.05, crough=0.0, dt=1.0)
+        g.set_initial(h, u, np.zeros_like(u))
+        g.set_sweep_kernel(kind)
+        out.append(g)
+    return out
+
+
+@pytest.mark.parametrize("nx,ny", [(61, 73), (512, 500), (1300, 320), (1700, 800)])
+def test_remainders_match_sweeps(nx, ny):
+    a, b = _grids(nx, ny, nx)
+    for steps in (3, 4, 2):
+        a.step(steps)
+        b.step(steps)
+    for x, y in zip((*a.download_state(), *a.maxwave()), (*b.download_state(), *b.maxwave())):
+        assert np.array_equal(x, y)
+    assert a.status() == b.status()
+    assert np.count_nonzero(a.download_state()[1][ny // 2 + 8:, nx // 2 + 8:]) > 0  # they were kept
+
+
+def test_remainders_cost_no_more_than_sweeps():
+    """At most half as much again as a launch per sweep (a scan for each cell: four times as much)."""
+    took = []
+    for g in _grids(512, 512, 512):
+        t = []
+        g.step(9)
+        for _ in range(5):
+            g.sync()
+            t0 = time.perf_counter()
+            g.step(8)
+            g.sync()
+            t.append(time.perf_counter() - t0)
+        took.append(sorted(t)[2])
+    assert took[0] <= 1.5 * took[1], took
