@@ -338,16 +338,40 @@ __device__ __forceinline__ bool shore_cell(const RawCell<float>* w, int o, int n
   return true;
 }
 
-// general_value<0> out of line: the rare remainder of step_x_value.
+// All the rules on the step's input in global memory.
 __device__ __noinline__ OutCell<float> step_x_general(const SweepArgs& X, int L, int i) {
   return general_value<0, false>(X, L, i);
 }
 
+// A cell's value, unless all the rules have to decide (ok false).
+struct XValue {
+  OutCell<float> out;
+  bool ok;
+};
+
+// The constants of row L that the rules at and beside cell i need.
+__device__ __forceinline__ LineCtx<float> x_line(const SweepArgs& X, int L, int i, float& alpha, float& ialpha) {
+  alpha = ialpha = 1.f;
+  if (X.lscale) {
+    const float2 a = __ldg(X.lscale + (L - 1));
+    alpha = a.x;
+    ialpha = a.y;
+  }
+  LineCtx<float> C;
+  C.n = X.n;
+  C.eL = i == 1 ? edge_vals(X, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.eR = i == X.n ? edge_vals(X, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
+  C.inv_dx1 = X.inv_dx1 * ialpha;
+  C.inv_dxn1 = X.inv_dxn1 * ialpha;
+  C.scl1 = C.scln = 0.f;
+  return C;
+}
+
 // The x-swept value of grid cell (row L, column i), 1-based, from the step's
-// input in global memory.
-__device__ __noinline__ OutCell<float> step_x_value(const SweepArgs& X, int L, int i) {
-  const bool swept = L >= X.lo && L <= X.hi;
+// input in global memory, where no flooding is in play.
+__device__ __noinline__ XValue step_x_shore(const SweepArgs& X, int L, int i) {
   const int n = X.n;
+  XValue r;
   RawCell<float> w[5];
 #pragma unroll
   for (int t = 0; t < 5; ++t) {
@@ -359,22 +383,19 @@ __device__ __noinline__ OutCell<float> step_x_value(const SweepArgs& X, int L, i
                             ld_state<false>(X.yv + q), true};
     }
   }
-  if (!swept) return OutCell<float>{w[2].s, w[2].u, w[2].v};  // a row that is not swept
-  float alpha = 1.f, ialpha = 1.f;
-  if (X.lscale) {
-    const float2 a = __ldg(X.lscale + (L - 1));
-    alpha = a.x;
-    ialpha = a.y;
-  }
-  LineCtx<float> C;
-  C.eL = i == 1 ? edge_vals(X, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
-  C.eR = i == n ? edge_vals(X, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
-  C.inv_dx1 = X.inv_dx1 * ialpha;
-  C.inv_dxn1 = X.inv_dxn1 * ialpha;
-  C.scl1 = C.scln = 0.f;
-  OutCell<float> out;
-  if (shore_cell(w, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, out)) return out;
-  return step_x_general(X, L, i);
+  r.out = OutCell<float>{w[2].s, w[2].u, w[2].v};
+  r.ok = true;
+  if (L < X.lo || L > X.hi) return r;  // a row that is not swept
+  float alpha, ialpha;
+  const LineCtx<float> C = x_line(X, L, i, alpha, ialpha);
+  r.ok = shore_cell(w, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, r.out);
+  return r;
+}
+
+// The same by whichever rules it takes.
+__device__ __forceinline__ OutCell<float> step_x_value(const SweepArgs& X, int L, int i) {
+  const XValue r = step_x_shore(X, L, i);
+  return r.ok ? r.out : step_x_general(X, L, i);
 }
 
 // Whether the x-swept cell (row L, column i) is wet.  A dry cell between dry
@@ -405,36 +426,44 @@ __device__ __forceinline__ LineCtx<float> y_line(const SweepArgs& Y, int L, int 
   return C;
 }
 
-// The tile cell (t, c) of the x phase from the step's input in the window.
+// Cell `at` of the window sm, column k of the grid, as the x-sweep reads it.
 template <class T>
-__device__ __noinline__ OutCell<float> step_x_window(const SweepArgs& X, const float* sm, int rb, int c0, int t, int c) {
+__device__ __forceinline__ RawCell<float> step_x_raw(const float* sm, int at, int k, int n) {
+  const float* f = sm + at;
+  return RawCell<float>{f[0], f[T::Field], f[2 * T::Field], f[3 * T::Field], k >= 1 && k <= n};
+}
+
+// The tile cell (t, c) of the x phase from the step's input in the window,
+// where no flooding is in play.
+template <class T>
+__device__ __noinline__ XValue step_x_window_shore(const SweepArgs& X, const float* sm, int rb, int c0, int t, int c) {
+  const int L = rb + t, i = c0 + c + 1, n = X.n;
+  RawCell<float> w[5];
+#pragma unroll
+  for (int q = 0; q < 5; ++q) w[q] = step_x_raw<T>(sm, t * T::Win + 2 + c + q, i - 2 + q, n);
+  float alpha, ialpha;
+  const LineCtx<float> C = x_line(X, L, i, alpha, ialpha);
+  XValue r;
+  r.ok = shore_cell(w, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, r.out);
+  return r;
+}
+
+// And by all the rules.
+template <class T>
+__device__ __noinline__ OutCell<float> step_x_window_full(const SweepArgs& X, const float* sm, int rb, int c0, int t,
+                                                          int c) {
   const int L = rb + t, i = c0 + c + 1, n = X.n;
   RawCell<float> w[7];
   bool anywet = false;
 #pragma unroll
   for (int q = 0; q < 7; ++q) {
-    const int k = i - 3 + q;
-    const float* f = sm + t * T::Win + 1 + c + q;
-    w[q] = RawCell<float>{f[0], f[T::Field], f[2 * T::Field], f[3 * T::Field], k >= 1 && k <= n};
+    w[q] = step_x_raw<T>(sm, t * T::Win + 1 + c + q, i - 3 + q, n);
     anywet |= w[q].present && depth_of(w[q].s, w[q].d) > X.ph.ground;
   }
-  float alpha = 1.f, ialpha = 1.f;
-  if (X.lscale) {
-    const float2 a = __ldg(X.lscale + (L - 1));
-    alpha = a.x;
-    ialpha = a.y;
-  }
-  LineCtx<float> C;
-  C.n = n;
-  C.wet = anywet;
-  C.eL = i == 1 ? edge_vals(X, L, 0) : EdgeVals<float>{0.f, 0.f, 0.f};
-  C.eR = i == n ? edge_vals(X, L, 1) : EdgeVals<float>{0.f, 0.f, 0.f};
-  C.inv_dx1 = X.inv_dx1 * ialpha;
-  C.inv_dxn1 = X.inv_dxn1 * ialpha;
-  C.scl1 = C.scln = 0.f;
-  OutCell<float> out;
-  if (shore_cell(w + 1, i, n, C, geo_at(X, i, alpha, ialpha), X.ph, out)) return out;
   if (!anywet) return step_x_general(X, L, i);  // does the row hold a wet cell elsewhere?
+  float alpha, ialpha;
+  LineCtx<float> C = x_line(X, L, i, alpha, ialpha);
+  C.wet = anywet;
   Geo<float> g[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q) g[q] = geo_at(X, i - 1 + q, alpha, ialpha);
@@ -457,14 +486,14 @@ __device__ __forceinline__ RawCell<float> step_y_raw(const float* sm, int t, int
 
 struct YValue {
   OutCell<float> out;
-  int state;  // 0: out holds; 1: step_y_full has to decide; 2: the column's wet scan has to
+  bool scan;  // the column's wet scan has to decide
 };
 
 // The y-swept value of tile cell (t, c) (row rb + t, column c0 + c + 1, 1-based)
 // from the x-swept window sm, unless a flooded cell, a remainder on land or a
-// cell outside the window has a say in it (state 1).
+// cell outside the window has a say in it.
 template <class T>
-__device__ __noinline__ YValue step_y_shore(const SweepArgs& Y, const float* sm, int rb, int c0, int t, int c) {
+__device__ __noinline__ XValue step_y_shore(const SweepArgs& Y, const float* sm, int rb, int c0, int t, int c) {
   const int o = rb + t, L = c0 + c + 1, n = Y.n;
   const float ground = Y.ph.ground;
   RawCell<float> w[5];
@@ -476,34 +505,35 @@ __device__ __noinline__ YValue step_y_shore(const SweepArgs& Y, const float* sm,
     have[q] = k < 1 || k > n || (tt >= 0 && tt < T::Rows);
     if (k >= 1 && k <= n && have[q]) w[q] = step_y_raw<T>(sm, tt, c);
   }
-  YValue r;
+  XValue r;
   r.out = OutCell<float>{0.f, 0.f, 0.f};
   // a cell two rows away and outside the window matters to a wet cell beside a
   // land neighbour, and to a remainder on land
   const bool rest = w[2].u == 0.f && w[2].v == 0.f && depth_of(w[2].s, w[2].d) == 0.f;
-  r.state = 1;
+  r.ok = false;
   if (!have[0] && !rest && !(depth_of(w[1].s, w[1].d) > ground)) return r;
   if (!have[4] && !rest && !(depth_of(w[3].s, w[3].d) > ground)) return r;
   const LineCtx<float> C = y_line(Y, L, o);
-  r.state = shore_cell(w, o, n, C, geo_at(Y, o, 1.f, 1.f), Y.ph, r.out) ? 0 : 1;
+  r.ok = shore_cell(w, o, n, C, geo_at(Y, o, 1.f, 1.f), Y.ph, r.out);
   return r;
 }
 
-// The same by all the rules, from cells o-3 .. o+3, by two lanes: at most two of
-// the cells lie outside the window, on one side of it, and each lane sweeps one of
-// them again (one lane sweeping both, the few blocks with a flooded cell in their
-// first or last rows ended 4 to 9 us after the others and held up the step).  Both
-// lanes have the value.  The whole warp calls it; on: the pair has a cell.
+// The same by all the rules, from cells o-3 .. o+3.  pair: by two lanes, for cells
+// in the tile's first and last rows: at most two of the cells lie outside the
+// window, on one side of it, and each lane sweeps one of them again (one lane
+// sweeping both, the few blocks with a flooded cell there ended 4 to 9 us after
+// the others and held up the step).  Both lanes have the value.  The whole warp
+// calls it, with the same `pair`; on: the lane (its pair) has a cell.
 template <class T>
 __device__ __noinline__ YValue step_y_full(const SweepArgs& X, const SweepArgs& Y, const float* sm, int rb, int c0,
-                                           bool on, int t, int c) {
+                                           bool pair, bool on, int t, int c) {
   static_assert(T::Halo >= 1 && (T::Halo >= 3 || T::R >= 4), "at most two cells outside");
   const int o = rb + t, L = c0 + c + 1, n = Y.n, odd = (int)(threadIdx.x & 1);
   const float ground = Y.ph.ground;
   // above the window: rows t - 3, t - 2; below: t + 2, t + 3
   const bool above = t < 3;
   RawCell<float> mine{0.f, 0.f, 0.f, 0.f, false};
-  if (T::Halo < 3) {
+  if (T::Halo < 3 && pair) {
     const int tt = above ? t - 3 + odd : t + 2 + odd, k = rb + tt;
     if (on && (tt < 0 || tt >= T::Rows) && k >= 1 && k <= n) mine = step_y_outside(X, k, L);
     __syncwarp();
@@ -519,7 +549,7 @@ __device__ __noinline__ YValue step_y_full(const SweepArgs& X, const SweepArgs& 
     w[q] = RawCell<float>{0.f, 0.f, 0.f, 0.f, false};
     if (k >= 1 && k <= n && tt >= 0 && tt < T::Rows) w[q] = step_y_raw<T>(sm, tt, c);
   }
-  if (T::Halo < 3) {
+  if (T::Halo < 3 && pair) {
     RawCell<float> its;
     its.d = __shfl_xor_sync(0xffffffffu, mine.d, 1);
     its.s = __shfl_xor_sync(0xffffffffu, mine.s, 1);
@@ -537,11 +567,11 @@ __device__ __noinline__ YValue step_y_full(const SweepArgs& X, const SweepArgs& 
   for (int q = 0; q < 7; ++q) anywet |= w[q].present && depth_of(w[q].s, w[q].d) > ground;
   YValue r;
   r.out = OutCell<float>{w[3].s, w[3].u, w[3].v};
-  r.state = 0;
+  r.scan = false;
   if (!on) return r;
   const bool rest = w[3].u == 0.f && w[3].v == 0.f && depth_of(w[3].s, w[3].d) == 0.f;
   if (!anywet && !rest) {  // whether its column holds a wet cell elsewhere decides (cliffs.f:113)
-    r.state = 2;
+    r.scan = true;
     return r;
   }
   C.wet = anywet;
@@ -560,6 +590,32 @@ __device__ __forceinline__ void courant_status(const SweepArgs& A, float cour) {
 }
 
 // ---- the x phase ------------------------------------------------------------------
+
+// Numbers that lanes of a warp leave behind, to be taken 16 or 32 at a time by
+// lanes next to each other.  The whole warp calls each of the functions.
+struct WarpQueue {
+  uint16_t* q;     // 64 places in shared memory
+  unsigned n = 0;  // how many are taken
+
+  __device__ __forceinline__ void push(bool want, unsigned v) {  // n <= 32
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (want) q[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = (uint16_t)v;
+    n += __popc(m);
+    __syncwarp();
+  }
+  __device__ __forceinline__ bool peek(unsigned k, unsigned& v) const {  // the k-th
+    v = k < n ? q[k] : 0u;
+    return k < n;
+  }
+  __device__ __forceinline__ void pop(unsigned k) {  // the first k, or all
+    const unsigned left = n > k ? n - k : 0u, lane = threadIdx.x & 31;
+    const uint16_t v = lane < left ? q[k + lane] : (uint16_t)0;
+    __syncwarp();
+    if (lane < left) q[lane] = v;
+    n = left;
+    __syncwarp();
+  }
+};
 
 // Appends the entries first + (bits of mask) to the block's list.
 __device__ __forceinline__ void list_push(unsigned mask, unsigned first, uint16_t* s_list, unsigned* s_n) {
@@ -931,9 +987,9 @@ struct StepShared {
   // dep, srf, xu, yv (and the swept srf, xu, yv): [row + Halo - r0][col + 4 - c0]
   __align__(128) float win[T::Floats];
   uint16_t list[T::Rows * T::W];             // listed cells: window row * W + tile column
-  unsigned n[2];                             // their number, x phase and y phase
-  unsigned full;                             // cells left for step_y_full
-  unsigned scans[2];                         // and of these the columns (a bit each) that need the wet scan
+  uint16_t queue[T::Threads / 32][2][64];    // places in the list that wait for all the rules (WarpQueue)
+  unsigned n[2];                             // listed cells, x phase and y phase
+  unsigned scans[2];                         // the columns (a bit each) of the y phase that need the wet scan
   PairConst k[2];                            // x and y axis
   __align__(8) uint64_t bar;
 };
@@ -1021,17 +1077,47 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
   bool bad = false;
   step_x_phase<T, GX>(X, &S.k[0], S.win, rb, c0, S.list, &S.n[0], bad);
   __syncthreads();
+  // The listed cells, a warp's share of them: those where no flooding is in play
+  // (most of a coast) at once, the others gathered so that the warp's lanes go
+  // through all the rules together.  A warp of both kinds pays for both: taken as
+  // they came, a sea floor of random depths, a third of it land, took 560 us a step
+  // at 2048 x 2048 and 51 at 600 x 600, 262 and 32 this way (a launch per sweep 259
+  // and 46).  Gathered by the block after a barrier, 256 x 256 with one beach took
+  // 9.9 us, 9.1 by warps (9.5 as they came).
+  const int lane = tid & 31;
+  const unsigned first = (unsigned)(tid & ~31);
   const unsigned cx = S.n[0];
   if (cx) {
-    for (unsigned i = tid; i < cx; i += T::Threads) {
-      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
-      const OutCell<float> r = T::InPlace ? step_x_value(X, rb + t, c0 + c + 1)
-                                          : step_x_window<T>(X, S.win, rb, c0, t, c);
+    const auto put = [&](int t, int c, const OutCell<float>& r) {
       float* f = S.win + T::Out + t * T::Win + 4 + c;
       f[T::Field] = r.s;
       f[2 * T::Field] = r.u;
       f[3 * T::Field] = r.v;
       bad = bad || !isfinite(r.s + r.u + r.v);
+    };
+    WarpQueue Q{S.queue[tid >> 5][0]};
+    for (unsigned base = first;; base += T::Threads) {
+      const unsigned i = base + lane;
+      bool hard = false;
+      if (i < cx) {
+        const int t = S.list[i] / T::W, c = S.list[i] % T::W;
+        const XValue r = T::InPlace ? step_x_shore(X, rb + t, c0 + c + 1)
+                                    : step_x_window_shore<T>(X, S.win, rb, c0, t, c);
+        hard = !r.ok;
+        if (r.ok) put(t, c, r.out);
+      }
+      Q.push(hard, i);
+      const bool more = base + T::Threads < cx;
+      if (Q.n >= 32 || (Q.n && !more)) {
+        unsigned at;
+        if (Q.peek(lane, at)) {
+          const int t = S.list[at] / T::W, c = S.list[at] % T::W;
+          put(t, c, T::InPlace ? step_x_general(X, rb + t, c0 + c + 1)
+                               : step_x_window_full<T>(X, S.win, rb, c0, t, c));
+        }
+        Q.pop(32);
+      }
+      if (!more && !Q.n) break;
     }
     __syncthreads();
   }
@@ -1046,37 +1132,52 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
       Y.yv_o[q] = r.u;
       bad = bad || !isfinite(r.s + r.u + r.v);
     };
-    for (unsigned i = tid; i < cy; i += T::Threads) {
-      const int t = S.list[i] / T::W, c = S.list[i] % T::W;
-      const YValue r = step_y_shore<T>(Y, S.win, rb, c0, t, c);
-      if (r.state) {
-        S.list[i] |= 0x4000u;
-        S.full = 1u;
+    // by all the rules, the cell in place `at` of the list, if this lane (its
+    // pair) has one
+    const auto full = [&](bool pair, bool on, bool stores, unsigned at) {
+      const unsigned ent = on ? S.list[at] : (unsigned)(T::Halo * T::W);
+      const int t = (int)ent / T::W, c = (int)ent % T::W;
+      const YValue r = step_y_full<T>(X, Y, S.win, rb, c0, pair, on, t, c);
+      if (!on || !stores) return;
+      if (r.scan) {
+        S.list[at] = (uint16_t)(ent | 0x8000u);
+        atomicOr(&S.scans[c >> 5], 1u << (c & 31));
       } else {
         store(t, c, r.out);
       }
-    }
-    __syncthreads();
-    if (S.full) {  // a pair of lanes each
-      const int lane = tid & 31;
-      for (unsigned base = (unsigned)(tid >> 5) * 16u; base < cy; base += T::Threads / 2) {
-        const unsigned i = base + (unsigned)(lane >> 1);
-        const unsigned ent = i < cy ? S.list[i] : 0u;
-        const bool on = (ent & 0x4000u) != 0u;
-        if (!__any_sync(0xffffffffu, on)) continue;
-        const int t = on ? (int)(ent & 0x3fffu) / T::W : T::Halo, c = (int)(ent & 0x3fffu) % T::W;
-        const YValue r = step_y_full<T>(X, Y, S.win, rb, c0, on, t, c);
-        if (on && !(lane & 1)) {
-          if (r.state == 2) {
-            S.list[i] = (uint16_t)((ent & 0x3fffu) | 0x8000u);
-            atomicOr(&S.scans[c >> 5], 1u << (c & 31));
-          } else {
-            store(t, c, r.out);
-          }
+    };
+    // cells with all the rules' rows in the window, and those in the first and
+    // last rows, a pair of lanes each
+    WarpQueue Q{S.queue[tid >> 5][0]}, E{S.queue[tid >> 5][1]};
+    for (unsigned base = first;; base += T::Threads) {
+      const unsigned i = base + lane;
+      bool hard = false, end = false;
+      if (i < cy) {
+        const int t = S.list[i] / T::W, c = S.list[i] % T::W;
+        const XValue r = step_y_shore<T>(Y, S.win, rb, c0, t, c);
+        hard = !r.ok;
+        end = T::Halo < 3 && (t < 3 || t >= T::Rows - 3);
+        if (r.ok) store(t, c, r.out);
+      }
+      const bool more = base + T::Threads < cy;
+      unsigned at;
+      Q.push(hard && !end, i);
+      if (Q.n >= 32 || (Q.n && !more)) {
+        const bool on = Q.peek(lane, at);
+        full(false, on, true, at);
+        Q.pop(32);
+      }
+      if (T::Halo < 3) {
+        E.push(hard && end, i);
+        while (E.n >= 16 || (E.n && !more)) {
+          const bool on = E.peek(lane >> 1, at);
+          full(true, on, !(lane & 1), at);
+          E.pop(16);
         }
       }
-      __syncthreads();
+      if (!more && !Q.n) break;
     }
+    __syncthreads();
     if (S.scans[0] | S.scans[1]) {
       // remainders on land: zeroed when the x-swept column holds a wet cell
       // anywhere, else left as they are; the block looks through each of their
@@ -1175,7 +1276,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     mbar_init(&S.bar, 1);
-    S.n[0] = S.n[1] = S.full = S.scans[0] = S.scans[1] = 0u;
+    S.n[0] = S.n[1] = S.scans[0] = S.scans[1] = 0u;
     S.k[0] = K.x;
     S.k[1] = K.y;
     fence_mbar_init();
@@ -1228,7 +1329,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const
   copy(S.k, &A->K, sizeof(PairPair));
   if (tid == 0) {
     mbar_init(&S.bar, 1);
-    S.n[0] = S.n[1] = S.full = S.scans[0] = S.scans[1] = 0u;
+    S.n[0] = S.n[1] = S.scans[0] = S.scans[1] = 0u;
     fence_mbar_init();
   }
   __syncthreads();
