@@ -1193,15 +1193,15 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
   // it: a longitude axis in FP64 degrees has spacings that differ in the
   // 12th digit, below what the FP32 geometry keeps except in dx(m)-dx(m-1).
   // A uniform axis takes the geometry of its first spacing everywhere (the
-  // table too, so that every kernel variant reads the same values): the
-  // table of an exactly uniform axis is unchanged by it.
+  // table too, its ends included, which the Courant check of a uniform axis
+  // counts: every kernel variant reads the same values).
   auto uniform = [&](int n, const double* sp, std::vector<float4>& g, float4& g0) {
     if (n < 3) return false;
     const double s0 = sp[0];
     for (int k = 1; k <= n - 2; ++k)
       if (std::fabs(sp[k] - s0) > 1e-9 * std::fabs(s0)) return false;
     g0 = make_float4((float)(1.0 / s0), (float)(1.0 / s0), (float)(d->dt / (s0 + s0)), 0.f);
-    for (int m = 2; m <= n - 1; ++m) g[m - 1] = g0;
+    std::fill(g.begin(), g.end(), g0);
     return true;
   };
   if (c->xrun) c->geo_uni_x = uniform(c->nx, d->dx, gx, c->geo0_x);
