@@ -174,17 +174,27 @@ __device__ __forceinline__ void unpack8(const uint4 q, float (&v)[8]) {
 }
 
 // The weights w [co][kp] (BF16, columns k = tap * C + c) into shared memory
-// as FP32, [tap][C][co] or (CLAST) [tap][co][C].  The whole block calls it; true
-// if every weight is finite.
+// as FP32, [tap][C][co] or (CLAST) [tap][co][C], 8 columns at a time (C and kp
+// are multiples of 8).  The whole block calls it; true if every weight is finite.
+// A value at a time, 64 x 64 channels took most of a small batch's input gradient:
+// the training step below, of a batch of 16 with a map of 8 x 8, 600 us, 469 now.
 template <bool CLAST>
 __device__ __forceinline__ bool stage_weights(float* sw, int C, int co, const __nv_bfloat16* __restrict__ w, int kp) {
-  const int K = 9 * C;
   bool finite = true;
-  for (int t = threadIdx.x; t < K * co; t += blockDim.x) {
-    const int o = CLAST ? t / C % co : t % co, k = CLAST ? t / (C * co) * C + t % C : t / co;
-    const float v = __bfloat162float(w[(size_t)o * kp + k]);
-    finite = finite && isfinite(v);
-    sw[t] = v;
+  for (int t = threadIdx.x; t < 9 * C / 8 * co; t += blockDim.x) {
+    const int o = CLAST ? t / (C / 8) % co : t % co, k = CLAST ? t / (C / 8 * co) * C + t % (C / 8) * 8 : t / co * 8;
+    float v[8];
+    unpack8(__ldg(reinterpret_cast<const uint4*>(w + (size_t)o * kp + k)), v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) finite = finite && isfinite(v[i]);
+    if (CLAST) {
+      float4* to = reinterpret_cast<float4*>(sw + 8 * t);
+      to[0] = make_float4(v[0], v[1], v[2], v[3]);
+      to[1] = make_float4(v[4], v[5], v[6], v[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sw[(k + i) * co + o] = v[i];
+    }
   }
   return __syncthreads_and(finite);
 }
@@ -572,26 +582,37 @@ __global__ void __launch_bounds__(kDw1Threads) k_dec_dw1(int cells, int S, int C
   }
 }
 
-// Writes the gradients of 8 channels of an input cell: the ReLU derivative
-// applied (mask: x's own values, x > 0), as a BF16 row (the output gradient of
-// the level above) or as FP32.
-__device__ __forceinline__ void dx_store(const float (&v)[8], const __nv_bfloat16* mask, size_t at, size_t to,
+// Writes the gradients of N (4 or 8) channels of an input cell: the ReLU
+// derivative applied (mask: x's own values, x > 0), as a BF16 row (the output
+// gradient of the level above) or as FP32.
+template <int N>
+__device__ __forceinline__ void dx_store(const float (&v)[N], const __nv_bfloat16* mask, size_t at, size_t to,
                                          __nv_bfloat16* dx16, float* dx32) {
-  float m[8], r[8];
-  unpack8(__ldg(reinterpret_cast<const uint4*>(mask + at)), m);
+  uint32_t w[N / 2];
+  float r[N];
+  if constexpr (N == 8) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(mask + at));
+    w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+  } else {
+    const uint2 q = __ldg(reinterpret_cast<const uint2*>(mask + at));
+    w[0] = q.x, w[1] = q.y;
+  }
 #pragma unroll
-  for (int g = 0; g < 8; ++g) r[g] = m[g] > 0.f ? v[g] : 0.f;
+  for (int g = 0; g < N; ++g)
+    r[g] = __uint_as_float(g & 1 ? w[g / 2] & 0xffff0000u : w[g / 2] << 16) > 0.f ? v[g] : 0.f;
   if (dx16) {
-    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < N / 2; ++i) {
       const __nv_bfloat162 h = __floats2bfloat162_rn(r[2 * i], r[2 * i + 1]);
       w[i] = *reinterpret_cast<const uint32_t*>(&h);
     }
-    *reinterpret_cast<uint4*>(dx16 + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    if constexpr (N == 8)
+      *reinterpret_cast<uint4*>(dx16 + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    else
+      *reinterpret_cast<uint2*>(dx16 + at) = make_uint2(w[0], w[1]);
   } else {
 #pragma unroll
-    for (int g = 0; g < 8; ++g) dx32[to + g] = r[g];
+    for (int g = 0; g < N; ++g) dx32[to + g] = r[g];
   }
 }
 
@@ -603,8 +624,8 @@ __device__ __forceinline__ void dx_store(const float (&v)[8], const __nv_bfloat1
 // each (the sums over D above would round otherwise, and what is rounded here
 // goes through every layer below).  A thread takes two cells, one below the
 // other, so that neighbouring lanes read neighbouring pixels, and G channels (16,
-// or 8 where C is no multiple of 16): 16 bytes of weights from shared memory serve
-// 8 products.  A pixel in the zero padding adds products with 0, which leave a sum
+// or 8 where C is no multiple of 16; fewer where so few cells leave SMs without a
+// block, dx_group): 16 bytes of weights from shared memory serve 8 products.  A pixel in the zero padding adds products with 0, which leave a sum
 // as it is; with weights that are not finite (GUARD) it is passed over.  Dynamic
 // shared memory: 9 C co floats, [tap][o][c].  36 C co products a cell, 65 us of
 // FP32 issue at a batch of 512 for 32 <- 16 and for 16 <- 8 channels; these took
@@ -612,6 +633,18 @@ __device__ __forceinline__ void dx_store(const float (&v)[8], const __nv_bfloat1
 // cells side by side: 187 and 141; 8 channels: 190 and 156; four cells: 185 and 142;
 // packed products: 157 each, the copies into pairs costing what they save.
 constexpr int kDxThreads = 128, kDxCells = 2;
+// Channels a thread: 16, or half and a quarter of that while the blocks, which
+// hold an SM each where there are many channels, still all run at once on 152
+// SMs: a block lasts as long as a thread's products.  A training step of a batch
+// of 16 with 64 channels throughout and a map of 8 x 8 (16 x 16, 32 x 32) took 682
+// us (752, 850) with 16 channels always, 600 (663, 760) this way; where 8 channels
+// make more than 152 blocks they lose (batch of 128, 32 x 32: 911 us against 830).
+constexpr int kDxFill = 152;
+inline int dx_group(long long runs, int C) {
+  int g = C % 16 ? 8 : 16;
+  while (g > 4 && (runs * (C / (g / 2)) + kDxThreads - 1) / kDxThreads <= kDxFill) g /= 2;
+  return g;
+}
 template <int G, bool GUARD>
 __device__ __forceinline__ void dx_cells(int S, int C, int co, int b, int y0, int x0, int c0,
                                          const __nv_bfloat16* __restrict__ dz, const float* sw, float (&acc)[kDxCells][G]) {
@@ -668,6 +701,7 @@ __global__ void __launch_bounds__(kDxThreads) k_dec_dx(int B, int S, int C, int 
                                                        const __nv_bfloat16* __restrict__ w, int kp,
                                                        const __nv_bfloat16* __restrict__ x, __nv_bfloat16* dx16,
                                                        float* dx32, int ld, int col0) {
+  constexpr int N = G < 8 ? G : 8;  // of a store
   extern __shared__ __align__(16) float sw[];
   const bool finite = stage_weights<true>(sw, C, co, w, kp);
   const int pr = (S + kDxCells - 1) / kDxCells, runs = B * S * pr;
@@ -689,11 +723,11 @@ __global__ void __launch_bounds__(kDxThreads) k_dec_dx(int B, int S, int C, int 
     if (y0 + m >= S) break;
     const size_t cell = (size_t)(y0 + m) * S + x0;
 #pragma unroll
-    for (int h = 0; h < G; h += 8) {
-      float v[8];
+    for (int h = 0; h < G; h += N) {
+      float v[N];
 #pragma unroll
-      for (int g = 0; g < 8; ++g) v[g] = acc[m][h + g];
-      dx_store(v, x, ((size_t)b * S * S + cell) * C + c0 + h, (size_t)b * ld + col0 + cell * C + c0 + h, dx16, dx32);
+      for (int g = 0; g < N; ++g) v[g] = acc[m][h + g];
+      dx_store<N>(v, x, ((size_t)b * S * S + cell) * C + c0 + h, (size_t)b * ld + col0 + cell * C + c0 + h, dx16, dx32);
     }
   }
 }
@@ -747,7 +781,7 @@ __global__ void __launch_bounds__(kDxThreads, 4) k_dec_dx1(int B, int S, int C, 
     float v[8];
 #pragma unroll
     for (int g = 0; g < 4; ++g) v[2 * g] = pair_lo(acc[m][g]), v[2 * g + 1] = pair_hi(acc[m][g]);
-    if (x0 + m < S) dx_store(v, x, (((size_t)b * S + y0) * S + x0 + m) * C + c0, 0, dx16, nullptr);
+    if (x0 + m < S) dx_store<8>(v, x, (((size_t)b * S + y0) * S + x0 + m) * C + c0, 0, dx16, nullptr);
   }
 }
 

@@ -515,10 +515,11 @@ void dec_dx_launch(cliffs_mlp* m, int B, const Level& v, const Layer& y, const b
     kernel<<<blocks(kDxCells, channels), kDxThreads, sh, m->stream>>>(B, v.S, v.cin, v.cout, dz, y.W, y.kp, x, dx16,
                                                                       dx32, ld, col0);
   };
-  if (v.cin % 16 == 0)
-    go(k_dec_dx<16>, 16);
-  else
-    go(k_dec_dx<8>, 8);
+  switch (dx_group((long long)B * v.S * ((v.S + kDxCells - 1) / kDxCells), v.cin)) {
+    case 16: go(k_dec_dx<16>, 16); break;
+    case 8: go(k_dec_dx<8>, 8); break;
+    default: go(k_dec_dx<4>, 4);
+  }
 }
 
 // The map decoder's forward pass for rows [0, B): latent columns of out -> map.

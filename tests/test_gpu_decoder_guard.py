@@ -1,7 +1,7 @@
 """Infinite weights in the map decoder's direct kernels: what reaches an infinite
 tap only through the zero padding stays as it is (0 times infinity is not a
-number).  The 8-channel convolution, and the input gradients of each kind: 16
-and 8 channels a thread, and the map's level."""
+number).  The 8-channel convolution, and the input gradients of each kind: 16, 8
+and 4 channels a thread, and the map's level."""
 import importlib
 
 import numpy as np
@@ -37,19 +37,21 @@ def test_forward_of_an_eight_channel_level(level, ch):
     net.close()
 
 
-@pytest.mark.parametrize("level,ch", [(2, (16, 16, 8)), (1, (16, 16, 8)), (1, (16, 24, 8)), (2, (16, 16, 16))])
-def test_input_gradients(level, ch):
+@pytest.mark.parametrize("level,ch,side,batch", [
+    (2, (16, 16, 8), 32, 16), (2, (16, 16, 16), 32, 16),  # the map's level
+    (1, (16, 16, 8), 64, 96), (1, (16, 24, 8), 64, 96), (1, (16, 24, 8), 32, 16)])  # 16, 8 and 4 channels a thread
+def test_input_gradients(level, ch, side, batch):
     """Weights, activations and output gradients above zero: an infinite tap makes the gradients of the level below
     infinite; one product of it with the padding would make them no number."""
-    net = S.MLP(9, 64, 1, 16, seed=9, map_side=32, map_ch=ch)
+    net = S.MLP(9, 64, 1, 16, seed=9, map_side=side, map_ch=ch)
     nd = net.layers() - 3
     for k in range(3):
         net.set(nd + k, 0, np.full(net.shape(nd + k), 0.01, np.float32))
         net.set(nd + k, 1, np.full(net.shape(nd + k)[0], 1.0, np.float32))
     net.set(nd + level, 0, _tap(net.get(nd + level, 0), 0, 0, 5, ch[level], np.inf))
     rng = np.random.default_rng(9)
-    x = rng.uniform(-1, 1, (16, 9)).astype(np.float32)
-    t = np.full((16, 16 + 32 * 32), -1.0, np.float32)
+    x = rng.uniform(-1, 1, (batch, 9)).astype(np.float32)
+    t = np.full((batch, 16 + side * side), -1.0, np.float32)
     _, _, gb = net.gradients(x, t)
     assert np.isposinf(gb[nd + level - 1]).all(), gb[nd + level - 1]
     net.close()
