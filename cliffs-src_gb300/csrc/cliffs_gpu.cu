@@ -186,8 +186,7 @@ struct cliffs_ctx {
   } win[2];  // StepLarge's; StepSmall's and StepTiny's
   bool step_ok = false;
   int step_size = STEP_LARGE;  // the tile of the grid's whole steps
-  int* step_order = nullptr;   // its tiles with the coasts first (nullptr: by bands), and the coasts' number
-  int step_coast = 0;
+  int* step_order = nullptr;   // its tiles with the coasts first, for steps from either copy (nullptr: by bands)
   int grid_sx = 0, grid_sy = 0;  // resident blocks of staged_x / staged_y
   unsigned long long stage_ns = 2000000000ull;  // limit of one stage wait
   // fast-kernel sweeps launched as programmatic dependents of the previous
@@ -552,14 +551,15 @@ bool coasts_first(int64_t tiles, int size, int sms) {
   return tiles <= 6ll * sms * (size == STEP_LARGE ? StepLarge::Blocks : StepSmall::Blocks);
 }
 
-// Flags of the tiles that hold a coast.
-void tile_coasts(int size, int tiles, int nx, int ny, int pitch, const float* dep, uint8_t* flags, cudaStream_t st) {
+// Calls f with a value of the type of tiles of this size.
+template <class F>
+void with_tile(int size, F f) {
   if (size == STEP_LARGE)
-    k_tile_coast<StepLarge><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+    f(StepLarge{});
   else if (size == STEP_SMALL)
-    k_tile_coast<StepSmall><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+    f(StepSmall{});
   else
-    k_tile_coast<StepTiny><<<tiles, 128, 0, st>>>(nx, ny, pitch, dep, flags);
+    f(StepTiny{});
 }
 
 int device_sms(int dev) {
@@ -909,7 +909,7 @@ cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepA
   const unsigned gx = (unsigned)((c->nx + T::W - 1) / T::W), gy = (unsigned)((c->ny + T::R - 1) / T::R);
   cfg.gridDim = ORDERED ? dim3(gx * gy) : dim3(gx, gy);
   cfg.blockDim = dim3(T::Threads);
-  const int* o = c->step_order;
+  const int* o = c->step_order + (ORDERED && C.flip ? gx * gy : 0u);
   if (!c->geo_uni_x || !c->geo_uni_y)
     return cudaLaunchKernelEx(&cfg, step_kernel<T, GEO_TABLE, GEO_TABLE, ORDERED>, A.X, A.Y, A.M, C, A.K, o);
   if (c->scl_y || c->lscale)
@@ -922,7 +922,7 @@ cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepA
 int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
   const int s = c->cur;
   const StepArgs A = step_args(c, s, ex, ey, c->step_size);
-  const StepCtl C{S.wait_ns, S.extra, s, c->step_coast};
+  const StepCtl C{S.wait_ns, S.extra, s};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -1131,6 +1131,9 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
   c->step_size = step_size(step_tiles(STEP_LARGE, c->nx, c->ny), step_tiles(STEP_TINY, c->nx, c->ny), sms);
   const int tiles = step_tiles(c->step_size, c->nx, c->ny);
   uint8_t* tile_flags = nullptr;
+  // the status words, the worklist's counters and the tile order's, 256 bytes
+  // each, cleared together
+  constexpr int kWords = 3 * 64;
   auto layout = [&](char* base) {
     size_t off = 0;
     carve(base, off, &c->dep, cells);
@@ -1145,20 +1148,20 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     carve(base, off, &c->geo_y, (size_t)c->ny);
     carve(base, off, &c->scl_y, (size_t)c->ny);
     carve(base, off, &c->lscale, (size_t)c->ny);
-    carve(base, off, &c->status, 2);
+    carve(base, off, &c->status, kWords);
     carve(base, off, &c->d_flag, 1);
     carve(base, off, &c->list, n64);
     carve(base, off, &c->edge_x, (size_t)c->ny * 6);
     carve(base, off, &c->edge_y, (size_t)c->nx * 6);
-    carve(base, off, &c->cnt, 2);
     carve(base, off, &c->dep64, n64);
     carve(base, off, &c->xfer, 3 * n64);
-    carve(base, off, &c->step_order, (size_t)tiles + 1);
+    carve(base, off, &c->step_order, 2 * (size_t)tiles);
     carve(base, off, &tile_flags, (size_t)tiles);
     return off;
   };
   if (dalloc(&c->arena, layout(nullptr))) return fail(CLIFFS_ERR_NOMEM);
   layout(c->arena);
+  c->cnt = c->status + kWords / 3;
   // bathymetry: the FP64 depth as passed, and its rounding in padded rows;
   // the host builds the geometry meanwhile, and one synchronisation at the
   // end covers both
@@ -1167,11 +1170,14 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     return fail(CLIFFS_ERR_CUDA);
   ++c->launches;
   k_dep_from64<<<grid2(c->pitch, c->ny), 128, 0, c->stream>>>(c->nx, c->ny, c->pitch, c->dep64, c->dep);
+  if (cudaMemsetAsync(c->status, 0, kWords * sizeof(unsigned), c->stream) != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   const bool ordered = c->xrun && c->yrun && coasts_first(tiles, c->step_size, sms);
   if (ordered) {  // the order of whole steps' tiles
-    c->launches += 2;
-    tile_coasts(c->step_size, tiles, c->nx, c->ny, c->pitch, c->dep, tile_flags, c->stream);
-    k_tile_order<<<1, 1024, 0, c->stream>>>(tiles, tile_flags, c->step_order, c->step_order + tiles);
+    ++c->launches;
+    with_tile(c->step_size, [&](auto T) {
+      k_tile_order<decltype(T)><<<tiles, 128, 0, c->stream>>>(c->nx, c->ny, c->pitch, c->dep, tile_flags,
+                                                              c->status + kWords / 3 * 2, c->step_order);
+    });
   }
   if (cudaGetLastError() != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   // geometry tables
@@ -1230,11 +1236,6 @@ int cliffs_gpu_create(const cliffs_grid_desc* d, cliffs_ctx** out) {
     put(c->scl_y, sy.data(), sy.size() * sizeof(float));
     put(c->lscale, ls.data(), ls.size() * sizeof(float2));
     if (cudaMemcpyAsync(lo, span.data(), span.size(), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
-        cudaMemsetAsync(c->status, 0, 2 * sizeof(unsigned), c->stream) != cudaSuccess ||
-        cudaMemsetAsync(c->cnt, 0, 2 * sizeof(uint32_t), c->stream) != cudaSuccess ||
-        (ordered &&
-         cudaMemcpyAsync(&c->step_coast, c->step_order + tiles, sizeof(int), cudaMemcpyDeviceToHost, c->stream) !=
-             cudaSuccess) ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
       return fail(CLIFFS_ERR_CUDA);
   }
@@ -2915,9 +2916,11 @@ struct cliffs_batch {
   // whole steps in one kernel (batch_step_kernel) for the one-tile graph
   // plans: every scenario's arguments for the steps from its state copy cur
   // ([0]) and back to it ([1]), the tile list, and the variant
+  char* d_whole = nullptr;  // the allocation that holds them
   StepArgs* d_step[2] = {nullptr, nullptr};
   int4* d_step_order = nullptr;
-  int step_tiles = 0, step_coast = 0;
+  int step_tiles = 0;
+  bool step_ordered = false;  // coasts first, in an order for each copy
   int step_geo = GEO_FLAT;
   int step_size = STEP_LARGE;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
@@ -2984,9 +2987,7 @@ static void batch_free(cliffs_batch* b) {
   if (b->d_gauge) cudaFree(b->d_gauge);
   if (b->d_grec) cudaFree(b->d_grec);
   if (b->d_ymaps) cudaFree(b->d_ymaps);
-  for (StepArgs* a : b->d_step)
-    if (a) cudaFree(a);
-  if (b->d_step_order) cudaFree(b->d_step_order);
+  if (b->d_whole) cudaFree(b->d_whole);
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 
@@ -3070,8 +3071,6 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
   bool whole = true;
   for (int k = 0; k < n; ++k) whole = whole && ctxs[k]->step_ok;
   if (whole) {
-    std::vector<StepArgs> sa[2];
-    std::vector<int4> order;
     bool uniform = true, plain = true;
     int64_t large = 0, tiny = 0;
     for (int k = 0; k < n; ++k) {
@@ -3079,50 +3078,46 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
       tiny += step_tiles(STEP_TINY, ctxs[k]->nx, ctxs[k]->ny);
     }
     b->step_size = step_size(large, tiny, b->sms);
+    b->step_tiles = 0;
+    for (int k = 0; k < n; ++k) b->step_tiles += step_tiles(b->step_size, ctxs[k]->nx, ctxs[k]->ny);
+    // on the device in one piece: the arguments and the tiles in the scenarios'
+    // order, copied; with coasts first also their two orders, a counter and the flags
+    const size_t na = n * sizeof(StepArgs), nt = b->step_tiles * sizeof(int4);
+    b->step_ordered = coasts_first(b->step_tiles, b->step_size, b->sms);
+    const size_t copied = 2 * na + nt, words = copied + 2 * nt;
+    if (dalloc(&b->d_whole, b->step_ordered ? words + 16 + b->step_tiles : copied)) return fail(CLIFFS_ERR_NOMEM);
+    std::vector<char> host(copied);
+    int4* tile = reinterpret_cast<int4*>(host.data() + 2 * na);
+    int w = 0, r = 0;
+    with_tile(b->step_size, [&](auto T) { w = T.W, r = T.R; });
     for (int k = 0; k < n; ++k) {
       const cliffs_ctx* c = ctxs[k];
-      for (int q = 0; q < 2; ++q)
-        sa[q].push_back(step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr, b->step_size));
-      const int t = step_tiles(b->step_size, c->nx, c->ny);
-      const int w = b->step_size == STEP_LARGE ? StepLarge::W : StepSmall::W;
-      const int r = b->step_size == STEP_LARGE ? StepLarge::R : b->step_size == STEP_SMALL ? StepSmall::R : StepTiny::R;
-      const int across = (c->nx + w - 1) / w;
-      for (int q = 0; q < t; ++q) order.push_back(make_int4(k, q / across * r, q % across * w, 0));
+      for (int q = 0; q < 2; ++q) {
+        const StepArgs A = step_args(c, q ? 1 - c->cur : c->cur, nullptr, nullptr, b->step_size);
+        std::memcpy(host.data() + q * na + k * sizeof(StepArgs), &A, sizeof(StepArgs));
+      }
+      for (int y = 0; y < c->ny; y += r)
+        for (int x = 0; x < c->nx; x += w) *tile++ = make_int4(k, y, x, 0);
       uniform = uniform && c->geo_uni_x && c->geo_uni_y;
       plain = plain && !c->scl_y && !c->lscale;
     }
     b->step_geo = !uniform ? GEO_TABLE : plain ? GEO_FLAT : GEO_METRIC;
-    b->step_tiles = (int)order.size();
-    if (coasts_first(b->step_tiles, b->step_size, b->sms)) {  // coasts first, then the others
-      uint8_t* d_flags = nullptr;
-      std::vector<uint8_t> flags(order.size());
-      if (dalloc(&d_flags, flags.size())) return fail(CLIFFS_ERR_NOMEM);
-      int t0 = 0;
-      for (int k = 0; k < n; ++k) {
-        const cliffs_ctx* c = ctxs[k];
-        const int t = step_tiles(b->step_size, c->nx, c->ny);
-        tile_coasts(b->step_size, t, c->nx, c->ny, c->pitch, c->dep, d_flags + t0, b->stream);
-        t0 += t;
-      }
-      const bool got = cudaMemcpyAsync(flags.data(), d_flags, flags.size(), cudaMemcpyDeviceToHost, b->stream) ==
-                           cudaSuccess &&
-                       cudaStreamSynchronize(b->stream) == cudaSuccess;
-      cudaFree(d_flags);
-      if (!got) return fail(CLIFFS_ERR_CUDA);
-      std::vector<int4> sorted;
-      for (int pass = 0; pass < 2; ++pass) {
-        for (size_t q = 0; q < order.size(); ++q)
-          if ((flags[q] != 0) == (pass == 0)) sorted.push_back(order[q]);
-        if (pass == 0) b->step_coast = (int)sorted.size();
-      }
-      order.swap(sorted);
+    for (int q = 0; q < 2; ++q) b->d_step[q] = reinterpret_cast<StepArgs*>(b->d_whole + q * na);
+    b->d_step_order = reinterpret_cast<int4*>(b->d_whole + 2 * na);
+    bool ok = cudaMemcpyAsync(b->d_whole, host.data(), copied, cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
+    if (b->step_ordered) {
+      const int4* list = b->d_step_order;
+      b->d_step_order += b->step_tiles;
+      unsigned* done = reinterpret_cast<unsigned*>(b->d_whole + words);
+      uint8_t* flags = reinterpret_cast<uint8_t*>(done + 4);
+      ok = ok && cudaMemsetAsync(done, 0, sizeof(unsigned), b->stream) == cudaSuccess;
+      with_tile(b->step_size, [&](auto T) {
+        k_batch_order<decltype(T)><<<b->step_tiles, 128, 0, b->stream>>>(b->d_step[0], list, flags, done,
+                                                                         b->d_step_order);
+      });
+      ok = ok && cudaGetLastError() == cudaSuccess;
     }
-    if (dalloc(&b->d_step[0], (size_t)n) || dalloc(&b->d_step[1], (size_t)n) || dalloc(&b->d_step_order, order.size()))
-      return fail(CLIFFS_ERR_NOMEM);
-    if (cudaMemcpy(b->d_step[0], sa[0].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
-        cudaMemcpy(b->d_step[1], sa[1].data(), n * sizeof(StepArgs), cudaMemcpyHostToDevice) ||
-        cudaMemcpy(b->d_step_order, order.data(), order.size() * sizeof(int4), cudaMemcpyHostToDevice))
-      return fail(CLIFFS_ERR_CUDA);
+    if (!ok || cudaStreamSynchronize(b->stream) != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   }
   b->plan.mode = b->max_ctas > 0 ? CLIFFS_BATCH_PERSISTENT : CLIFFS_BATCH_GRAPH;
   b->plan.ctas_per_sm = std::max(1, b->max_ctas);
@@ -3229,8 +3224,8 @@ static void batch_step_launch(cliffs_batch* b, const BatchStep& B, const StepCtl
 }
 
 static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
-  const BatchStep B{b->d_step[odd], b->d_step_order};
-  const StepCtl C{S.wait_ns, S.extra, odd, b->step_coast};
+  const BatchStep B{b->d_step[odd], b->d_step_order + (b->step_ordered && odd ? b->step_tiles : 0)};
+  const StepCtl C{S.wait_ns, S.extra, !b->step_ordered && odd};
   if (b->step_size == STEP_LARGE)
     batch_step_launch<StepLarge>(b, B, C);
   else if (b->step_size == STEP_SMALL)

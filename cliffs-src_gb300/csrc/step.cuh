@@ -156,8 +156,7 @@ struct PairPair {
 struct StepCtl {
   unsigned long long wait_ns;  // limit of the window's wait
   unsigned extra;              // bytes it waits for beyond its copies: 0, except in the timeout self-test
-  int flip;                    // tiles beyond the first `coast` last to first, or bands
-  int coast;                   // tiles at the front of the order that go first in every step
+  int flip;                    // bands, or a batch's tiles without coasts first, last to first
 };
 
 // rsqrtf for arguments that are not subnormal (celerities: g * max(H, ground);
@@ -1211,19 +1210,17 @@ __device__ __forceinline__ void step_tile(const SweepArgs& X, const SweepArgs& Y
 // cells make them last longer (a step ends with its slowest block, which is to
 // start early); the others band by band, every other step last to first: a
 // step starts on the rows that the one before it wrote last, which are still
-// in L2.  The coast is that of the depth at the context's creation: the order
-// changes no result.
-__device__ __forceinline__ int tile_at(const StepCtl& C, int id, int tiles) {
-  return C.flip && id >= C.coast ? tiles - 1 - (id - C.coast) : id;
-}
+// in L2.  So there are two orders of a grid's tiles, one behind the other, for the
+// steps from either copy of the state.  The coast is that of the depth at the
+// context's creation: the order changes no result.
 
-// Whether a tile or a cell beside it holds land and sea.
+// Whether the tile of T at column x0, row y0 (0-based), or a cell beside it, holds
+// land and sea.  The whole block calls it.
 template <class T>
-__global__ void k_tile_coast(int nx, int ny, int pitch, const float* __restrict__ dep, uint8_t* flags) {
-  const int tx = (int)blockIdx.x % ((nx + T::W - 1) / T::W), ty = (int)blockIdx.x / ((nx + T::W - 1) / T::W);
+__device__ __forceinline__ bool coast_tile(int nx, int ny, int pitch, const float* __restrict__ dep, int x0, int y0) {
   bool land = false, sea = false;
   for (int i = threadIdx.x; i < (T::W + 2) * (T::R + 2); i += blockDim.x) {
-    const int x = tx * T::W - 1 + i % (T::W + 2), y = ty * T::R - 1 + i / (T::W + 2);
+    const int x = x0 - 1 + i % (T::W + 2), y = y0 - 1 + i / (T::W + 2);
     if (x < 0 || x >= nx || y < 0 || y >= ny) continue;
     const bool l = dep[(size_t)y * pitch + x] < 0.f;
     land = land || l;
@@ -1231,38 +1228,59 @@ __global__ void k_tile_coast(int nx, int ny, int pitch, const float* __restrict_
   }
   land = __syncthreads_or(land);
   sea = __syncthreads_or(sea);
-  if (threadIdx.x == 0) flags[blockIdx.x] = land && sea;
+  return land && sea;
 }
 
-// order: the tiles with a flag, then the others, each in their order; count:
-// those with one.  One block of 1024 threads.
-__global__ void k_tile_order(int tiles, const uint8_t* __restrict__ flags, int* order, int* count) {
-  __shared__ int s_warp[32], s_base;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int base = 0;
-  for (int pass = 0; pass < 2; ++pass) {
-    for (int i0 = 0; i0 < tiles; i0 += 1024) {
-      const int i = i0 + tid;
-      const bool take = i < tiles && (flags[i] != 0) == (pass == 0);
-      const unsigned m = __ballot_sync(0xffffffffu, take);
-      if (lane == 0) s_warp[warp] = __popc(m);
-      __syncthreads();
-      if (tid == 0) {
-        int sum = base;
-        for (int w = 0; w < 32; ++w) {
-          const int c = s_warp[w];
-          s_warp[w] = sum;
-          sum += c;
-        }
-        s_base = sum;
-      }
-      __syncthreads();
-      if (take) order[s_warp[warp] + __popc(m & ((1u << lane) - 1u))] = i;
-      base = s_base;
-      __syncthreads();
-    }
-    if (pass == 0 && tid == 0) *count = base;
+// A block of 128 threads a tile: its flag, and in the block that finishes last both
+// orders of them all by put(place, tile): from place 0 the tiles with a flag, then
+// the others, each in their order; from place gridDim.x the others last to first.
+// done: 0 before the launch.
+template <class Put>
+__device__ __forceinline__ void order_tiles(bool coast, uint8_t* flags, unsigned* done, Put put) {
+  __shared__ int s_warp[4];
+  __shared__ bool s_last;
+  const int tid = threadIdx.x, lane = tid & 31, tiles = (int)gridDim.x;
+  if (tid == 0) {
+    flags[blockIdx.x] = coast;
+    __threadfence();
+    s_last = atomicAdd(done, 1u) == (unsigned)tiles - 1u;
   }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const int per = (tiles + 127) / 128, lo = min(tid * per, tiles), hi = min(lo + per, tiles);
+  int mine = 0;
+  for (int i = lo; i < hi; ++i) mine += __ldcg(flags + i);
+  int upto = mine;  // of the warp's lanes so far
+#pragma unroll
+  for (int d = 1; d < 32; d *= 2) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, d);
+    if (lane >= d) upto += v;
+  }
+  if (lane == 31) s_warp[tid >> 5] = upto;
+  __syncthreads();
+  int before = upto - mine, all = 0;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    if (w < tid >> 5) before += s_warp[w];
+    all += s_warp[w];
+  }
+  int a = before, b = all + lo - before;
+  for (int i = lo; i < hi; ++i) {
+    const bool first = __ldcg(flags + i) != 0;
+    const int place = first ? a++ : b++;
+    put(place, i);
+    put(tiles + (first ? place : tiles - 1 - (place - all)), i);
+  }
+}
+
+// The order of a grid's tiles (gridDim.x of them).
+template <class T>
+__global__ void __launch_bounds__(128) k_tile_order(int nx, int ny, int pitch, const float* __restrict__ dep,
+                                                    uint8_t* flags, unsigned* done, int* order) {
+  const int across = (nx + T::W - 1) / T::W;
+  const bool coast = coast_tile<T>(nx, ny, pitch, dep, (int)blockIdx.x % across * T::W, (int)blockIdx.x / across * T::R);
+  order_tiles(coast, flags, done, [&](int place, int tile) { order[place] = tile; });
 }
 
 // ORDERED: a one-dimensional grid, the tiles from the order; else a grid of
@@ -1284,7 +1302,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
   int bx, by;
   if (ORDERED) {  // written once, before the context's first launch: read ahead
     const int gx = (X.n + T::W - 1) / T::W;
-    const int tile = __ldg(order + tile_at(C, (int)blockIdx.x, (int)gridDim.x));
+    const int tile = __ldg(order + blockIdx.x);
     bx = tile % gx;
     by = tile / gx;
   } else {
@@ -1312,12 +1330,22 @@ struct BatchStep {
   const int4* order;     // scenario, first row and first column of each tile
 };
 
+// The order of a batch's tiles, from the scenarios' own order `list`.
+template <class T>
+__global__ void __launch_bounds__(128) k_batch_order(const StepArgs* __restrict__ args, const int4* __restrict__ list,
+                                                     uint8_t* flags, unsigned* done, int4* order) {
+  const int4 at = list[blockIdx.x];
+  const SweepArgs& X = args[at.x].X;
+  const bool coast = coast_tile<T>(X.n, X.nlines, X.pitch, X.dep, at.z, at.y);
+  order_tiles(coast, flags, done, [&](int place, int tile) { order[place] = list[tile]; });
+}
+
 template <class T, int GX, int GY>
 __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const BatchStep B, const StepCtl C) {
   __shared__ StepShared<T> S;
   __shared__ SweepArgs sA[2];
   const int tid = threadIdx.x;
-  const int4 at = __ldg(B.order + tile_at(C, (int)blockIdx.x, (int)gridDim.x));
+  const int4 at = __ldg(B.order + (C.flip ? gridDim.x - 1 - blockIdx.x : blockIdx.x));
   const StepArgs* A = B.args + at.x;
   static_assert(sizeof(SweepArgs) % 8 == 0 && sizeof(PairPair) % 8 == 0, "copied in 8-byte words");
   const auto copy = [&](void* to, const void* from, int bytes) {
