@@ -541,12 +541,14 @@ int step_size(int64_t large, int64_t tiny, int sms) {
                                                   : STEP_TINY;
 }
 
-// Whether coasts go first among so many tiles: up to six times what the chip
-// holds at once.  Beyond, the end of a step is a small part of it, and tiles
-// taken out of their bands cost more in L2, and places that are not the block's
-// own more registers (us per step, bands and coasts first: 4320 x 2160, 8 times,
-// 90.4 and 91.8; 2048 x 2048, 3.6 times, 47.0 and 45.0; 1003 x 777 18.3 and
-// 16.1; 600 x 600 13.7 and 13.2).
+// Whether coasts go first among so many tiles of one grid: up to six times what the
+// chip holds at once.  Beyond, the end of a step is a small part of it, and tiles
+// taken out of their bands cost more in L2 (us per step, bands and coasts first:
+// 1003 x 777 18.3 and 16.1; 2048 x 2048, 3.6 times, 45.9 and 44.5; 2650 x 2650, 6.2
+// times, 69.1 and 68.9; 2900 x 2900, 7.3 times, 79.9 and 80.3; 4096 x 4096, 14 times,
+// 144.4 and 146.2).  A batch's tiles come as scenarios, not as bands of one grid, and
+// always take the order: 4 times 57.6 and 53.1, 7 times 91.1 and 87.3, 20 times 235.8
+// and 233.2, 61 times 689 and 685.
 bool coasts_first(int64_t tiles, int size, int sms) {
   return tiles <= 6ll * sms * (size == STEP_LARGE ? StepLarge::Blocks : StepSmall::Blocks);
 }
@@ -2920,7 +2922,6 @@ struct cliffs_batch {
   StepArgs* d_step[2] = {nullptr, nullptr};
   int4* d_step_order = nullptr;
   int step_tiles = 0;
-  bool step_ordered = false;  // coasts first, in an order for each copy
   int step_geo = GEO_FLAT;
   int step_size = STEP_LARGE;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
@@ -3081,11 +3082,10 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
     b->step_tiles = 0;
     for (int k = 0; k < n; ++k) b->step_tiles += step_tiles(b->step_size, ctxs[k]->nx, ctxs[k]->ny);
     // on the device in one piece: the arguments and the tiles in the scenarios'
-    // order, copied; with coasts first also their two orders, a counter and the flags
+    // order, copied, then the two orders with coasts first, a counter and the flags
     const size_t na = n * sizeof(StepArgs), nt = b->step_tiles * sizeof(int4);
-    b->step_ordered = coasts_first(b->step_tiles, b->step_size, b->sms);
     const size_t copied = 2 * na + nt, words = copied + 2 * nt;
-    if (dalloc(&b->d_whole, b->step_ordered ? words + 16 + b->step_tiles : copied)) return fail(CLIFFS_ERR_NOMEM);
+    if (dalloc(&b->d_whole, words + 16 + b->step_tiles)) return fail(CLIFFS_ERR_NOMEM);
     std::vector<char> host(copied);
     int4* tile = reinterpret_cast<int4*>(host.data() + 2 * na);
     int w = 0, r = 0;
@@ -3103,20 +3103,17 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
     }
     b->step_geo = !uniform ? GEO_TABLE : plain ? GEO_FLAT : GEO_METRIC;
     for (int q = 0; q < 2; ++q) b->d_step[q] = reinterpret_cast<StepArgs*>(b->d_whole + q * na);
-    b->d_step_order = reinterpret_cast<int4*>(b->d_whole + 2 * na);
-    bool ok = cudaMemcpyAsync(b->d_whole, host.data(), copied, cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
-    if (b->step_ordered) {
-      const int4* list = b->d_step_order;
-      b->d_step_order += b->step_tiles;
-      unsigned* done = reinterpret_cast<unsigned*>(b->d_whole + words);
-      uint8_t* flags = reinterpret_cast<uint8_t*>(done + 4);
-      ok = ok && cudaMemsetAsync(done, 0, sizeof(unsigned), b->stream) == cudaSuccess;
-      with_tile(b->step_size, [&](auto T) {
-        k_batch_order<decltype(T)><<<b->step_tiles, 128, 0, b->stream>>>(b->d_step[0], list, flags, done,
-                                                                         b->d_step_order);
-      });
-      ok = ok && cudaGetLastError() == cudaSuccess;
-    }
+    const int4* list = reinterpret_cast<const int4*>(b->d_whole + 2 * na);
+    b->d_step_order = reinterpret_cast<int4*>(b->d_whole + copied);
+    unsigned* done = reinterpret_cast<unsigned*>(b->d_whole + words);
+    uint8_t* flags = reinterpret_cast<uint8_t*>(done + 4);
+    bool ok = cudaMemcpyAsync(b->d_whole, host.data(), copied, cudaMemcpyHostToDevice, b->stream) == cudaSuccess &&
+              cudaMemsetAsync(done, 0, sizeof(unsigned), b->stream) == cudaSuccess;
+    with_tile(b->step_size, [&](auto T) {
+      k_batch_order<decltype(T)><<<b->step_tiles, 128, 0, b->stream>>>(b->d_step[0], list, flags, done,
+                                                                       b->d_step_order);
+    });
+    ok = ok && cudaGetLastError() == cudaSuccess;
     if (!ok || cudaStreamSynchronize(b->stream) != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   }
   b->plan.mode = b->max_ctas > 0 ? CLIFFS_BATCH_PERSISTENT : CLIFFS_BATCH_GRAPH;
@@ -3224,8 +3221,8 @@ static void batch_step_launch(cliffs_batch* b, const BatchStep& B, const StepCtl
 }
 
 static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
-  const BatchStep B{b->d_step[odd], b->d_step_order + (b->step_ordered && odd ? b->step_tiles : 0)};
-  const StepCtl C{S.wait_ns, S.extra, !b->step_ordered && odd};
+  const BatchStep B{b->d_step[odd], b->d_step_order + (odd ? b->step_tiles : 0)};
+  const StepCtl C{S.wait_ns, S.extra, 0};
   if (b->step_size == STEP_LARGE)
     batch_step_launch<StepLarge>(b, B, C);
   else if (b->step_size == STEP_SMALL)

@@ -156,7 +156,7 @@ struct PairPair {
 struct StepCtl {
   unsigned long long wait_ns;  // limit of the window's wait
   unsigned extra;              // bytes it waits for beyond its copies: 0, except in the timeout self-test
-  int flip;                    // bands, or a batch's tiles without coasts first, last to first
+  int flip;                    // bands last to first
 };
 
 // rsqrtf for arguments that are not subnormal (celerities: g * max(H, ground);
@@ -1345,7 +1345,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks) batch_step_kernel(const
   __shared__ StepShared<T> S;
   __shared__ SweepArgs sA[2];
   const int tid = threadIdx.x;
-  const int4 at = __ldg(B.order + (C.flip ? gridDim.x - 1 - blockIdx.x : blockIdx.x));
+  const int4 at = __ldg(B.order + blockIdx.x);
   const StepArgs* A = B.args + at.x;
   static_assert(sizeof(SweepArgs) % 8 == 0 && sizeof(PairPair) % 8 == 0, "copied in 8-byte words");
   const auto copy = [&](void* to, const void* from, int bytes) {

@@ -1,8 +1,7 @@
 """Whole steps beyond the sizes of test_gpu_step.py, against a launch per sweep
 (CLIFFS_SWEEP_DIRECT), bit for bit: batches on 64 x 30 tiles (more than 608 of
-them), with coasts first and, beyond 3648 tiles, in the scenarios' own order;
-single grids beyond 3648 tiles, which run by bands; and a line whose forcing
-ends, which goes on in one launch."""
+them); single grids beyond 3648 tiles, which run by bands; and a line whose
+forcing ends, which goes on in one launch."""
 import importlib
 
 import numpy as np
