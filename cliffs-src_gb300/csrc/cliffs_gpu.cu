@@ -924,7 +924,7 @@ cudaError_t step_launch(const cliffs_ctx* c, cudaLaunchConfig_t cfg, const StepA
 int launch_step(cliffs_ctx* c, const float* ex, const float* ey, const StageCtl& S) {
   const int s = c->cur;
   const StepArgs A = step_args(c, s, ex, ey, c->step_size);
-  const StepCtl C{S.wait_ns, S.extra, s};
+  const StepCtl C{S.wait_ns, S.extra, s, 0};
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -2921,7 +2921,7 @@ struct cliffs_batch {
   char* d_whole = nullptr;  // the allocation that holds them
   StepArgs* d_step[2] = {nullptr, nullptr};
   int4* d_step_order = nullptr;
-  int step_tiles = 0;
+  int step_tiles = 0, step_coast = 0;
   int step_geo = GEO_FLAT;
   int step_size = STEP_LARGE;
   // per scenario, in single-grid tiles: x (column chunks, rows), y (row
@@ -3082,9 +3082,10 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
     b->step_tiles = 0;
     for (int k = 0; k < n; ++k) b->step_tiles += step_tiles(b->step_size, ctxs[k]->nx, ctxs[k]->ny);
     // on the device in one piece: the arguments and the tiles in the scenarios'
-    // order, copied, then the two orders with coasts first, a counter and the flags
+    // order, copied, then the order with coasts first, their number, a counter and
+    // the flags
     const size_t na = n * sizeof(StepArgs), nt = b->step_tiles * sizeof(int4);
-    const size_t copied = 2 * na + nt, words = copied + 2 * nt;
+    const size_t copied = 2 * na + nt, words = copied + nt;
     if (dalloc(&b->d_whole, words + 16 + b->step_tiles)) return fail(CLIFFS_ERR_NOMEM);
     std::vector<char> host(copied);
     int4* tile = reinterpret_cast<int4*>(host.data() + 2 * na);
@@ -3105,15 +3106,17 @@ int cliffs_batch_create(cliffs_ctx* const* ctxs, int32_t n, cliffs_batch** out) 
     for (int q = 0; q < 2; ++q) b->d_step[q] = reinterpret_cast<StepArgs*>(b->d_whole + q * na);
     const int4* list = reinterpret_cast<const int4*>(b->d_whole + 2 * na);
     b->d_step_order = reinterpret_cast<int4*>(b->d_whole + copied);
-    unsigned* done = reinterpret_cast<unsigned*>(b->d_whole + words);
-    uint8_t* flags = reinterpret_cast<uint8_t*>(done + 4);
+    int* count = reinterpret_cast<int*>(b->d_whole + words);
+    unsigned* done = reinterpret_cast<unsigned*>(count + 1);
+    uint8_t* flags = reinterpret_cast<uint8_t*>(count + 4);
     bool ok = cudaMemcpyAsync(b->d_whole, host.data(), copied, cudaMemcpyHostToDevice, b->stream) == cudaSuccess &&
               cudaMemsetAsync(done, 0, sizeof(unsigned), b->stream) == cudaSuccess;
     with_tile(b->step_size, [&](auto T) {
       k_batch_order<decltype(T)><<<b->step_tiles, 128, 0, b->stream>>>(b->d_step[0], list, flags, done,
-                                                                       b->d_step_order);
+                                                                       b->d_step_order, count);
     });
-    ok = ok && cudaGetLastError() == cudaSuccess;
+    ok = ok && cudaGetLastError() == cudaSuccess &&
+         cudaMemcpyAsync(&b->step_coast, count, sizeof(int), cudaMemcpyDeviceToHost, b->stream) == cudaSuccess;
     if (!ok || cudaStreamSynchronize(b->stream) != cudaSuccess) return fail(CLIFFS_ERR_CUDA);
   }
   b->plan.mode = b->max_ctas > 0 ? CLIFFS_BATCH_PERSISTENT : CLIFFS_BATCH_GRAPH;
@@ -3221,8 +3224,8 @@ static void batch_step_launch(cliffs_batch* b, const BatchStep& B, const StepCtl
 }
 
 static int batch_launch_whole(cliffs_batch* b, int odd, const StageCtl& S) {
-  const BatchStep B{b->d_step[odd], b->d_step_order + (odd ? b->step_tiles : 0)};
-  const StepCtl C{S.wait_ns, S.extra, 0};
+  const BatchStep B{b->d_step[odd], b->d_step_order};
+  const StepCtl C{S.wait_ns, S.extra, odd, b->step_coast};
   if (b->step_size == STEP_LARGE)
     batch_step_launch<StepLarge>(b, B, C);
   else if (b->step_size == STEP_SMALL)
