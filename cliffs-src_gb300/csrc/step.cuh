@@ -20,18 +20,19 @@
 // Classification.  As in sweep.cuh, a cell takes the plain update when it is
 // interior and it and its neighbours are wet and subcritical; every other cell
 // is left out of the thread's stores and, unless it is dry land at rest, put
-// on the block's list, which the whole block finishes after the phase: by
-// shore_cell where no cell is flooded, else by all the rules (general_cell).
+// on the block's list, which its warps finish after the phase: by shore_cell
+// where no cell is flooded, else by all the rules (general_cell), a warp's
+// cells of the second kind together.
 // The x phase's listed cells are evaluated on the step's input, in the window
 // or, where the rows are swept in place, in global memory; the y phase's on the
 // x-swept tile.  Tiles with a coast in them take longest and go first.
 //
 // Measured (us per step, replayed from graphs, against a launch per sweep;
-// the same state bits): 4320 x 2160 sphere 89 from 144; 2048 x 2048 shelf 44.2
-// from 68.6; 1500 x 1500 28.4 from 41.0; 1201 x 903 stretched 21.1 from 29.3;
-// 1003 x 777 15.5 from 21.8; 600 x 600 12.1 from 18.4; 256 x 256 9.5 from 15.1.
-// On the shelf 204 thread instructions a cell (400 in the two sweeps), 39 bytes
-// a cell to and from DRAM, 16 warps an SM at 128 registers and 0.54
+// the same state bits): 4320 x 2160 sphere 88 from 144; 2048 x 2048 shelf 44.2
+// from 68.6; 1500 x 1500 28.4 from 41.0; 1201 x 903 stretched 20.8 from 29.3;
+// 1003 x 777 15.3 from 21.8; 600 x 600 11.6 from 18.4; 256 x 256 9.0 from 15.1.
+// On the shelf 209 thread instructions a cell (400 in the two sweeps), 39 bytes
+// a cell to and from DRAM, 16 warps an SM at 128 registers and 0.53
 // instructions an SM sub-core and cycle while it is busy: what bounds it is the
 // latency of the march and of the window's copies.  A small grid's step is the
 // time of its slowest block: on 256 x 256 (64 threads an SM) 0.95 us for the
@@ -401,15 +402,17 @@ __device__ __forceinline__ OutCell<float> step_x_value(const SweepArgs& X, int L
 // Whether the x-swept cell (row L, column i) is wet.  A dry cell between dry
 // neighbours stays dry without an evaluation.
 __device__ __forceinline__ bool step_x_wet(const SweepArgs& X, int L, int i) {
-  bool any = false;
-  float dq = 0.f;
-  for (int k = max(i - 1, 1); k <= min(i + 1, X.n); ++k) {
-    const size_t q = cidx<0>(L, k, X.pitch);
-    const float d = __ldg(X.dep + q);
-    any = any || depth_of(ld_state<false>(X.srf + q), d) > X.ph.ground;
-    if (k == i) dq = d;
+  float d[3], s[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {  // all loads at once; at a line's end the end twice
+    const size_t q = cidx<0>(L, min(max(i - 1 + t, 1), X.n), X.pitch);
+    d[t] = __ldg(X.dep + q);
+    s[t] = ld_state<false>(X.srf + q);
   }
-  return any && depth_of(step_x_value(X, L, i).s, dq) > X.ph.ground;
+  bool any = false;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) any |= depth_of(s[t], d[t]) > X.ph.ground;
+  return any && depth_of(step_x_value(X, L, i).s, d[1]) > X.ph.ground;
 }
 
 // The constants of column L that the rules at and beside cell o need.
@@ -571,8 +574,18 @@ __device__ __noinline__ YValue step_y_full(const SweepArgs& X, const SweepArgs& 
   if (!on) return r;
   const bool rest = w[3].u == 0.f && w[3].v == 0.f && depth_of(w[3].s, w[3].d) == 0.f;
   if (!anywet && !rest) {  // whether its column holds a wet cell elsewhere decides (cliffs.f:113)
-    r.scan = true;
-    return r;
+    // in the window first (rows outside the grid hold no water): a beach that a wave
+    // has left has such cells in every step, and the one block that looked through
+    // its column took a 600 x 600 step from 14.5 to 20.5 us
+#pragma unroll 4
+    for (int tt = 0; tt < T::Rows; ++tt) {
+      const RawCell<float> x = step_y_raw<T>(sm, tt, c);
+      anywet |= depth_of(x.s, x.d) > ground;
+    }
+    if (!anywet) {
+      r.scan = true;
+      return r;
+    }
   }
   C.wet = anywet;
   r.out = general_cell(w, o, C, g, Y.ph);
@@ -1036,12 +1049,23 @@ __device__ __forceinline__ bool fold_cell(const SweepArgs& X, int rb, int c0, in
 // and 46).  Gathered by the block after a barrier, 256 x 256 with one beach took
 // 9.9 us, 9.0 by warps (9.5 as they came).
 
+// The cells of a list that a warp takes at a time.  In the smaller tiles, whose
+// slowest block is the step's time, a short list is shared evenly (1003 x 777 with a
+// rough coast 18.3 us a step, 19.4 by full turns); in large tiles fewer warps take
+// full turns, and other blocks the rest (2048 x 2048 44.3, 44.5 shared; a batch of 24
+// grids 74.6, 75.2).
+template <class T>
+__device__ __forceinline__ unsigned list_share(unsigned n) {
+  constexpr unsigned kWarps = T::Threads / 32;
+  return T::InPlace ? 32u : min((n + kWarps - 1) / kWarps, 32u);
+}
+
 // The x phase's, into the window; true if a value is not finite.  The whole block
 // calls it.
 template <class T>
 __device__ __forceinline__ bool step_x_list(const SweepArgs& X, int rb, int c0, StepShared<T>& S) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const unsigned cx = S.n[0];
+  const int tid = threadIdx.x;
+  const unsigned lane = tid & 31, cx = S.n[0];
   bool bad = false;
   const auto put = [&](int t, int c, const OutCell<float>& r) {
     float* f = S.win + T::Out + t * T::Win + 4 + c;
@@ -1051,10 +1075,11 @@ __device__ __forceinline__ bool step_x_list(const SweepArgs& X, int rb, int c0, 
     bad = bad || !isfinite(r.s + r.u + r.v);
   };
   WarpQueue Q{S.queue[tid >> 5][0]};
-  for (unsigned base = (unsigned)(tid & ~31);; base += T::Threads) {
+  const unsigned share = list_share<T>(cx), round = share * (T::Threads / 32);
+  for (unsigned base = share * (unsigned)(tid >> 5);; base += round) {
     const unsigned i = base + lane;
     bool hard = false;
-    if (i < cx) {
+    if (lane < share && i < cx) {
       const int t = S.list[i] / T::W, c = S.list[i] % T::W;
       const XValue r = T::InPlace ? step_x_shore(X, rb + t, c0 + c + 1)
                                   : step_x_window_shore<T>(X, S.win, rb, c0, t, c);
@@ -1062,7 +1087,7 @@ __device__ __forceinline__ bool step_x_list(const SweepArgs& X, int rb, int c0, 
       if (r.ok) put(t, c, r.out);
     }
     Q.push(hard, i);
-    const bool last = base + T::Threads >= cx;
+    const bool last = base + round >= cx;
     if (Q.n >= 32 || (Q.n && last)) {
       unsigned at;
       if (Q.peek(lane, at)) {
@@ -1078,8 +1103,8 @@ __device__ __forceinline__ bool step_x_list(const SweepArgs& X, int rb, int c0, 
   return bad;
 }
 
-// Remainders on land, marked in the list: zeroed when the x-swept column holds a
-// wet cell anywhere, else left as they are.  The block looks through each of their
+// Remainders on land with no water in the window's part of their column, marked in
+// the list: zeroed when the x-swept column holds a wet cell anywhere, else left as they are.  The block looks through each of their
 // columns once, together: a 512 x 512 grid with a quarter of such land 0.61 ms a
 // step, 2.1 with a look for each cell (0.50 a launch per sweep).
 template <class T>
@@ -1116,8 +1141,8 @@ __device__ __noinline__ bool step_y_scan(const SweepArgs& X, const SweepArgs& Y,
 // The y phase's, to the output fields.
 template <class T>
 __device__ __forceinline__ bool step_y_list(const SweepArgs& X, const SweepArgs& Y, int rb, int c0, StepShared<T>& S) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const unsigned cy = S.n[1];
+  const int tid = threadIdx.x;
+  const unsigned lane = tid & 31, cy = S.n[1];
   bool bad = false;
   const auto store = [&](int t, int c, const OutCell<float>& r) {
     const size_t q = (size_t)(rb + t - 1) * (size_t)Y.pitch + (size_t)(c0 + c);
@@ -1130,17 +1155,18 @@ __device__ __forceinline__ bool step_y_list(const SweepArgs& X, const SweepArgs&
   // rows, a pair of lanes each; a few of both kinds go by pairs together (apart,
   // the one block of a 1003 x 777 grid with both took 21.1 us a step for its 19.1)
   WarpQueue Q{S.queue[tid >> 5][0]}, E{S.queue[tid >> 5][1]};
-  for (unsigned base = (unsigned)(tid & ~31);; base += T::Threads) {
+  const unsigned share = list_share<T>(cy), round = share * (T::Threads / 32);
+  for (unsigned base = share * (unsigned)(tid >> 5);; base += round) {
     const unsigned i = base + lane;
     bool hard = false, end = false;
-    if (i < cy) {
+    if (lane < share && i < cy) {
       const int t = S.list[i] / T::W, c = S.list[i] % T::W;
       const XValue r = step_y_shore<T>(Y, S.win, rb, c0, t, c);
       hard = !r.ok;
       end = T::Halo < 3 && (t < 3 || t >= T::Rows - 3);
       if (r.ok) store(t, c, r.out);
     }
-    const bool last = base + T::Threads >= cy;
+    const bool last = base + round >= cy;
     Q.push(hard && !end, i);
     if (T::Halo < 3) {
       E.push(hard && end, i);
@@ -1367,7 +1393,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
 // all scenarios' tiles (coasts first, as above), the scenario's arguments
 // staged in shared memory and its tensor maps read from device memory.  24
 // scenarios of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with
-// its uploads and maxima: 6.7 ms, from 12.2 with a launch per sweep phase.
+// its uploads and maxima: 6.6 ms, from 12.2 with a launch per sweep phase.
 struct StepArgs {
   SweepArgs X, Y;
   PairPair K;
