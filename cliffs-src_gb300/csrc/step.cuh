@@ -28,9 +28,9 @@
 // x-swept tile.  Tiles with a coast in them take longest and go first.
 //
 // Measured (us per step, replayed from graphs, against a launch per sweep;
-// the same state bits): 4320 x 2160 sphere 88 from 144; 2048 x 2048 shelf 44.2
-// from 68.6; 1500 x 1500 28.4 from 41.0; 1201 x 903 stretched 20.8 from 29.3;
-// 1003 x 777 15.3 from 21.8; 600 x 600 11.6 from 18.4; 256 x 256 9.0 from 15.1.
+// the same state bits): 4320 x 2160 sphere 88 from 144; 2048 x 2048 shelf 44.3
+// from 68.6; 1500 x 1500 28.4 from 41.0; 1201 x 903 stretched 20.9 from 29.3;
+// 1003 x 777 15.3 from 21.8; 600 x 600 11.5 from 18.4; 256 x 256 9.1 from 15.1.
 // On the shelf 209 thread instructions a cell (400 in the two sweeps), 39 bytes
 // a cell to and from DRAM, 16 warps an SM at 128 registers and 0.53
 // instructions an SM sub-core and cycle while it is busy: what bounds it is the
@@ -1393,7 +1393,7 @@ __global__ void __launch_bounds__(T::Threads, T::Blocks)
 // all scenarios' tiles (coasts first, as above), the scenario's arguments
 // staged in shared memory and its tensor maps read from device memory.  24
 // scenarios of 256 to 768 nodes a side (6.8 M cells), a run of 64 steps with
-// its uploads and maxima: 6.6 ms, from 12.2 with a launch per sweep phase.
+// its uploads and maxima: 6.7 ms, from 12.2 with a launch per sweep phase.
 struct StepArgs {
   SweepArgs X, Y;
   PairPair K;

@@ -132,6 +132,7 @@ class MLP:
     def predict(self, x):
         x = _f32(x)
         y = np.empty((x.shape[0], self.n_y), np.float32)  # all of it written: 16 MB of maps take 0.28 ms to clear
+        # (on pages that the allocator hands back; the first touch of fresh ones takes longer than the call)
         cg._chk(self.L.cliffs_mlp_predict(self.h, x.shape[0], x.ctypes.data_as(_fp), y.ctypes.data_as(_fp)),
                 "mlp_predict")
         return y

@@ -299,13 +299,19 @@ int cliffs_gpu_launch_count(cliffs_ctx *ctx, int64_t *n);
  * no graph).  Steps without profiling or a rising source are replayed from
  * a graph, one launch per k steps; the last steps of a call, when fewer than
  * k but at least 2, from a graph of their own length (a few such lengths are
- * kept per context).  Plain steps that find no graph of their length yet
+ * kept per context).  Whole steps in one kernel leave the state in its other
+ * copy, so graphs of plain ones hold an even number (k - 1 where k is odd), a
+ * call's last odd step runs a launch per sweep, and without graphs they run in
+ * pairs.  Plain steps that find no graph of their length yet
  * run launch by launch while the graph is captured for the calls that
  * follow.  A fresh state's first step (after set_initial, an upload, a
- * source, a single sweep) runs on its own.  With boundary forcing
- * (two-dimensional grids) the graph first fills the k steps' edge tables in
- * one kernel, from the records and weights the library's cursor gives each
- * step; a chunk in which the forcing ends runs step by step. */
+ * source, a single sweep) runs on its own, a launch per sweep.  With boundary
+ * forcing (two-dimensional grids) the graph first fills the k steps' edge
+ * tables in one kernel, from the records and weights the library's cursor
+ * gives each step (whole steps where k is even, else a launch per sweep); fewer
+ * than k forced steps, and a chunk in which the forcing ends, run step by step
+ * with a launch per sweep.  An unforced one-dimensional grid of at most 7648
+ * cells needs no graph: its steps run many to a launch. */
 int cliffs_gpu_set_graph_steps(cliffs_ctx *ctx, int32_t k);
 /* Capture and instantiate, without running them, the graphs that a
  * cliffs_gpu_step(ctx, nsteps) call made from the current state would
@@ -316,34 +322,42 @@ int cliffs_gpu_prepare_steps(cliffs_ctx *ctx, int32_t nsteps);
 
 /* Tuning: threads per block of the x-sweep kernel (multiple of 32, <= 256)
  * and warps per block of the y-sweep kernel (<= 8).  0 keeps the current
- * value.  Results do not depend on the tiling.  Applies to the tiled sweep
- * kernels. */
+ * value.  Results do not depend on the tiling; the time does: whole steps in
+ * one kernel, and the many steps a launch of a one-dimensional grid, are for
+ * the default shape (128 threads, 4 warps), and any other runs a launch per
+ * sweep.  Applies to the tiled sweep kernels. */
 int cliffs_gpu_set_tiling(cliffs_ctx *ctx, int32_t block_x, int32_t warps_y);
 
 /* The sweep kernels, three choices with identical results:
- * - CLIFFS_SWEEP_TILED (the default): one block per tile.  The x-sweep loads
- *   its window straight into registers; the y-sweep of a two-dimensional step
- *   has its tile (16 rows x 32 columns and a halo row each side) brought into
- *   shared memory by tensor-map copies (TMA) and stored back the same way.
- * - CLIFFS_SWEEP_DIRECT: the tiled kernels with the y-sweep's window loaded
+ * - CLIFFS_SWEEP_TILED (the default): a two-dimensional step in one launch, one
+ *   block per tile (64 x 30 cells, smaller ones on smaller grids), the tile's
+ *   window brought into shared memory by tensor-map copies (TMA) and both sweeps
+ *   taken there; a one-dimensional grid's steps many to a launch.  Steps that
+ *   these do not take (cliffs_gpu_set_graph_steps) run a launch per sweep: the
+ *   x-sweep with its window loaded straight into registers, the y-sweep's tile
+ *   (16 rows x 32 columns and a halo row each side) brought in and stored back
+ *   by tensor-map copies.
+ * - CLIFFS_SWEEP_DIRECT: a launch per sweep, the y-sweep's window loaded
  *   straight into registers too.
  * - CLIFFS_SWEEP_STAGED: persistent kernels, one resident grid walking the
  *   tiles.  Each block's window loads arrive in shared memory by bulk copies
  *   (TMA), one tile ahead of the compute.  On GB300 it is the slowest of the
  *   three.
  * A context whose tensor maps could not be made runs the direct kernels
- * whichever is chosen; so does a y-sweep tiling (cliffs_gpu_set_tiling) other
- * than 4 warps. */
+ * whichever is chosen (one-dimensional grids aside); so does a y-sweep tiling
+ * (cliffs_gpu_set_tiling) other than 4 warps. */
 enum { CLIFFS_SWEEP_TILED = 0, CLIFFS_SWEEP_STAGED = 1, CLIFFS_SWEEP_DIRECT = 2 };
 int cliffs_gpu_set_sweep_kernel(cliffs_ctx *ctx, int32_t kind);
 /* Failure-detection check of the kernels' waits for their tensor-map and
  * bulk copies: one staged x-sweep, then (on a two-dimensional grid) one tiled
- * y-sweep, whose waits expect 16 bytes more than the copies bring, each wait
- * limited to wait_ms (1..2000); a y block waits twice before it leaves, so
- * the check takes about 2 * wait_ms per wave of y blocks.  Expected result:
- * CLIFFS_ERR_TIMEOUT, read by the host, when both sweeps reported their
- * waits running out, with the device usable afterwards.  The state is
- * unchanged: the sweeps write the other state copy, which is not taken.
+ * y-sweep and one whole step, whose waits expect 16 bytes more than the copies
+ * bring, each wait limited to wait_ms (1..2000); a block of the last two waits
+ * twice before it leaves, so the check takes about 2 * wait_ms per wave of y
+ * blocks and of step blocks.  Expected result: CLIFFS_ERR_TIMEOUT, read by the
+ * host, when all of them reported their waits running out, with the device
+ * usable afterwards.  The state and the maxima are unchanged: the sweeps write
+ * the other state copy, which is not taken, and the step's blocks leave before
+ * they write anything.
  * CLIFFS_ERR_STATE without a state, an x-sweep or the staged kernels. */
 int cliffs_gpu_check_stage_timeout(cliffs_ctx *ctx, int32_t wait_ms);
 
@@ -396,9 +410,10 @@ int cliffs_gpu_sweep_noalloc_status(void *stream, uint32_t *flags, uint32_t *lis
  * size) together: every scenario's sweeps are cut into the single-grid
  * kernels' tiles, the tiles of all scenarios form one list (of whole steps or
  * per sweep direction), and either one cooperative launch covers many steps
- * (blocks meet at a grid barrier between the x and y phases) or one launch per
- * step (a phase, where a scenario does not take whole steps) covers every
- * scenario, replayed from a CUDA graph.  Results are
+ * (blocks meet at a grid barrier between the x and y phases; what a new batch
+ * does) or one launch per step covers every scenario, replayed from a CUDA graph
+ * (graph plans of one tile an entry where every scenario takes whole steps, in
+ * pairs; otherwise, and for the last odd step, a launch per phase).  Results are
  * bit-identical to stepping the contexts one by one with cliffs_gpu_step.
  * Contexts must be 2-D, hold a state, have no boundary forcing, and live on
  * the current device; a source still rising (cliffs_gpu_add_source) is
@@ -441,9 +456,10 @@ int cliffs_batch_autotune(cliffs_batch *b, int32_t probe_steps, double *ms_per_s
  * first barrier waits for an arrival that no block makes, with the wait
  * limited to wait_ms (1..2000).  Then, when the batch's y phase runs on
  * tiles by tensor-map copies, one such phase whose copy waits expect 16
- * bytes more than the copies bring (each block waits twice, about
- * 2 * wait_ms per wave of blocks).  Expected result: CLIFFS_ERR_TIMEOUT
- * (both reported), read by the host, with the device usable afterwards.
+ * bytes more than the copies bring, and, when its scenarios take whole steps,
+ * one such step likewise (each block waits twice, about 2 * wait_ms per wave of
+ * blocks).  Expected result: CLIFFS_ERR_TIMEOUT (all of them reported), read by
+ * the host, with the device usable afterwards.
  * The persistent launch applies the x-sweep of one step to the contexts
  * before the barrier: their state is undefined until uploaded again. */
 int cliffs_batch_check_barrier_timeout(cliffs_batch *b, int32_t wait_ms);
