@@ -1104,9 +1104,10 @@ __device__ __forceinline__ bool step_x_list(const SweepArgs& X, int rb, int c0, 
 }
 
 // Remainders on land with no water in the window's part of their column, marked in
-// the list: zeroed when the x-swept column holds a wet cell anywhere, else left as they are.  The block looks through each of their
-// columns once, together: a 512 x 512 grid with a quarter of such land 0.61 ms a
-// step, 2.1 with a look for each cell (0.50 a launch per sweep).
+// the list: zeroed when the x-swept column holds a wet cell anywhere, else left as
+// they are.  The block looks through each of their columns once, together: a 512 x
+// 512 grid with a quarter of such land 0.61 ms a step, 2.1 with a look for each cell
+// (0.50 a launch per sweep).
 template <class T>
 __device__ __noinline__ bool step_y_scan(const SweepArgs& X, const SweepArgs& Y, int rb, int c0, StepShared<T>& S) {
   const int tid = threadIdx.x;
